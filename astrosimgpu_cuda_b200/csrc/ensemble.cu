@@ -1,15 +1,17 @@
 // ensemble.cu -- batched stepping of many independent networks (see ensemble.cuh).
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <thread>
 #include <type_traits>
+#include <utility>
 
 #include "ensemble.cuh"
-#include "window_kernels.cuh"
+#include "window_cells.cuh"
 
 namespace astrosim {
 
@@ -23,29 +25,38 @@ struct alignas(16) NetDesc {
     i64 mark;  // last step of the pre-run (src/astrosim_fused.cu:1066)
 };
 
-// Variants the autotuner chooses from: (tile size = block size, minimum resident
-// blocks per SM).  A tile is `tile` consecutive cells of one population of one
+// Variants the autotuner chooses from: (block size, minimum resident blocks per SM, cells
+// per thread).  A tile is block * cells consecutive cells of one population of one
 // network; each block stages its network's descriptor once, so larger tiles stage
 // less per cell and smaller tiles balance networks of very different sizes better.
+// One cell per thread suits batches that do not fill the chip (see window.cu).
 struct EnsVariant {
-    int tile, min_blocks;
+    int block, min_blocks, cells;
 };
-constexpr EnsVariant kEnsVariantsF32[] = {{128, 6}, {128, 8}, {128, 4}, {64, 12}, {64, 16}, {64, 8},
-                                          {256, 3}, {256, 4}, {256, 2}};
-constexpr EnsVariant kEnsVariantsF64[] = {{128, 4}, {128, 5}, {128, 3}, {64, 8}, {64, 10}, {64, 6},
-                                          {256, 2}, {256, 3}, {256, 1}};
+#ifndef ASTROSIM_FP32_IEEE
+constexpr EnsVariant kEnsVariantsF32[] = {{128, 5, 2}, {128, 6, 2}, {128, 8, 1}, {64, 10, 2}, {64, 12, 2}, {64, 12, 1},
+                                          {256, 2, 2}, {256, 3, 2}, {256, 4, 1}};
+#else
+constexpr EnsVariant kEnsVariantsF32[] = {{128, 6, 1}, {128, 8, 1}, {128, 4, 1}, {64, 12, 1}, {64, 16, 1}, {64, 8, 1},
+                                          {256, 3, 1}, {256, 4, 1}, {256, 2, 1}};
+#endif
+constexpr EnsVariant kEnsVariantsF64[] = {{128, 4, 1}, {128, 5, 1}, {128, 3, 1}, {64, 8, 1}, {64, 10, 1}, {64, 6, 1},
+                                          {256, 2, 1}, {256, 3, 1}, {256, 1, 1}};
 constexpr int kEnsNumVariants = 9;
-constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256};
-int tile_index(int tile) { return tile == 64 ? 0 : (tile == 256 ? 2 : 1); }
+constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256, 512};
+int tile_index(int tile) { return tile == 64 ? 0 : tile == 128 ? 1 : tile == 256 ? 2 : 3; }
 constexpr int kEnsTuneRounds = 2;
 constexpr int kGraphWindows = 10;
 constexpr u32 kPushBlocksPerNet = 4;
+// A tile table entry: the population in the upper bits, the tile's index within it below.
+constexpr u32 kTileKindShift = 30;
+constexpr u32 kTileIndexMask = (1u << kTileKindShift) - 1;
 
-// One window of one tile of blockDim.x cells.  UNI: every network shares the constants
+// One window of one tile (the cells of one block).  UNI: every network shares the constants
 // outside NetScalars, which then come from the kernel parameters (`common`); otherwise
 // each block also stages its network's full constants (`rcs`) into shared memory.
-template <typename R, int TILE, int MB, bool UNI>
-__global__ void __launch_bounds__(TILE, MB) ens_window_kernel(RunConsts common, const RunConsts* __restrict__ rcs,
+template <typename R, int BLOCK, int MB, int CELLS, bool UNI>
+__global__ void __launch_bounds__(BLOCK, MB) ens_window_kernel(RunConsts common, const RunConsts* __restrict__ rcs,
                                                              const NetDesc<R>* __restrict__ descs,
                                                              const u32* __restrict__ tile_net,
                                                              const u32* __restrict__ tile_blk,
@@ -74,25 +85,52 @@ __global__ void __launch_bounds__(TILE, MB) ens_window_kernel(RunConsts common, 
     const NetDesc<R>& d = *reinterpret_cast<const NetDesc<R>*>(smem);
     const int s_end = static_cast<int>(end - start < W ? end - start : W);
     const u32 tb = tile_blk[blockIdx.x];
+    const int kind = static_cast<int>(tb >> kTileKindShift);
+    const u32 first = kind == kInhCells ? d.ns.n_exc : 0;
+    const u32 last = kind == kAstroCells ? d.ns.n_astro : (kind == kExcCells ? d.ns.n_exc : d.ns.n_neurons);
+    const Tile tile{kind, first + (tb & kTileIndexMask) * static_cast<u32>(BLOCK * CELLS), last};
     if constexpr (UNI) {
-        window_cells<R>(common, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tb & 0x7FFFFFFFu,
-                        (tb >> 31) != 0);
+        window_cells<R, CELLS>(common, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tile);
     } else {
         const RunConsts& rc = *reinterpret_cast<const RunConsts*>(smem + kDescBytes);
-        window_cells<R>(rc, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tb & 0x7FFFFFFFu,
-                        (tb >> 31) != 0);
+        window_cells<R, CELLS>(rc, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tile);
     }
 }
 
+constexpr int kEnsPushBlock = 256;
+constexpr int kEnsDrawCells = 2;
+
+// After every network's window: the first kPushBlocksPerNet * n_nets blocks deliver its
+// spikes, the others draw the background events of the window that follows (one tile of
+// the draw table each).  `ahead`: 1 after a window, 0 to draw for the current window
+// (no delivery).
 template <typename R>
-__global__ void ens_push_kernel(const NetDesc<R>* __restrict__ descs, const i64* __restrict__ win,
-                                const i64* __restrict__ stop, int W) {
-    const u32 net = blockIdx.y;
-    const i64 k = win[net];
-    if (k * W + W > stop[net]) return;  // the window did not complete: no window follows it
-    const NetDesc<R>& d = descs[net];
-    push_cells<R>(d.w, d.ns.n_exc, d.ns.n_neurons - d.ns.n_exc, d.ns.n_neurons, d.ns.n_astro,
-                  static_cast<int>(k & 1), blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(kEnsPushBlock) ens_push_kernel(const NetDesc<R>* __restrict__ descs,
+                                                                 const i64* __restrict__ win,
+                                                                 const i64* __restrict__ stop, int W, u32 push_blocks,
+                                                                 const u32* __restrict__ draw_net,
+                                                                 const u32* __restrict__ draw_blk, int ahead) {
+    extern __shared__ u32 rows[];
+    if (blockIdx.x < push_blocks) {
+        const u32 net = blockIdx.x / kPushBlocksPerNet;
+        const i64 k = win[net];
+        if (k * W + W > stop[net]) return;  // the window did not complete: no window follows it
+        const NetDesc<R>& d = descs[net];
+        push_cells<R>(d.w, d.ns.n_exc, d.ns.n_neurons - d.ns.n_exc, d.ns.n_neurons, d.ns.n_astro,
+                      static_cast<int>(k & 1), blockIdx.x % kPushBlocksPerNet, kPushBlocksPerNet);
+        return;
+    }
+    const u32 net = draw_net[blockIdx.x - push_blocks];
+    const i64 start = (win[net] + ahead) * W;
+    if (start >= stop[net]) return;  // no such window
+    const NetScalars ns = descs[net].ns;
+    const u32 tb = draw_blk[blockIdx.x - push_blocks];
+    const int kind = static_cast<int>(tb >> kTileKindShift);
+    const u32 first = kind == kInhCells ? ns.n_exc : 0;
+    draw_events<kEnsDrawCells>(ns, descs[net].w.events, start, W,
+                Tile{kind, first + (tb & kTileIndexMask) * static_cast<u32>(kEnsPushBlock * kEnsDrawCells),
+                     kind == kExcCells ? ns.n_exc : ns.n_neurons},
+                rows);
 }
 
 __global__ void ens_advance_kernel(i64* win, const i64* stop, u32 n, int W) {
@@ -100,52 +138,39 @@ __global__ void ens_advance_kernel(i64* win, const i64* stop, u32 n, int W) {
     if (i < n && win[i] * W < stop[i]) win[i] += 1;
 }
 
-template <typename R, bool UNI>
-void launch_ens_window_v(int v, u32 grid, cudaStream_t st, const RunConsts& common, const RunConsts* rcs,
-                         const NetDesc<R>* d, const u32* tn, const u32* tb, const i64* win, const i64* stop, int W) {
-    constexpr bool f32 = std::is_same<R, float>::value;
-    const EnsVariant x = f32 ? kEnsVariantsF32[v] : kEnsVariantsF64[v];
-#define AS_ENS(T, M) ens_window_kernel<R, T, M, UNI><<<grid, T, 0, st>>>(common, rcs, d, tn, tb, win, stop, W)
-    if constexpr (f32) {
-        switch (x.tile * 100 + x.min_blocks) {
-            case 12808: AS_ENS(128, 8); break;
-            case 12804: AS_ENS(128, 4); break;
-            case 6412: AS_ENS(64, 12); break;
-            case 6416: AS_ENS(64, 16); break;
-            case 6408: AS_ENS(64, 8); break;
-            case 25603: AS_ENS(256, 3); break;
-            case 25604: AS_ENS(256, 4); break;
-            case 25602: AS_ENS(256, 2); break;
-            default: AS_ENS(128, 6); break;
-        }
-    } else {
-        switch (x.tile * 100 + x.min_blocks) {
-            case 12805: AS_ENS(128, 5); break;
-            case 12803: AS_ENS(128, 3); break;
-            case 6408: AS_ENS(64, 8); break;
-            case 6410: AS_ENS(64, 10); break;
-            case 6406: AS_ENS(64, 6); break;
-            case 25602: AS_ENS(256, 2); break;
-            case 25603: AS_ENS(256, 3); break;
-            case 25601: AS_ENS(256, 1); break;
-            default: AS_ENS(128, 4); break;
-        }
-    }
-#undef AS_ENS
+template <typename R>
+using EnsLaunchFn = void (*)(u32, cudaStream_t, const RunConsts&, const RunConsts*, const NetDesc<R>*, const u32*,
+                             const u32*, const i64*, const i64*, int);
+template <typename R, bool UNI, int V>
+void launch_ens_window_v(u32 grid, cudaStream_t st, const RunConsts& common, const RunConsts* rcs, const NetDesc<R>* d,
+                         const u32* tn, const u32* tb, const i64* win, const i64* stop, int W) {
+    constexpr EnsVariant v = std::is_same<R, float>::value ? kEnsVariantsF32[V] : kEnsVariantsF64[V];
+    ens_window_kernel<R, v.block, v.min_blocks, v.cells, UNI>
+        <<<grid, v.block, 0, st>>>(common, rcs, d, tn, tb, win, stop, W);
+}
+template <typename R, bool UNI, int... V>
+constexpr std::array<EnsLaunchFn<R>, sizeof...(V)> ens_launches(std::integer_sequence<int, V...>) {
+    return {&launch_ens_window_v<R, UNI, V>...};
 }
 
-int variant_tile(bool fp32, int v) { return fp32 ? kEnsVariantsF32[v].tile : kEnsVariantsF64[v].tile; }
+int variant_tile(bool fp32, int v) {
+    const EnsVariant x = fp32 ? kEnsVariantsF32[v] : kEnsVariantsF64[v];
+    return x.block * x.cells;
+}
 
 // One window and its push for every network.
 template <typename R>
 void launch_ens_window(int v, bool uniform, u32 grid, u32 n, cudaStream_t st, const RunConsts& common,
                        const void* rcs, const void* descs, const u32* tn, const u32* tb, const i64* win,
-                       const i64* stop, int W) {
+                       const i64* stop, int W, u32 draws, const u32* draw_net, const u32* draw_blk) {
     const RunConsts* r = static_cast<const RunConsts*>(rcs);
     const NetDesc<R>* d = static_cast<const NetDesc<R>*>(descs);
-    if (uniform) launch_ens_window_v<R, true>(v, grid, st, common, r, d, tn, tb, win, stop, W);
-    else launch_ens_window_v<R, false>(v, grid, st, common, r, d, tn, tb, win, stop, W);
-    ens_push_kernel<R><<<dim3(kPushBlocksPerNet, n), 256, 0, st>>>(d, win, stop, W);
+    constexpr auto seq = std::make_integer_sequence<int, kEnsNumVariants>();
+    static constexpr auto shared_table = ens_launches<R, true>(seq), own_table = ens_launches<R, false>(seq);
+    (uniform ? shared_table : own_table)[v](grid, st, common, r, d, tn, tb, win, stop, W);
+    const u32 push_blocks = kPushBlocksPerNet * n;
+    ens_push_kernel<R><<<push_blocks + draws, kEnsPushBlock, poisson_bytes(kEnsDrawCells, W, kEnsPushBlock), st>>>(
+        d, win, stop, W, push_blocks, draw_net, draw_blk, 1);
 }
 
 // `rc` with the NetScalars fields cleared.  RunConsts has no implicit padding, so
@@ -221,6 +246,8 @@ Ensemble::~Ensemble() {
         tile_net_[ti].release();
         tile_blk_[ti].release();
     }
+    draw_net_.release();
+    draw_blk_.release();
     win_.release();
     stop_.release();
     if (stream_) {
@@ -330,14 +357,12 @@ Status Ensemble::rebuild() {
         for (u32 i = 0; i < nets_.size(); ++i) {
             if (!nets_[i]) continue;
             const RunConsts& rc = nets_[i]->consts();
-            for (u32 b = 0; b < ceil_div(rc.n_astro, tile); ++b) {
-                tn.push_back(i);
-                tb.push_back(b | 0x80000000u);
-            }
-            for (u32 b = 0; b < ceil_div(rc.n_neurons, tile); ++b) {
-                tn.push_back(i);
-                tb.push_back(b);
-            }
+            const CellTiles t = cell_tiles(rc.n_exc, 0, rc.n_neurons, 0, rc.n_astro, tile);
+            for (const u32 kind : {u32(kAstroCells), u32(kExcCells), u32(kInhCells)})
+                for (u32 b = 0; b < t.tiles[kind]; ++b) {
+                    tn.push_back(i);
+                    tb.push_back(b | kind << kTileKindShift);
+                }
         }
         n_tiles_[ti] = static_cast<u32>(tn.size());
         AS_TRY(tile_net_[ti].alloc(std::max<size_t>(1, tn.size())));
@@ -349,6 +374,30 @@ Status Ensemble::rebuild() {
                                     stream_));
         }
         AS_CUDA(cudaStreamSynchronize(stream_));  // the host vectors die at the end of this iteration
+    }
+    {
+        std::vector<u32> dn, db;
+        for (u32 i = 0; i < nets_.size(); ++i) {
+            if (!nets_[i]) continue;
+            const RunConsts& rc = nets_[i]->consts();
+            const CellTiles t = event_tiles(rc.n_exc, 0, rc.n_neurons, kEnsPushBlock, kEnsDrawCells);
+            for (const u32 kind : {u32(kExcCells), u32(kInhCells)})
+                for (u32 b = 0; b < t.tiles[kind]; ++b) {
+                    dn.push_back(i);
+                    db.push_back(b | kind << kTileKindShift);
+                }
+        }
+        n_draws_ = static_cast<u32>(dn.size());
+        AS_TRY(draw_net_.alloc(std::max<size_t>(1, dn.size())));
+        AS_TRY(draw_blk_.alloc(std::max<size_t>(1, db.size())));
+        if (!dn.empty()) {
+            AS_CUDA(cudaMemcpyAsync(draw_net_.get(), dn.data(), dn.size() * sizeof(u32), cudaMemcpyHostToDevice,
+                                    stream_));
+            AS_CUDA(cudaMemcpyAsync(draw_blk_.get(), db.data(), db.size() * sizeof(u32), cudaMemcpyHostToDevice,
+                                    stream_));
+        }
+        AS_TRY(draw_current());
+        AS_CUDA(cudaStreamSynchronize(stream_));  // the host vectors die here
     }
     if (graph_) {
         cudaGraphExecDestroy(graph_);
@@ -363,10 +412,29 @@ void Ensemble::launch_window(int v) {
     const int ti = tile_index(variant_tile(fp32_, v));
     if (fp32_)
         launch_ens_window<float>(v, uniform_, n_tiles_[ti], n, stream_, common_, rcs_.get(), descs_.get(),
-                                 tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_);
+                                 tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_, n_draws_,
+                                 draw_net_.get(), draw_blk_.get());
     else
         launch_ens_window<double>(v, uniform_, n_tiles_[ti], n, stream_, common_, rcs_.get(), descs_.get(),
-                                  tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_);
+                                  tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_, n_draws_,
+                                  draw_net_.get(), draw_blk_.get());
+}
+
+// The background events of every network's current window: after a change of membership,
+// whose new networks have none yet (the others' are drawn again, to the same counts).
+Status Ensemble::draw_current() {
+    if (n_draws_ == 0) return Status::Ok();
+    const size_t smem = poisson_bytes(kEnsDrawCells, W_, kEnsPushBlock);
+    if (fp32_)
+        ens_push_kernel<float><<<n_draws_, kEnsPushBlock, smem, stream_>>>(
+            reinterpret_cast<const NetDesc<float>*>(descs_.get()), win_.get(), stop_.get(), W_, 0, draw_net_.get(),
+            draw_blk_.get(), 0);
+    else
+        ens_push_kernel<double><<<n_draws_, kEnsPushBlock, smem, stream_>>>(
+            reinterpret_cast<const NetDesc<double>*>(descs_.get()), win_.get(), stop_.get(), W_, 0, draw_net_.get(),
+            draw_blk_.get(), 0);
+    AS_CUDA(cudaGetLastError());
+    return Status::Ok();
 }
 
 Status Ensemble::capture_graph() {

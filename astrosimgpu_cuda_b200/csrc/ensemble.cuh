@@ -2,14 +2,13 @@
 //
 // Each network keeps its own device state exactly as a single Simulation (its own
 // windowed engine buffers).  One window launch covers every cell of every network:
-// a tile table maps each block (a tile of 64, 128 or 256 cells: the autotuner times
-// each size with three occupancy targets) to (network, population, tile), and each
-// block reads its network's descriptor (constants and pointers) into shared memory.
+// a tile table maps each block (64, 128 or 256 threads with one or two cells each: the
+// autotuner times them) to (network, population, tile), and each block reads its network's descriptor (constants and pointers) into shared memory.
 // The constants that differ between networks (NetScalars) sit in the descriptor;
 // when every network shares the rest (the same biology, dt and substeps) those come
 // from the kernel parameters, else each block also stages its network's full
 // constants.  Every network has its own window counter and stop step on the device, so the
-// per-window sequence {window, push, advance} is identical for every window and is
+// per-window sequence {window, push and next window's draws, advance} is identical for every window and is
 // captured once in a CUDA graph and replayed.
 #pragma once
 
@@ -21,7 +20,7 @@
 
 namespace astrosim {
 
-constexpr int kNumTileSizes = 3;  // tiles of 64, 128 or 256 cells, chosen by the autotuner
+constexpr int kNumTileSizes = 4;  // tiles of 64, 128, 256 or 512 cells, chosen by the autotuner
 
 class Ensemble {
 public:
@@ -52,6 +51,7 @@ private:
     Status capture_graph();
     Status sync_progress();
     void launch_window(int v);  // window + push kernels for variant v
+    Status draw_current();      // background events of the current windows
 
     std::vector<std::unique_ptr<Simulation>> nets_;
     std::vector<cudaStream_t> build_streams_;  // lent to the networks create() built
@@ -67,10 +67,12 @@ private:
     DevBuf<unsigned char> rcs_;  // RunConsts per network (read when !uniform_)
     RunConsts common_{};         // shared constants (NetScalars fields cleared)
     bool uniform_ = true;
-    // tile tables for tiles of 64, 128 and 256 cells
+    // tile tables by tile size
     DevBuf<u32> tile_net_[kNumTileSizes], tile_blk_[kNumTileSizes];
+    DevBuf<u32> draw_net_, draw_blk_;  // tiles of the background draws
+    u32 n_draws_ = 0;
     DevBuf<i64> win_, stop_;
-    u32 n_tiles_[kNumTileSizes] = {0, 0, 0};
+    u32 n_tiles_[kNumTileSizes] = {};
     bool dirty_ = true;
     int variant_ = -1;  // (tile size, launch bounds) variant; -1 while the autotuner times them
     int tune_step_ = 0;

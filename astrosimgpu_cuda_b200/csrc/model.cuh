@@ -38,6 +38,14 @@ __host__ __device__ __forceinline__ u64 rng_mix(u64 z) {
     return z ^ (z >> 31);
 }
 
+// The upper 32 bits of rng_mix(z), without the lower half's last multiply and fold.
+__host__ __device__ __forceinline__ u32 rng_mix_hi(u64 z) {
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+    const u32 hi = static_cast<u32>(z >> 32);
+    return hi ^ (hi >> 31);
+}
+
 __host__ __device__ __forceinline__ u64 rng_bits(u64 seed, u64 stream, u64 counter) {
     u64 z = seed;
     z += stream * kStreamMul;
@@ -198,8 +206,12 @@ struct NeuronK {
     int pad_;  // explicit, zero: the struct has no implicit padding
     // RN(1 / x) of the constant divisors, for the exact division by a constant (div_by).
     double rcp_C_m, rcp_tau_w, rcp_Delta_T;
+    // exp(-h_step / tau_syn) in the stage type, evaluated on the device once per network
+    // (src/astrosim_fused.cu:515-516 evaluates it in every step).
+    double ex_decay, in_decay;
+    float f_ex_decay, f_in_decay;
 };
-static_assert(sizeof(NeuronK) == 17 * 8 + 22 * 4 + 2 * 4 + 3 * 8, "NeuronK has no implicit padding");
+static_assert(sizeof(NeuronK) == 17 * 8 + 24 * 4 + 2 * 4 + 5 * 8, "NeuronK has no implicit padding");
 
 // Biology defaults, compiled into the reference (src/astrosim_fused.cu:742-781).
 struct Biology {
@@ -534,8 +546,8 @@ __device__ __forceinline__ float normal_fast(u64 base) {
     const float l1 = d1 > 0.0 ? log_fast(static_cast<float>(d1)) : -690.775528f;
     return sqrt_ftz(-2.0f * l1) * cos_ftz(static_cast<float>(kTwoPi) * static_cast<float>(d2));
 #else
-    const u32 a = static_cast<u32>(rng_mix(base) >> 40);
-    const u32 b = static_cast<u32>(rng_mix(base + kCounterMul) >> 40);
+    const u32 a = rng_mix_hi(base) >> 8;  // the upper 24 bits of each draw
+    const u32 b = rng_mix_hi(base + kCounterMul) >> 8;
     const float u1 = (static_cast<float>(a) + 0.5f) * (1.0f / 16777216.0f);
     const float u2 = static_cast<float>(b) * (1.0f / 16777216.0f);
     return sqrt_ftz(-2.0f * log_fast(u1)) * cos_ftz(static_cast<float>(kTwoPi) * u2);

@@ -11,7 +11,7 @@
 #include <thread>
 
 #include "shard.cuh"
-#include "window_kernels.cuh"
+#include "window_cells.cuh"
 
 namespace astrosim {
 
@@ -26,15 +26,26 @@ ShardPlan shard_plan(u32 n_neurons, u32 n_astro, int rank, int world) {
 
 namespace {
 
-// One window of this rank's cells: astrocyte blocks [a_blk0, a_blk0 + a_nblk), then
-// neuron blocks from n_blk0.
+// Cells per thread: two in the FP32 form (a sharded network fills its GPUs).
+template <typename R>
+constexpr int kShardCells = 1;
+#ifndef ASTROSIM_FP32_IEEE
+template <>
+constexpr int kShardCells<float> = 2;
+#endif
+
+// One window of this rank's cells.
 template <typename R, int MB>
 __global__ void __launch_bounds__(128, MB) shard_window_kernel(RunConsts rc, StepPtrs<R> p, WinPtrs<R> w,
-                                                               i64 win_start, int buf, i64 mark, u32 a_blk0,
-                                                               u32 a_nblk, u32 n_blk0) {
-    const bool astro = blockIdx.x < a_nblk;
-    window_cells<R>(rc, net_scalars(rc), p, w, win_start, 0, w.W, buf, mark, astro ? a_blk0 + blockIdx.x : n_blk0 + (blockIdx.x - a_nblk),
-                    astro);
+                                                               i64 win_start, int buf, i64 mark, CellTiles tiles) {
+    window_cells<R, kShardCells<R>>(rc, net_scalars(rc), p, w, win_start, 0, w.W, buf, mark, tile_of(tiles, blockIdx.x));
+}
+
+// The background events of this rank's neurons in the window that starts at win_start.
+__global__ void __launch_bounds__(256) shard_draw_kernel(NetScalars ns, u64* events, i64 win_start, int W,
+                                                         CellTiles tiles) {
+    extern __shared__ u32 rows[];
+    draw_events<2>(ns, events, win_start, W, tile_of(tiles, blockIdx.x), rows);
 }
 
 template <typename R>
@@ -107,14 +118,20 @@ Status window_phase(ShardSim& s, i64 k) {
     WindowState& ws = *sim.window_state();
     StepPtrs<R> p = make_ptrs<R>(sim.state_buffers(), sim.network(), rc, sim.raster_steps());
     WinPtrs<R> w = win_ptrs<R>(ws, rc);
-    const u32 a_blk0 = s.plan.a_lo / 128, a_nblk = ceil_div(s.plan.a_hi - s.plan.a_lo, 128);
-    const u32 n_blk0 = s.plan.n_lo / 128, n_nblk = ceil_div(s.plan.n_hi - s.plan.n_lo, 128);
-    const u32 grid = a_nblk + n_nblk;
+    const CellTiles tiles = cell_tiles(rc.n_exc, s.plan.n_lo, s.plan.n_hi, s.plan.a_lo, s.plan.a_hi,
+                                       128 * kShardCells<R>);
+    const u32 grid = total_tiles(tiles);
     const i64 mark = sim.pre_steps() == 0 ? 0 : sim.pre_steps() - 1;
     if (grid == 0) return Status::Ok();
-    constexpr int MB = std::is_same<R, float>::value ? 6 : 4;
+    constexpr int MB = std::is_same<R, float>::value ? 5 : 4;
+    const CellTiles draws = event_tiles(rc.n_exc, s.plan.n_lo, s.plan.n_hi, 256, 2);
+    if (total_tiles(draws)) {
+        shard_draw_kernel<<<total_tiles(draws), 256, poisson_bytes(2, ws.W, 256), sim.stream()>>>(
+            net_scalars(rc), w.events, k * ws.W, ws.W, draws);
+        AS_CUDA(cudaGetLastError());
+    }
     shard_window_kernel<R, MB><<<grid, 128, 0, sim.stream()>>>(rc, p, w, k * ws.W, static_cast<int>(k & 1), mark,
-                                                               a_blk0, a_nblk, n_blk0);
+                                                               tiles);
     AS_CUDA(cudaGetLastError());
     return Status::Ok();
 }

@@ -54,10 +54,22 @@ __global__ void fused_step_kernel(RunConsts rc, StepPtrs<R> p, i64 step, u32 ast
 
 // exp(-lambda) of the Poisson drives and the constant synaptic decays are evaluated
 // on the device, where the reference evaluates them (src/astrosim_fused.cu:167, 515-516).
-__global__ void device_constants_kernel(double la, double le, double li, double* out) {
-    out[0] = exp(-la);
-    out[1] = exp(-le);
-    out[2] = exp(-li);
+struct DeviceConstants {
+    double limit_astro, limit_exc, limit_inh;
+    double decay[2][2];   // [population][excitatory, inhibitory conductance]
+    float f_decay[2][2];
+};
+__global__ void device_constants_kernel(RunConsts rc, DeviceConstants* out) {
+    out->limit_astro = exp(-rc.lambda_astro);
+    out->limit_exc = exp(-rc.lambda_exc);
+    out->limit_inh = exp(-rc.lambda_inh);
+    for (int i = 0; i < 2; ++i) {
+        const NeuronK& k = i == 0 ? rc.pe : rc.pi;
+        out->decay[i][0] = exp_r(-rc.h_step / k.tau_syn_ex);
+        out->decay[i][1] = exp_r(-rc.h_step / k.tau_syn_in);
+        out->f_decay[i][0] = exp_r(-rc.f_h_step / static_cast<float>(k.tau_syn_ex));
+        out->f_decay[i][1] = exp_r(-rc.f_h_step / static_cast<float>(k.tau_syn_in));
+    }
 }
 
 template <typename R>
@@ -107,6 +119,35 @@ void fill_stage_constants(RunConsts& rc) {
     rc.f_weight_exc = static_cast<float>(rc.weight_exc);
     rc.f_weight_inh = static_cast<float>(rc.weight_inh);
     rc.f_noise_astro = static_cast<float>(rc.noise_astro);
+    auto twice = [](float x) {
+        u32 b;
+        std::memcpy(&b, &x, sizeof b);
+        return static_cast<u64>(b) << 32 | b;
+    };
+    for (const bool exc : {true, false}) {
+        const NeuronK& k = exc ? rc.pe : rc.pi;
+        AdexPairK& q = exc ? rc.pair_e : rc.pair_i;
+        q.neg_inv_Cm = twice(-k.f_inv_Cm);
+        q.A0 = twice(k.f_A0);
+        q.Eex_c = twice(k.f_Eex_c);
+        q.Ein_c = twice(k.f_Ein_c);
+        q.neg_E_L = twice(-k.f_E_L);
+        q.neg_V_th = twice(-k.f_V_th);
+        q.K1 = twice(k.f_K1);
+        q.K2 = twice(k.f_K2);
+        q.Wa = twice(k.f_Wa);
+        q.neg_inv_tauw = twice(-k.f_inv_tauw);
+        q.psc_ex = twice(k.f_psc_init_ex);
+        q.psc_in = twice(k.f_psc_init_in);
+        q.ex_decay = twice(k.f_ex_decay);
+        q.in_decay = twice(k.f_in_decay);
+        q.V_peak = k.f_V_peak;
+        q.pad_ = 0.0f;
+    }
+    rc.pair_hs = twice(rc.f_h_step);
+    rc.pair_half_hs = twice(0.5f * rc.f_h_step);
+    rc.pair_h6 = twice(rc.f_h6);
+    rc.pair_pad_ = 0;
     rc.pe.ref_steps = static_cast<int>(rc.pe.t_ref / rc.h_step + 0.5);
     rc.pi.ref_steps = static_cast<int>(rc.pi.t_ref / rc.h_step + 0.5);
 }
@@ -205,19 +246,27 @@ Status Simulation::create(const astrosim_config& cfg, const char* biology_json, 
     rc.words = (sz.n_neurons + 31) / 32;
     fill_stage_constants(rc);
     {
-        DevBuf<double> lim;
-        AS_TRY(lim.alloc(3));
-        device_constants_kernel<<<1, 1, 0, stream_>>>(rc.lambda_astro, rc.lambda_exc, rc.lambda_inh, lim.get());
+        DevBuf<DeviceConstants> dev;
+        AS_TRY(dev.alloc(1));
+        device_constants_kernel<<<1, 1, 0, stream_>>>(rc, dev.get());
         AS_CUDA(cudaGetLastError());
-        double h[3];
-        AS_CUDA(cudaMemcpyAsync(h, lim.get(), sizeof(h), cudaMemcpyDeviceToHost, stream_));
+        DeviceConstants h;
+        AS_CUDA(cudaMemcpyAsync(&h, dev.get(), sizeof(h), cudaMemcpyDeviceToHost, stream_));
         AS_CUDA(cudaStreamSynchronize(stream_));
-        rc.limit_astro = h[0];
-        rc.limit_exc = h[1];
-        rc.limit_inh = h[2];
-        rc.lim53_astro = static_cast<u64>(std::floor(h[0] * 9007199254740992.0));
-        rc.lim53_exc = static_cast<u64>(std::floor(h[1] * 9007199254740992.0));
-        rc.lim53_inh = static_cast<u64>(std::floor(h[2] * 9007199254740992.0));
+        rc.limit_astro = h.limit_astro;
+        rc.limit_exc = h.limit_exc;
+        rc.limit_inh = h.limit_inh;
+        rc.lim53_astro = static_cast<u64>(std::floor(h.limit_astro * 9007199254740992.0));
+        rc.lim53_exc = static_cast<u64>(std::floor(h.limit_exc * 9007199254740992.0));
+        rc.lim53_inh = static_cast<u64>(std::floor(h.limit_inh * 9007199254740992.0));
+        for (int i = 0; i < 2; ++i) {
+            NeuronK& k = i == 0 ? rc.pe : rc.pi;
+            k.ex_decay = h.decay[i][0];
+            k.in_decay = h.decay[i][1];
+            k.f_ex_decay = h.f_decay[i][0];
+            k.f_in_decay = h.f_decay[i][1];
+        }
+        fill_stage_constants(rc);  // the pair copies of the decays
     }
 
     pre_steps_ = static_cast<i64>(cfg.pre_ms / cfg.dt + 0.5);

@@ -125,16 +125,41 @@ __device__ __forceinline__ void astro_advance(const AstroK& c, AstroRegs<R>& s, 
     }
 }
 
+// rng_poisson_at out of line, for the window kernels' rare exact draws: its normal
+// approximation inlines a double log, cos and sqrt that the common step never runs.
+static __device__ __noinline__ int poisson_exact(u64 base, double lambda, double limit, u64 lim53) {
+    return rng_poisson_at(base, lambda, limit, lim53);
+}
+
+// The IP3 input of one astrocyte and step: its delayed spike sum and its background
+// events (src/astrosim_fused.cu:390-401).
+template <typename R>
+__device__ __forceinline__ R astro_kick(const RunConsts& rc, const NetScalars& ns, R gathered, u64 poisson_base) {
+    R ip3_input = as_r<R>(rc.w_n2a, rc.f_w_n2a) * gathered;
+    // an event needs a first draw whose upper part reaches the limit's (see rng_poisson_at)
+    if (ns.lambda_astro > 0.0 && rng_mix_hi(poisson_base) >= static_cast<u32>(ns.lim53_astro >> 21)) {
+        const int ev = poisson_exact(poisson_base, ns.lambda_astro, ns.limit_astro, ns.lim53_astro);
+        if (ev > 0) ip3_input += as_r<R>(rc.weight_astro, rc.f_weight_astro) * static_cast<R>(ev);
+    }
+    return ip3_input;
+}
+
+// SIC factor (src/astrosim_fused.cu:416-417); the threshold test runs on the double Ca
+// in every precision.
+template <typename R>
+__device__ __forceinline__ R sic_factor(const RunConsts& rc, double Ca) {
+    const double y = (Ca - rc.ak.SIC_th) * 1000.0;
+    R factor = static_cast<R>(0.0);
+    if (!(y <= 1.0)) factor = as_r<R>(rc.ak.SIC_scale, rc.ak.f_SIC_scale) * log_r(static_cast<R>(y));
+    return factor;
+}
+
 // Everything astrocyte `a` does in step `step` once its delayed spike sum is known
 // (src/astrosim_fused.cu:390-417): Poisson IP3 drive, noise, RK4, SIC factor.
 template <typename R>
 __device__ __forceinline__ R astro_advance_step(const RunConsts& rc, const NetScalars& ns, AstroRegs<R>& s, R gathered, u32 a, i64 step,
                                                 u64 poisson_base, u64 noise_base) {
-    R ip3_input = as_r<R>(rc.w_n2a, rc.f_w_n2a) * gathered;
-    if (ns.lambda_astro > 0.0) {
-        const int ev = rng_poisson_at(poisson_base, ns.lambda_astro, ns.limit_astro, ns.lim53_astro);
-        if (ev > 0) ip3_input += as_r<R>(rc.weight_astro, rc.f_weight_astro) * static_cast<R>(ev);
-    }
+    const R ip3_input = astro_kick<R>(rc, ns, gathered, poisson_base);
     R noise = static_cast<R>(0.0);
     if (rc.noise_astro > 0.0) {
         u64 base = noise_base;
@@ -151,11 +176,7 @@ __device__ __forceinline__ R astro_advance_step(const RunConsts& rc, const NetSc
     }
     astro_advance<R>(rc.ak, s, ip3_input, noise, as_r<R>(rc.h_step, rc.f_h_step), as_r<R>(rc.h6, rc.f_h6),
                      rc.substeps);
-    // SIC factor (416-417); the threshold test runs on the double Ca in every precision
-    const double y = (s.Ca - rc.ak.SIC_th) * 1000.0;
-    R factor = static_cast<R>(0.0);
-    if (!(y <= 1.0)) factor = as_r<R>(rc.ak.SIC_scale, rc.ak.f_SIC_scale) * log_r(static_cast<R>(y));
-    return factor;
+    return sic_factor<R>(rc, s.Ca);
 }
 
 // Stream bases of a cell's per-step draws (stream = step * 1000003 + cell); the next
@@ -212,38 +233,32 @@ struct AdexStage<float> {
 };
 #endif
 
-// Register-resident state of one neuron.
+// Register-resident state of one neuron.  Its V_reset and b are read where they are
+// used (a spike, a refractory step): most steps of most neurons need neither.
 template <typename R>
 struct NeuronRegs {
-    double V, w, V_reset, b;
+    double V, w;
+    const double *V_reset, *b;
     R g_ex, dg_ex, g_in, dg_in, I_sic;
     int refr;
 };
 
-// Everything neuron j does in step `step` once its delayed sums are known
-// (src/astrosim_fused.cu:465-558): synaptic inputs, Poisson drive, SIC refresh,
-// noise, the alpha-cascade closed form and AdEx RK4 (or the refractory Euler step),
-// the spike test.  `noise` is noise_std * N(0,1) for this step when `has_noise`.
+// The synaptic input of one step once its delayed sum and background events are known
+// (src/astrosim_fused.cu:465-486).
 template <typename R>
-__device__ __forceinline__ bool neuron_advance_step(const RunConsts& rc, const NetScalars& ns, const NeuronK& pk,
-                                                    bool excitatory,
-                                                    NeuronRegs<R>& n, R exc_sum, R inh_sum, bool sic_refresh,
-                                                    R sic_sum, bool has_noise, double noise, u64 poisson_base,
-                                                    R ex_decay, R in_decay) {
+__device__ __forceinline__ R exc_input_of(const RunConsts& rc, bool excitatory, R exc_sum, int events) {
     R exc_input = as_r<R>(rc.w_e, rc.f_w_e) * exc_sum;
-    const R inh_input = as_r<R>(-rc.w_i, rc.f_neg_w_i) * inh_sum;
-    const double lambda = excitatory ? ns.lambda_exc : ns.lambda_inh;
-    if (lambda > 0.0) {
-        const int ev = rng_poisson_at(poisson_base, lambda, excitatory ? ns.limit_exc : ns.limit_inh,
-                                      excitatory ? ns.lim53_exc : ns.lim53_inh);
-        if (ev > 0)
-            exc_input += (excitatory ? as_r<R>(rc.weight_exc, rc.f_weight_exc) : as_r<R>(rc.weight_inh, rc.f_weight_inh)) *
-                         static_cast<R>(ev);
-    }
-    if (sic_refresh) n.I_sic = as_r<R>(ns.w_a2n, ns.f_w_a2n) * sic_sum;
-    R I_ext = n.I_sic;
-    if (has_noise) I_ext += static_cast<R>(noise);
+    if (events > 0)
+        exc_input += (excitatory ? as_r<R>(rc.weight_exc, rc.f_weight_exc) : as_r<R>(rc.weight_inh, rc.f_weight_inh)) *
+                     static_cast<R>(events);
+    return exc_input;
+}
 
+// One step of a neuron's own dynamics (src/astrosim_fused.cu:506-558): the
+// alpha-cascade closed form and AdEx RK4 (or the refractory Euler step), the spike test.
+template <typename R>
+__device__ __forceinline__ bool neuron_ode_step(const RunConsts& rc, const NeuronK& pk, NeuronRegs<R>& n, R exc_input,
+                                                R inh_input, R I_ext, R ex_decay, R in_decay) {
     double V = n.V, w = n.w;
     R g_ex = n.g_ex, dg_ex = n.dg_ex + exc_input * as_r<R>(pk.psc_init_ex, pk.f_psc_init_ex);
     R g_in = n.g_in, dg_in = n.dg_in + inh_input * as_r<R>(pk.psc_init_in, pk.f_psc_init_in);
@@ -257,7 +272,7 @@ __device__ __forceinline__ bool neuron_advance_step(const RunConsts& rc, const N
         const R g_in_next = in_decay * (g_in + hs * dg_in);
         const R dg_in_next = in_decay * dg_in;
         if (refractory > 0) {
-            V = n.V_reset;
+            V = *n.V_reset;
             R dV, dw;
             const AdexStage<R> r0(pk, g_ex, g_in, I_ext);
             r0(static_cast<R>(V), static_cast<R>(w), dV, dw);
@@ -284,8 +299,8 @@ __device__ __forceinline__ bool neuron_advance_step(const RunConsts& rc, const N
         if (refractory > 0) {
             --refractory;
         } else if (V >= pk.V_peak) {  // threshold test in double
-            V = n.V_reset;
-            w += n.b;
+            V = *n.V_reset;
+            w += *n.b;
             refractory = pk.ref_steps;  // static_cast<int>(t_ref / h_step + 0.5)
             spiked = true;
         }
@@ -364,14 +379,19 @@ __device__ __forceinline__ bool neuron_cell_step(const RunConsts& rc, const NetS
     const double nstd = excitatory ? rc.noise_exc : rc.noise_inh;
     const bool has_noise = nstd > 0.0 && rc.independent_noise;
     const double noise = has_noise ? neuron_noise<R>(ns, nstd, noise_idx, j) : 0.0;
-    NeuronRegs<R> n{p.V[j], p.w[j], p.V_reset[j], p.b[j], p.g_ex[j], p.dg_ex[j], p.g_in[j], p.dg_in[j], p.I_sic[j],
-                    p.refr[j]};
-    const R hs = as_r<R>(rc.h_step, rc.f_h_step);
-    const R ex_decay = exp_r(-hs / static_cast<R>(pk.tau_syn_ex));
-    const R in_decay = exp_r(-hs / static_cast<R>(pk.tau_syn_in));
-    const bool spiked = neuron_advance_step<R>(rc, ns, pk, excitatory, n, exc_sum, inh_sum, sic_refresh, sic_sum,
-                                               has_noise, noise, step_base(ns.seed, kNeuronPoissonKey, step, j),
-                                               ex_decay, in_decay);
+    NeuronRegs<R> n{p.V[j],     p.w[j],     p.V_reset + j, p.b + j, p.g_ex[j],
+                    p.dg_ex[j], p.g_in[j], p.dg_in[j],    p.I_sic[j], p.refr[j]};
+    const R ex_decay = as_r<R>(pk.ex_decay, pk.f_ex_decay), in_decay = as_r<R>(pk.in_decay, pk.f_in_decay);
+    const double lambda = excitatory ? ns.lambda_exc : ns.lambda_inh;
+    int events = 0;
+    if (lambda > 0.0)
+        events = rng_poisson_at(step_base(ns.seed, kNeuronPoissonKey, step, j), lambda,
+                                excitatory ? ns.limit_exc : ns.limit_inh, excitatory ? ns.lim53_exc : ns.lim53_inh);
+    if (sic_refresh) n.I_sic = as_r<R>(ns.w_a2n, ns.f_w_a2n) * sic_sum;
+    R I_ext = n.I_sic;
+    if (has_noise) I_ext += static_cast<R>(noise);
+    const bool spiked = neuron_ode_step<R>(rc, pk, n, exc_input_of<R>(rc, excitatory, exc_sum, events),
+                                           as_r<R>(-rc.w_i, rc.f_neg_w_i) * inh_sum, I_ext, ex_decay, in_decay);
     p.V[j] = n.V;
     p.w[j] = n.w;
     p.g_ex[j] = n.g_ex;

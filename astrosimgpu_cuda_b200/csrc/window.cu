@@ -4,6 +4,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdlib>
 #include <map>
@@ -12,29 +13,56 @@
 #include <type_traits>
 #include <utility>
 
-#include "window_kernels.cuh"
+#include "window_cells.cuh"
 
 namespace astrosim {
 
 namespace {
 
 // Block and MinBlocks are the block size and the launch-bounds occupancy target
-// (resident blocks per SM): the autotuner (window_launch) times the instantiated
+// (resident blocks per SM), Cells the cells per thread: the autotuner (window_launch) times the instantiated
 // pairs on the first windows of a run and keeps the fastest.  The per-cell
 // arithmetic is the same in every instantiation; the kernel indexes cells by
 // blockDim.x, so Block = 1024 with MinBlocks = 1 serves any other block size.
-template <typename R, int Block, int MinBlocks>
+template <typename R, int Block, int MinBlocks, int Cells>
 __global__ void __launch_bounds__(Block, MinBlocks) window_kernel(RunConsts rc, StepPtrs<R> p, WinPtrs<R> w,
                                                                   i64 win_start, int s_begin, int s_end, int buf,
-                                                                  i64 mark, u32 astro_blocks) {
-    const bool astro = blockIdx.x < astro_blocks;
-    window_cells<R>(rc, net_scalars(rc), p, w, win_start, s_begin, s_end, buf, mark, astro ? blockIdx.x : blockIdx.x - astro_blocks,
-                    astro);
+                                                                  i64 mark, CellTiles tiles) {
+    window_cells<R, Cells>(rc, net_scalars(rc), p, w, win_start, s_begin, s_end, buf, mark, tile_of(tiles, blockIdx.x));
 }
 
+// The first push_blocks blocks deliver window `buf`'s spikes; the others draw the
+// background events of the window that starts at next_start (tiles), Cells neurons per
+// thread.  Either part may be absent.  The two touch nothing in common.
+template <typename R, int Block, int Cells>
+__global__ void __launch_bounds__(Block) push_kernel(WinPtrs<R> w, NetScalars ns, int buf, u32 push_blocks,
+                                                     i64 next_start, CellTiles tiles) {
+    extern __shared__ u32 rows[];
+    if (blockIdx.x < push_blocks)
+        push_cells<R>(w, ns.n_exc, ns.n_neurons - ns.n_exc, ns.n_neurons, ns.n_astro, buf, blockIdx.x, push_blocks);
+    else
+        draw_events<Cells>(ns, w.events, next_start, w.W, tile_of(tiles, blockIdx.x - push_blocks), rows);
+}
+
+// Delivers window `buf` (push_warps > 0) and draws the window that starts at next_start
+// (draw).  A network that leaves schedulers idle draws one cell per thread in blocks of
+// two warps, which spreads the draws over more of them (N = 500: with two cells in blocks
+// of eight warps the launch took 8.6 us, of which the draws 7.6); a larger one draws two,
+// which shares a warp's unluckiest lane between more draws (67 instead of 74 warp
+// instructions per warp of cells and step).
 template <typename R>
-__global__ void push_kernel(WinPtrs<R> w, u32 n_exc, u32 n_inh, u64 n_neurons, u64 n_astro, int buf) {
-    push_cells<R>(w, n_exc, n_inh, n_neurons, n_astro, buf, blockIdx.x, gridDim.x);
+cudaError_t launch_push(const WinPtrs<R>& w, const NetScalars& ns, int buf, u32 push_warps, bool draw, i64 next_start,
+                        cudaStream_t st) {
+    const bool spread = ns.n_neurons <= sm_count() * 4 * 32 * 2;
+    const int block = spread ? 64 : 256, cells = spread ? 1 : 2;
+    const CellTiles tiles = event_tiles(ns.n_exc, 0, ns.n_neurons, block, cells);
+    const u32 push_blocks = ceil_div(push_warps * 32, block);
+    const u32 grid = push_blocks + (draw ? total_tiles(tiles) : 0);
+    if (grid == 0) return cudaSuccess;
+    const size_t smem = draw ? poisson_bytes(cells, w.W, block) : 0;
+    if (spread) push_kernel<R, 64, 1><<<grid, block, smem, st>>>(w, ns, buf, push_blocks, next_start, tiles);
+    else push_kernel<R, 256, 2><<<grid, block, smem, st>>>(w, ns, buf, push_blocks, next_start, tiles);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ forward CSRs
@@ -188,22 +216,30 @@ Status window_setup(const RunConsts& rc, Network& net, bool fp32, WindowState& w
     AS_TRY(ws.astro_active.alloc_zero(2 * ((nA + 31) / 32), st));
     AS_TRY(ws.sic_flag.alloc_zero(2 * ((nN + 31) / 32), st));
     AS_TRY(ws.mode.alloc_zero(2, st));
+    AS_TRY(ws.events.alloc(nN));
     AS_CUDA(cudaStreamSynchronize(st));
     return Status::Ok();
 }
 
 namespace {
 
-// Variants the autotuner chooses from: (block size, minimum resident blocks per SM).
-// Each block size comes with three occupancy targets (the same threads per SM as
-// the 128-thread entries), trading registers (and a few spills) for occupancy.
+// Variants the autotuner chooses from: (block size, minimum resident blocks per SM, cells
+// per thread).  The FP32 form comes with two cells per thread at two register budgets, the
+// faster ones for networks that fill the chip, and with one (N = 500: 14.9 us per window
+// against 19.4 with two, whose warps are half as many and longer); the FP64 form with
+// three register budgets.
 struct Variant {
-    int block, min_blocks;
+    int block, min_blocks, cells;
 };
-constexpr Variant kVariantsF32[] = {{128, 6}, {128, 8}, {128, 4}, {64, 12}, {64, 16}, {64, 8},
-                                    {256, 3}, {256, 4}, {256, 2}};
-constexpr Variant kVariantsF64[] = {{128, 4}, {128, 5}, {128, 3}, {64, 8}, {64, 10}, {64, 6},
-                                    {256, 2}, {256, 3}, {256, 1}};
+#ifndef ASTROSIM_FP32_IEEE
+constexpr Variant kVariantsF32[] = {{128, 5, 2}, {128, 6, 2}, {128, 8, 1}, {64, 10, 2}, {64, 12, 2}, {64, 12, 1},
+                                    {256, 2, 2}, {256, 3, 2}, {256, 4, 1}};
+#else
+constexpr Variant kVariantsF32[] = {{128, 6, 1}, {128, 8, 1}, {128, 4, 1}, {64, 12, 1}, {64, 16, 1}, {64, 8, 1},
+                                    {256, 3, 1}, {256, 4, 1}, {256, 2, 1}};
+#endif
+constexpr Variant kVariantsF64[] = {{128, 4, 1}, {128, 5, 1}, {128, 3, 1}, {64, 8, 1}, {64, 10, 1}, {64, 6, 1},
+                                    {256, 2, 1}, {256, 3, 1}, {256, 1, 1}};
 constexpr int kNumVariants = 9;
 constexpr int kVariantsPerBlock = 3;
 constexpr int kTuneRounds = 2;
@@ -232,53 +268,36 @@ void variant_range(int block, int* first, int* count) {
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int> g_tuned;  // (precision, log2 size bucket, requested block) -> variant
 
-template <typename R, int B, int M>
-void launch_one(u32 cells_astro, u32 cells_neuron, cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p,
-                const WinPtrs<R>& w, i64 start, int s0, int s1, int buf, i64 mark, int block) {
-    const u32 astro_blocks = ceil_div(cells_astro, block);
-    const u32 grid = astro_blocks + ceil_div(cells_neuron, block);
-    window_kernel<R, B, M><<<grid, block, 0, st>>>(rc, p, w, start, s0, s1, buf, mark, astro_blocks);
+template <typename R, int B, int M, int C>
+cudaError_t launch_one(cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p, const WinPtrs<R>& w, i64 start,
+                       int s0, int s1, int buf, i64 mark, int block) {
+    const CellTiles tiles = cell_tiles(rc.n_exc, 0, rc.n_neurons, 0, rc.n_astro, static_cast<u32>(block * C));
+    window_kernel<R, B, M, C><<<total_tiles(tiles), block, 0, st>>>(rc, p, w, start, s0, s1, buf, mark, tiles);
+    return cudaGetLastError();
+}
+
+template <typename R>
+using LaunchFn = cudaError_t (*)(cudaStream_t, const RunConsts&, const StepPtrs<R>&, const WinPtrs<R>&, i64, int, int,
+                                 int, i64, int);
+template <typename R, int V>
+constexpr LaunchFn<R> variant_launch() {
+    constexpr Variant v = std::is_same<R, float>::value ? kVariantsF32[V] : kVariantsF64[V];
+    return &launch_one<R, v.block, v.min_blocks, v.cells>;
+}
+template <typename R, int... V>
+constexpr std::array<LaunchFn<R>, sizeof...(V)> variant_launches(std::integer_sequence<int, V...>) {
+    return {variant_launch<R, V>()...};
 }
 
 // Launches variant `variant` (an index into the table; -1 = the generic kernel at
 // `block` threads).
 template <typename R>
-void launch_window(int variant, int block, cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p,
-                   const WinPtrs<R>& w, i64 start, int s0, int s1, int buf, i64 mark) {
-    constexpr bool f32 = std::is_same<R, float>::value;
-    const u32 nA = rc.n_astro, nN = rc.n_neurons;
-#define AS_WIN(B, M) launch_one<R, B, M>(nA, nN, st, rc, p, w, start, s0, s1, buf, mark, B)
-    if (variant < 0) {
-        launch_one<R, 1024, 1>(nA, nN, st, rc, p, w, start, s0, s1, buf, mark, block);
-        return;
-    }
-    const Variant v = f32 ? kVariantsF32[variant] : kVariantsF64[variant];
-    if constexpr (f32) {
-        switch (v.block * 100 + v.min_blocks) {
-            case 12804: AS_WIN(128, 4); break;
-            case 12808: AS_WIN(128, 8); break;
-            case 6412: AS_WIN(64, 12); break;
-            case 6416: AS_WIN(64, 16); break;
-            case 6408: AS_WIN(64, 8); break;
-            case 25603: AS_WIN(256, 3); break;
-            case 25604: AS_WIN(256, 4); break;
-            case 25602: AS_WIN(256, 2); break;
-            default: AS_WIN(128, 6); break;
-        }
-    } else {
-        switch (v.block * 100 + v.min_blocks) {
-            case 12803: AS_WIN(128, 3); break;
-            case 12805: AS_WIN(128, 5); break;
-            case 6408: AS_WIN(64, 8); break;
-            case 6410: AS_WIN(64, 10); break;
-            case 6406: AS_WIN(64, 6); break;
-            case 25602: AS_WIN(256, 2); break;
-            case 25603: AS_WIN(256, 3); break;
-            case 25601: AS_WIN(256, 1); break;
-            default: AS_WIN(128, 4); break;
-        }
-    }
-#undef AS_WIN
+cudaError_t launch_window(int variant, int block, cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p,
+                          const WinPtrs<R>& w, i64 start, int s0, int s1, int buf, i64 mark) {
+    static constexpr auto table = variant_launches<R>(std::make_integer_sequence<int, kNumVariants>());
+    if (variant < 0) return launch_one<R, 1024, 1, 1>(st, rc, p, w, start, s0, s1, buf, mark, block);
+    const Variant v = std::is_same<R, float>::value ? kVariantsF32[variant] : kVariantsF64[variant];
+    return table[variant](st, rc, p, w, start, s0, s1, buf, mark, v.block);
 }
 
 template <typename R>
@@ -288,7 +307,7 @@ Status launch_impl(const RunConsts& rc, StateBuffers& sb, Network& net, WindowSt
     StepPtrs<R> p = make_ptrs<R>(sb, net, rc, raster_steps);
     WinPtrs<R> w = win_ptrs<R>(ws, rc);
     const int W = ws.W;
-    const u32 push_blocks = std::max<u32>(1, std::min<u32>(sm_count() * 8, ceil_div(ws.push_limit, 8)));
+    const u32 push_warps = std::max<u32>(8, std::min<u32>(sm_count() * 64, ws.push_limit));
     int v_first = 0, v_count = 0;
     variant_range(block, &v_first, &v_count);
     if (v_first < 0) ws.variant = -2;  // a block size outside the table: the generic kernel, nothing to tune
@@ -304,8 +323,15 @@ Status launch_impl(const RunConsts& rc, StateBuffers& sb, Network& net, WindowSt
             if (it != g_tuned.end()) ws.variant = it->second;
         }
     }
+    const NetScalars ns = net_scalars(rc);
+    auto push_and_draw = [&](int buf, u32 warps, bool draw, i64 next) -> Status {
+        AS_CUDA(launch_push<R>(w, ns, buf, warps, draw, next * W, st));
+        if (draw) ws.events_window = next;
+        return Status::Ok();
+    };
     i64 t = first;
     const i64 end = first + count;
+    if (ws.events_window != first / W) AS_TRY(push_and_draw(0, 0, true, first / W));
     while (t < end) {
         const i64 k = t / W;
         const int s0 = static_cast<int>(t - k * W);
@@ -319,8 +345,7 @@ Status launch_impl(const RunConsts& rc, StateBuffers& sb, Network& net, WindowSt
             AS_CUDA(cudaEventCreate(&ws.tune_ev[1]));
         }
         if (tuning) AS_CUDA(cudaEventRecord(ws.tune_ev[0], st));
-        launch_window<R>(v, block, st, rc, p, w, k * W, s0, s1, buf, mark);
-        AS_CUDA(cudaGetLastError());
+        AS_CUDA(launch_window<R>(v, block, st, rc, p, w, k * W, s0, s1, buf, mark));
         if (tuning) {
             AS_CUDA(cudaEventRecord(ws.tune_ev[1], st));
             AS_CUDA(cudaEventSynchronize(ws.tune_ev[1]));
@@ -337,10 +362,7 @@ Status launch_impl(const RunConsts& rc, StateBuffers& sb, Network& net, WindowSt
                 g_tuned[key] = best;
             }
         }
-        if (s1 == W) {
-            push_kernel<R><<<push_blocks, 256, 0, st>>>(w, rc.n_exc, net.sz.n_inh, rc.n_neurons, rc.n_astro, buf);
-            AS_CUDA(cudaGetLastError());
-        }
+        if (s1 == W) AS_TRY(push_and_draw(buf, push_warps, (k + 1) * W < end, k + 1));
         t = k * W + s1;
     }
     return Status::Ok();

@@ -17,6 +17,8 @@
 // neurons that the push flagged: those whose a2n row holds an astrocyte that was
 // active (the push walks each active astrocyte's forward a2n list), so a window
 // without active astrocytes costs every other neuron one flag-word read.
+// The launch that pushes a window's spikes also draws the next window's background events
+// (poisson_window.cuh).
 #pragma once
 
 #include "common.cuh"
@@ -58,6 +60,8 @@ struct WindowState {
     DevBuf<u32> astro_active;                 // [2][ceil(n_astro / 32)]
     DevBuf<u32> sic_flag;                     // [2][ceil(n_neurons / 32)]: a2n row holds an active astrocyte
     DevBuf<int> mode;                         // [2]: 0 push, 1 pull
+    DevBuf<u64> events;                       // background event counts of one window (poisson_window.cuh)
+    i64 events_window = -1;                   // the window whose counts `events` holds (single-network engine)
     // autotuner: (block size, launch bounds) variant of window_kernel, an index into
     // its table; -1 while timing the candidates, -2 for the generic kernel (a block
     // size outside the table, nothing to tune)

@@ -2,6 +2,7 @@
 // single-network kernels (window.cu) and the batched ensemble kernels (ensemble.cu).
 #pragma once
 
+#include "poisson_window.cuh"
 #include "step_kernels.cuh"
 #include "window.cuh"
 
@@ -19,6 +20,7 @@ struct WinPtrs {
     u32* astro_active;               // [2][astro_words]
     u32* sic_flag;                   // [2][neuron_words]
     int* mode;                       // [2]
+    u64* events;                     // [n_neurons]
     const u32 *fe_rs, *fe_dst, *fi_rs, *fi_dst, *fa_rs, *fa_astro, *fa_pos, *fs_rs, *fs_dst;
     u32 cap, push_limit, astro_words, neuron_words;
     int W;
@@ -39,6 +41,7 @@ inline WinPtrs<R> win_ptrs(WindowState& ws, const RunConsts& rc) {
     w.astro_active = ws.astro_active.get();
     w.sic_flag = ws.sic_flag.get();
     w.mode = ws.mode.get();
+    w.events = ws.events.get();
     w.fe_rs = ws.fwd.exc_rs.get();
     w.fe_dst = ws.fwd.exc_dst.get();
     w.fi_rs = ws.fwd.inh_rs.get();
@@ -92,29 +95,96 @@ __device__ __forceinline__ void pull_row(const u32* __restrict__ rs, const u32* 
     }
 }
 
-// Neuron j through steps [s_begin, s_end) of the window starting at win_start.
-template <typename R, bool EXC>
-__device__ __forceinline__ void neuron_window(const RunConsts& rc, const NetScalars& ns, const NeuronK& pk,
-                                              const StepPtrs<R>& p,
-                                              const WinPtrs<R>& w, u32 j, i64 win_start, int s_begin, int s_end,
-                                              int buf, bool pull, bool window_done) {
+// The steps of a window at which something besides the cells' own dynamics happens:
+// bit s of `refresh` when the SIC current is refreshed ((t - d_a2n) >= 0 and
+// (t - d_a2n) % sic_interval == 0), bit s of `noise` when a new noise index starts
+// (t / steps_per_noise; src/astrosim_fused.cu:1046-1050), and the index at s_begin.
+struct WindowSchedule {
+    u32 refresh, noise;
+    u64 noise_idx;
+};
+
+__device__ __forceinline__ WindowSchedule window_schedule(const RunConsts& rc, i64 win_start, int s_begin, int s_end) {
+    WindowSchedule w{0, 0, 0};
+    const i64 t0 = win_start + s_begin;
+    const int si = rc.sic_interval, spn = rc.steps_per_noise, n = s_end - s_begin;
+    // steps of the first refresh and of the first new noise index, counted from t0
+    int first = 0, fresh;
+    if (t0 < (i64(1) << 31)) {  // 32-bit division: a few instructions instead of a call
+        const u32 t = static_cast<u32>(t0);
+        w.noise_idx = t / static_cast<u32>(spn);
+        fresh = spn - static_cast<int>(t % static_cast<u32>(spn));
+        if (t0 < rc.d_a2n) first = rc.d_a2n - static_cast<int>(t0);
+        else if (si > 1) first = (si - static_cast<int>((t - static_cast<u32>(rc.d_a2n)) % static_cast<u32>(si))) % si;
+    } else {
+        w.noise_idx = static_cast<u64>(t0 / spn);
+        fresh = spn - static_cast<int>(t0 % spn);
+        if (si > 1) first = (si - static_cast<int>((t0 - rc.d_a2n) % si)) % si;
+    }
+    if (si == 1) {
+        if (first < n) w.refresh = (1u << n) - (1u << first);
+    } else {
+        for (int i = first; i < n; i += si) w.refresh |= 1u << i;
+    }
+    for (int i = fresh; i < n; i += spn) w.noise |= 1u << i;
+    w.refresh <<= s_begin;
+    w.noise <<= s_begin;
+    return w;
+}
+
+// The synaptic input of one neuron over a window: excitatory and inhibitory sums of the
+// steps whose bit is set in `mask` (the others have none), and the SIC sums when `sic`.
+template <typename R>
+struct WindowInput {
+    R ex[kMaxWindow], in[kMaxWindow], sic_sum[kMaxWindow];
+    u32 mask;
+    bool sic;
+};
+
+// What says whether a neuron has any input at all.  It is loaded with the state at the
+// window's start and the first deposit (the usual neuron with input has one) right after
+// the noise draw, so that neither load is waited for on its own.
+struct InboxState {
+    u32 count, flags;  // deposits; the word of SIC flags that holds the neuron's
+};
+template <typename R>
+__device__ __forceinline__ InboxState inbox_state(const NetScalars& ns, const WinPtrs<R>& w, u32 j, int buf) {
+    return InboxState{w.nin_cnt[static_cast<u64>(buf) * ns.n_neurons + j],
+                      w.sic_flag[static_cast<u64>(buf) * w.neuron_words + (j >> 5)]};
+}
+template <typename R>
+__device__ __forceinline__ Deposit<R> first_deposit(const NetScalars& ns, const WinPtrs<R>& w, u32 j, int buf,
+                                                    const InboxState& inbox) {
+    Deposit<R> d{0, 0, static_cast<R>(0.0)};
+    if (inbox.count) d = w.nin_ent[(static_cast<u64>(buf) * ns.n_neurons + j) * kInboxSlots];
+    return d;
+}
+
+template <typename R>
+__device__ __forceinline__ void window_input(const NetScalars& ns, const StepPtrs<R>& p, const WinPtrs<R>& w, u32 j,
+                                             const InboxState& inbox, const Deposit<R>& first, int s_begin, int s_end,
+                                             int buf, bool pull, bool window_done, WindowInput<R>& x) {
     const int prev = buf ^ 1;
     const int W = w.W;
     const u64 nN = ns.n_neurons;
-
-    // synaptic input of the window: deposits (push) or the row walk (pull); steps
-    // whose bit in ex_mask / in_mask is clear have none (+0.0)
-    R ex_acc[kMaxWindow], in_acc[kMaxWindow];
-    u32 ex_mask = 0, in_mask = 0;
+    x.mask = 0;
+    // deposits (push) or the row walk (pull)
     const u64 slot_base = static_cast<u64>(buf) * nN + j;
-    const u32 c = w.nin_cnt[slot_base];
+    const u32 c = inbox.count;
     if (pull || c > kInboxSlots) {
-        for (int i = 0; i < W; ++i) ex_acc[i] = in_acc[i] = static_cast<R>(0.0);
-        ex_mask = in_mask = (1u << W) - 1u;
+        for (int i = 0; i < W; ++i) x.ex[i] = x.in[i] = static_cast<R>(0.0);
+        x.mask = (1u << W) - 1u;
         const u32* words = w.spk_word + static_cast<u64>(prev) * nN;
         const R* vals = w.spk_val + static_cast<u64>(prev) * W * nN;
-        pull_row<R>(p.exc_rs, p.exc_src, j, words, vals, nN, s_begin, s_end, ex_acc);
-        pull_row<R>(p.inh_rs, p.inh_src, j, words, vals, nN, s_begin, s_end, in_acc);
+        pull_row<R>(p.exc_rs, p.exc_src, j, words, vals, nN, s_begin, s_end, x.ex);
+        pull_row<R>(p.inh_rs, p.inh_src, j, words, vals, nN, s_begin, s_end, x.in);
+    } else if (c == 1) {  // the usual case: nothing to sort or sum
+        const int st = static_cast<int>(first.meta & 0xFFu);
+        if (st >= s_begin && st < s_end) {
+            x.ex[st] = (first.meta >> 8) == 0 ? first.val : static_cast<R>(0.0);
+            x.in[st] = (first.meta >> 8) == 0 ? static_cast<R>(0.0) : first.val;
+            x.mask = 1u << st;
+        }
     } else if (c > 0) {
         Deposit<R> d[kInboxSlots];
         for (u32 i = 0; i < c; ++i) d[i] = w.nin_ent[slot_base * kInboxSlots + i];
@@ -123,13 +193,12 @@ __device__ __forceinline__ void neuron_window(const RunConsts& rc, const NetScal
             const int st = static_cast<int>(d[i].meta & 0xFFu);
             if (st < s_begin || st >= s_end) continue;
             const u32 bit = 1u << st;
-            if ((d[i].meta >> 8) == 0) {
-                ex_acc[st] = ((ex_mask & bit) ? ex_acc[st] : static_cast<R>(0.0)) + d[i].val;
-                ex_mask |= bit;
-            } else {
-                in_acc[st] = ((in_mask & bit) ? in_acc[st] : static_cast<R>(0.0)) + d[i].val;
-                in_mask |= bit;
+            if (!(x.mask & bit)) {
+                x.ex[st] = x.in[st] = static_cast<R>(0.0);
+                x.mask |= bit;
             }
+            if ((d[i].meta >> 8) == 0) x.ex[st] += d[i].val;
+            else x.in[st] += d[i].val;
         }
     }
     if (window_done && c) w.nin_cnt[slot_base] = 0;
@@ -137,71 +206,101 @@ __device__ __forceinline__ void neuron_window(const RunConsts& rc, const NetScal
     // SIC factors of the previous window through the active-astrocyte bitmask, for a
     // neuron the push flagged (its a2n row holds an astrocyte that was active); for
     // the others every factor in the row is 0, the same as the walk would find
-    R sic_acc[kMaxWindow];
-    bool sic_input = false;
-    u32* flag_word = w.sic_flag + static_cast<u64>(buf) * w.neuron_words + (j >> 5);
+    x.sic = false;
     const u32 flag_bit = 1u << (j & 31);
-    if (*flag_word & flag_bit) {
-        if (window_done) atomicAnd(flag_word, ~flag_bit);  // clean for the window after next
+    if (inbox.flags & flag_bit) {
+        if (window_done)  // clean for the window after next
+            atomicAnd(w.sic_flag + static_cast<u64>(buf) * w.neuron_words + (j >> 5), ~flag_bit);
         const u32* act = w.astro_active + static_cast<u64>(prev) * w.astro_words;
         const R* fac = w.sic_win + static_cast<u64>(prev) * ns.n_astro * W;
         const u32 k1 = p.sic_rs[j + 1];
         for (u32 k = p.sic_rs[j]; k < k1; ++k) {
             const u32 a = p.sic_src[k];
             if (!((act[a >> 5] >> (a & 31)) & 1u)) continue;  // every factor of this astrocyte was 0
-            if (!sic_input) {
-                for (int i = 0; i < W; ++i) sic_acc[i] = static_cast<R>(0.0);
-                sic_input = true;
+            if (!x.sic) {
+                for (int i = 0; i < W; ++i) x.sic_sum[i] = static_cast<R>(0.0);
+                x.sic = true;
             }
             const R* f = fac + static_cast<u64>(a) * W;
-            for (int st = s_begin; st < s_end; ++st) sic_acc[st] += f[st];
+            for (int st = s_begin; st < s_end; ++st) x.sic_sum[st] += f[st];
         }
     }
+}
 
-    NeuronRegs<R> n{p.V[j], p.w[j], p.V_reset[j], p.b[j], p.g_ex[j], p.dg_ex[j], p.g_in[j], p.dg_in[j], p.I_sic[j],
-                    p.refr[j]};
-    const R hs = as_r<R>(rc.h_step, rc.f_h_step);
-    const R ex_decay = exp_r(-hs / static_cast<R>(pk.tau_syn_ex));
-    const R in_decay = exp_r(-hs / static_cast<R>(pk.tau_syn_in));
+// What a spike of neuron j at window step st leaves behind: its synaptic multiplier, a
+// spike-list entry, its step's count and its raster bit.
+template <typename R>
+__device__ __forceinline__ void record_spike(const RunConsts& rc, const NetScalars& ns, const StepPtrs<R>& p,
+                                             const WinPtrs<R>& w, u32 j, i64 win_start, int st, int buf) {
+    const u64 nN = ns.n_neurons;
+    const i64 t = win_start + st;
+    const R out = stp_on_spike<R>(rc, p.stp_x[j], p.stp_u[j], p.stp_t[j], t);
+    w.spk_val[(static_cast<u64>(buf) * w.W + st) * nN + j] = out;
+    const u32 slot = atomicAdd(&w.spk_count[buf], 1u);
+    if (slot < w.cap) w.spk_list[static_cast<u64>(buf) * w.cap + slot] = (j << 5) | static_cast<u32>(st);
+    atomicAdd(&p.counts[t], 1u);
+    if (t < p.raster_steps) atomicOr(&p.raster[static_cast<u64>(t) * ns.words + (j >> 5)], 1u << (j & 31));
+}
+
+// Neuron j through steps [s_begin, s_end) of the window starting at win_start.  Steps at which anything but the
+// cell's own dynamics and its background events happens (a deposit, a SIC refresh that
+// changes the current, new noise, an exact Poisson draw) are rare and marked in
+// `special`, so that the common step reads its event count and integrates.
+template <typename R, bool EXC>
+__device__ __forceinline__ void neuron_window(const RunConsts& rc, const NetScalars& ns, const NeuronK& pk,
+                                              const StepPtrs<R>& p,
+                                              const WinPtrs<R>& w, u32 j, i64 win_start, int s_begin, int s_end,
+                                              int buf, bool window_done) {
+    const u64 nN = ns.n_neurons;
+    const InboxState inbox = inbox_state<R>(ns, w, j, buf);
+    const int pull = w.mode[buf];
+    NeuronRegs<R> n{p.V[j],     p.w[j],     p.V_reset + j, p.b + j, p.g_ex[j],
+                    p.dg_ex[j], p.g_in[j], p.dg_in[j],    p.I_sic[j], p.refr[j]};
+    const R I_sic0 = n.I_sic;
+    const int refr0 = n.refr;
+    const R ex_decay = as_r<R>(pk.ex_decay, pk.f_ex_decay), in_decay = as_r<R>(pk.in_decay, pk.f_in_decay);
     const double nstd = EXC ? rc.noise_exc : rc.noise_inh;
     const bool has_noise = nstd > 0.0 && rc.independent_noise;
-    // Per-step schedule by counters instead of divisions: the SIC refresh runs when
-    // (t - d_a2n) >= 0 and (t - d_a2n) % sic_interval == 0, the noise index is
-    // t / steps_per_noise (src/astrosim_fused.cu:1046-1050).
-    const i64 t0 = win_start + s_begin;
-    i64 since = t0 - rc.d_a2n;
-    const int si = rc.sic_interval, spn = rc.steps_per_noise;
-    int phase = static_cast<int>(((since % si) + si) % si);
-    u64 nidx = static_cast<u64>(t0 / spn);
-    int nphase = static_cast<int>(t0 % spn);
+    WindowSchedule sched = window_schedule(rc, win_start, s_begin, s_end);
+    const u64 pbase = step_base(ns.seed, kNeuronPoissonKey, win_start + s_begin, j);
+    const double lambda = EXC ? ns.lambda_exc : ns.lambda_inh;
+    const double limit = EXC ? ns.limit_exc : ns.limit_inh;
+    const u64 lim53 = EXC ? ns.lim53_exc : ns.lim53_inh;
+    u64 counts = w.events[j] >> (4 * s_begin);  // four bits per step, this step's lowest
     double noise = 0.0;
-    if (has_noise) noise = neuron_noise<R>(ns, nstd, nidx, j);
-    u64 pbase = step_base(ns.seed, kNeuronPoissonKey, t0, j);
+    if (has_noise) noise = neuron_noise<R>(ns, nstd, sched.noise_idx, j);
+    const Deposit<R> first = first_deposit<R>(ns, w, j, buf, inbox);
+    const u32 exact = exact_steps(counts) << s_begin;
+    WindowInput<R> x;
+    window_input<R>(ns, p, w, j, inbox, first, s_begin, s_end, buf, pull != 0, window_done, x);
+    // a refresh without SIC input sets the current to w_a2n * 0
+    const bool sic_changes = x.sic || n.I_sic != as_r<R>(ns.w_a2n, ns.f_w_a2n) * static_cast<R>(0.0);
+    const u32 special = x.mask | exact | (has_noise ? sched.noise : 0u) | (sic_changes ? sched.refresh : 0u);
+    R I_ext = n.I_sic;
+    if (has_noise) I_ext += static_cast<R>(noise);
     u32 word = 0;
-    R* vout = w.spk_val + static_cast<u64>(buf) * W * nN;
     for (int st = s_begin; st < s_end; ++st) {
-        const i64 t = win_start + st;
-        const bool refresh = since >= 0 && phase == 0;
-        if (has_noise && nphase == 0 && st != s_begin) noise = neuron_noise<R>(ns, nstd, nidx, j);
-        const R zero = static_cast<R>(0.0);
-        const bool spiked = neuron_advance_step<R>(
-            rc, ns, pk, EXC, n, ((ex_mask >> st) & 1u) ? ex_acc[st] : zero, ((in_mask >> st) & 1u) ? in_acc[st] : zero,
-            refresh, sic_input ? sic_acc[st] : zero, has_noise, noise, pbase, ex_decay, in_decay);
-        pbase += kStepAdvance;
-        ++since;
-        if (++phase == si) phase = 0;
-        if (++nphase == spn) {
-            nphase = 0;
-            ++nidx;
+        R exc_sum = static_cast<R>(0.0), inh_sum = static_cast<R>(0.0);
+        int events = static_cast<int>(counts & kExactCount);
+        counts >>= 4;
+        if ((special >> st) & 1u) {
+            if ((x.mask >> st) & 1u) {
+                exc_sum = x.ex[st];
+                inh_sum = x.in[st];
+            }
+            if ((exact >> st) & 1u)
+                events = poisson_exact(pbase + static_cast<u64>(st - s_begin) * kStepAdvance, lambda, limit, lim53);
+            if ((sched.refresh >> st) & 1u)
+                n.I_sic = as_r<R>(ns.w_a2n, ns.f_w_a2n) * (x.sic ? x.sic_sum[st] : static_cast<R>(0.0));
+            if (has_noise && ((sched.noise >> st) & 1u)) noise = neuron_noise<R>(ns, nstd, ++sched.noise_idx, j);
+            I_ext = n.I_sic;
+            if (has_noise) I_ext += static_cast<R>(noise);
         }
+        const bool spiked = neuron_ode_step<R>(rc, pk, n, exc_input_of<R>(rc, EXC, exc_sum, events),
+                                               as_r<R>(-rc.w_i, rc.f_neg_w_i) * inh_sum, I_ext, ex_decay, in_decay);
         if (spiked) {
-            const R out = stp_on_spike<R>(rc, p.stp_x[j], p.stp_u[j], p.stp_t[j], t);
-            vout[static_cast<u64>(st) * nN + j] = out;
+            record_spike<R>(rc, ns, p, w, j, win_start, st, buf);
             word |= 1u << st;
-            const u32 slot = atomicAdd(&w.spk_count[buf], 1u);
-            if (slot < w.cap) w.spk_list[static_cast<u64>(buf) * w.cap + slot] = (j << 5) | static_cast<u32>(st);
-            atomicAdd(&p.counts[t], 1u);
-            if (t < p.raster_steps) atomicOr(&p.raster[static_cast<u64>(t) * ns.words + (j >> 5)], 1u << (j & 31));
         }
     }
     p.V[j] = n.V;
@@ -210,100 +309,156 @@ __device__ __forceinline__ void neuron_window(const RunConsts& rc, const NetScal
     p.dg_ex[j] = n.dg_ex;
     p.g_in[j] = n.g_in;
     p.dg_in[j] = n.dg_in;
-    p.I_sic[j] = n.I_sic;
-    p.refr[j] = n.refr;
-    u32* sw = w.spk_word + slot_base;
+    if (n.I_sic != I_sic0) p.I_sic[j] = n.I_sic;
+    if (n.refr != refr0) p.refr[j] = n.refr;
+    u32* sw = w.spk_word + static_cast<u64>(buf) * nN + j;
     *sw = s_begin == 0 ? word : (*sw | word);
 }
 
-// One block of 128 cells advances through steps [s_begin, s_end) of the window that
-// starts at step win_start (buffer parity buf): block `blk` of the astrocytes when
-// `astro`, else block `blk` of the neurons.
+// A block advances a tile of cells of one population, so that the population's constants
+// are the same for the whole block.  The tiles of a cell range: astrocytes first (their
+// steps are the longest), then the excitatory, then the inhibitory neurons.
+enum CellKind : int { kExcCells = 0, kInhCells = 1, kAstroCells = 2 };
+struct CellTiles {
+    u32 lo[3], hi[3], tiles[3];  // by CellKind
+    u32 tile;
+};
+inline CellTiles cell_tiles(u32 n_exc, u32 n_lo, u32 n_hi, u32 a_lo, u32 a_hi, u32 tile) {
+    CellTiles t{};
+    t.tile = tile;
+    t.lo[kExcCells] = n_lo;
+    t.hi[kExcCells] = n_hi < n_exc ? n_hi : n_exc;
+    t.lo[kInhCells] = n_lo > n_exc ? n_lo : n_exc;
+    t.hi[kInhCells] = n_hi;
+    t.lo[kAstroCells] = a_lo;
+    t.hi[kAstroCells] = a_hi;
+    for (int k = 0; k < 3; ++k) t.tiles[k] = t.hi[k] > t.lo[k] ? ceil_div(t.hi[k] - t.lo[k], tile) : 0;
+    return t;
+}
+inline u32 total_tiles(const CellTiles& t) { return t.tiles[0] + t.tiles[1] + t.tiles[2]; }
+
+struct Tile {
+    int kind;
+    u32 base, end;  // cells [base, min(base + tile, end))
+};
+__device__ __forceinline__ Tile tile_of(const CellTiles& t, u32 blk) {
+    int kind = kAstroCells;
+    if (blk >= t.tiles[kAstroCells]) {
+        blk -= t.tiles[kAstroCells];
+        kind = kExcCells;
+        if (blk >= t.tiles[kExcCells]) {
+            blk -= t.tiles[kExcCells];
+            kind = kInhCells;
+        }
+    }
+    return Tile{kind, t.lo[kind] + blk * t.tile, t.hi[kind]};
+}
+
+// The IP3 input of one astrocyte over a window: the spike sums of the steps whose bit is
+// set in `mask` (the others have none), from its `c` deposits.
 template <typename R>
-__device__ __forceinline__ void window_cells(const RunConsts& rc, const NetScalars& ns, const StepPtrs<R>& p,
-                                             const WinPtrs<R>& w,
-                                             i64 win_start, int s_begin, int s_end, int buf, i64 mark, u32 blk,
-                                             bool astro) {
+struct AstroInput {
+    R sum[kMaxWindow];
+    u32 mask;
+};
+template <typename R>
+__device__ __forceinline__ void astro_input(const NetScalars& ns, const StepPtrs<R>& p, const WinPtrs<R>& w, u32 a, u32 c,
+                                            int s_begin, int s_end, int buf, bool pull, bool window_done,
+                                            AstroInput<R>& x) {
     const int prev = buf ^ 1;
     const int W = w.W;
-    const bool window_done = s_end == W;
-    const bool pull = w.mode[buf] != 0;
-    if (astro) {
-        // ------------------------------------------------------------ astrocytes
-        const u32 a = blk * blockDim.x + threadIdx.x;
-        const bool valid = a < ns.n_astro;
-        bool any_active = false;
-        if (valid) {
-            AstroRegs<R> s = load_astro<R>(p.Ca[a], p.IP3[a], p.h[a], p.Ca_tot[a], p.IP3_0[a], p.tau_IP3[a],
-                                           p.delta_IP3[a]);
-            // per-step IP3 input; steps whose bit in in_mask is clear have none (+0.0)
-            R acc[kMaxWindow];
-            u32 in_mask = 0;
-            const u64 slot_base = (static_cast<u64>(buf) * ns.n_astro + a);
-            const u32 c = w.ain_cnt[slot_base];
-            if (pull || c > kInboxSlots) {
-                for (int i = 0; i < W; ++i) acc[i] = static_cast<R>(0.0);
-                in_mask = (1u << W) - 1u;
-                pull_row<R>(p.e2a_rs, p.e2a_src, a, w.spk_word + static_cast<u64>(prev) * ns.n_neurons,
-                            w.spk_val + static_cast<u64>(prev) * W * ns.n_neurons, ns.n_neurons, s_begin, s_end, acc);
-            } else if (c > 0) {
-                Deposit<R> d[kInboxSlots];
-                for (u32 i = 0; i < c; ++i) d[i] = w.ain_ent[slot_base * kInboxSlots + i];
-                sort_deposits<R>(d, static_cast<int>(c));
-                for (u32 i = 0; i < c; ++i) {
-                    const int st = static_cast<int>(d[i].meta & 0xFFu);
-                    if (st < s_begin || st >= s_end) continue;
-                    const u32 bit = 1u << st;
-                    acc[st] = ((in_mask & bit) ? acc[st] : static_cast<R>(0.0)) + d[i].val;
-                    in_mask |= bit;
-                }
-            }
-            if (window_done && c) w.ain_cnt[slot_base] = 0;
-            unsigned char ever = p.ever_active[a];
-            R* out = w.sic_win + (static_cast<u64>(buf) * ns.n_astro + a) * W;
-            R factor = static_cast<R>(0.0);
-            u64 pbase = step_base(ns.seed, kAstroPoissonKey, win_start + s_begin, a);
-            u64 nbase = step_base(ns.seed, kAstroNoiseKey, win_start + s_begin, a);
-            // recording phase (t + 1) % rec_every, advanced by a counter
-            i64 rphase = p.ca_rec ? (win_start + s_begin + 1) % p.rec_every : 1;
-            for (int st = s_begin; st < s_end; ++st) {
-                const i64 t = win_start + st;
-                factor = astro_advance_step<R>(rc, ns, s, ((in_mask >> st) & 1u) ? acc[st] : static_cast<R>(0.0), a, t,
-                                               pbase, nbase);
-                pbase += kStepAdvance;
-                nbase += kStepAdvance;
-                if (p.ca_rec) {
-                    record_ca<R>(p, a, t, rphase == 0, s.Ca);
-                    if (++rphase == p.rec_every) rphase = 0;
-                }
-                out[st] = factor;
-                if (factor > static_cast<R>(0.0)) {
-                    ever = 1;
-                    any_active = true;
-                }
-                if (t == mark) ever = 0;  // end of the pre-run (src/astrosim_fused.cu:1075)
-            }
-            p.Ca[a] = s.Ca;
-            p.IP3[a] = s.IP3;
-            p.h[a] = s.h;
-            p.ever_active[a] = ever;
-            p.sic_last[a] = factor;
+    x.mask = 0;
+    const u64 slot_base = (static_cast<u64>(buf) * ns.n_astro + a);
+    if (pull || c > kInboxSlots) {
+        for (int i = 0; i < W; ++i) x.sum[i] = static_cast<R>(0.0);
+        x.mask = (1u << W) - 1u;
+        pull_row<R>(p.e2a_rs, p.e2a_src, a, w.spk_word + static_cast<u64>(prev) * ns.n_neurons,
+                    w.spk_val + static_cast<u64>(prev) * W * ns.n_neurons, ns.n_neurons, s_begin, s_end, x.sum);
+    } else if (c > 0) {
+        Deposit<R> d[kInboxSlots];
+        for (u32 i = 0; i < c; ++i) d[i] = w.ain_ent[slot_base * kInboxSlots + i];
+        sort_deposits<R>(d, static_cast<int>(c));
+        for (u32 i = 0; i < c; ++i) {
+            const int st = static_cast<int>(d[i].meta & 0xFFu);
+            if (st < s_begin || st >= s_end) continue;
+            const u32 bit = 1u << st;
+            x.sum[st] = ((x.mask & bit) ? x.sum[st] : static_cast<R>(0.0)) + d[i].val;
+            x.mask |= bit;
         }
-        const unsigned ballot = __ballot_sync(0xffffffffu, any_active);
-        if ((threadIdx.x & 31) == 0 && a < ns.n_astro) {
-            u32* word = w.astro_active + static_cast<u64>(buf) * w.astro_words + (a >> 5);
-            if (s_begin == 0) *word = ballot; else if (ballot) atomicOr(word, ballot);
-        }
-        return;
     }
-    // ---------------------------------------------------------------- neurons
-    const u32 j = blk * blockDim.x + threadIdx.x;
-    if (j >= ns.n_neurons) return;
-    // one instantiation per population, so its constants are compile-time operands
-    if (j < ns.n_exc)
-        neuron_window<R, true>(rc, ns, rc.pe, p, w, j, win_start, s_begin, s_end, buf, pull, window_done);
-    else
-        neuron_window<R, false>(rc, ns, rc.pi, p, w, j, win_start, s_begin, s_end, buf, pull, window_done);
+    if (window_done && c) w.ain_cnt[slot_base] = 0;
+}
+
+// The SIC factors of one astrocyte over a window.  A window's factors are read only for
+// astrocytes marked active in it, so they are written only from the first positive one
+// on (the steps before it as zeros); the second part of a split window continues what
+// the first part marked.
+template <typename R>
+struct SicWriter {
+    R* out;
+    R last;
+    unsigned char ever, ever_in;
+    bool writing, any;
+    __device__ __forceinline__ SicWriter(const StepPtrs<R>& p, const WinPtrs<R>& w, const NetScalars& ns, u32 a,
+                                         int buf, int s_begin)
+        : out(w.sic_win + (static_cast<u64>(buf) * ns.n_astro + a) * w.W), last(static_cast<R>(0.0)),
+          ever(p.ever_active[a]), ever_in(ever), writing(false), any(false) {
+        if (s_begin > 0)
+            writing = (w.astro_active[static_cast<u64>(buf) * w.astro_words + (a >> 5)] >> (a & 31)) & 1u;
+    }
+    // Step st's factor; `mark`: the pre-run ends here (src/astrosim_fused.cu:1075).
+    __device__ __forceinline__ void step(int st, R factor, bool mark, bool store) {
+        last = factor;
+        if (factor > static_cast<R>(0.0)) {
+            ever = 1;
+            any = true;
+            if (!writing && store)
+                for (int i = 0; i < st; ++i) out[i] = static_cast<R>(0.0);
+            writing = true;
+        }
+        if (writing && store) out[st] = factor;
+        if (mark) ever = 0;
+    }
+    __device__ __forceinline__ void finish(const StepPtrs<R>& p, u32 a) const {
+        if (ever != ever_in) p.ever_active[a] = ever;
+        p.sic_last[a] = last;
+    }
+};
+
+// Astrocyte a through steps [s_begin, s_end) of the window; returns whether its SIC
+// factor was positive at any of them.
+template <typename R>
+__device__ __forceinline__ bool astro_window(const RunConsts& rc, const NetScalars& ns, const StepPtrs<R>& p,
+                                             const WinPtrs<R>& w, u32 a, i64 win_start, int s_begin, int s_end,
+                                             int buf, i64 mark, bool window_done) {
+    const u32 deposits = w.ain_cnt[static_cast<u64>(buf) * ns.n_astro + a];
+    const int pull = w.mode[buf];
+    AstroRegs<R> s =
+        load_astro<R>(p.Ca[a], p.IP3[a], p.h[a], p.Ca_tot[a], p.IP3_0[a], p.tau_IP3[a], p.delta_IP3[a]);
+    SicWriter<R> out(p, w, ns, a, buf, s_begin);
+    AstroInput<R> x;
+    astro_input<R>(ns, p, w, a, deposits, s_begin, s_end, buf, pull != 0, window_done, x);
+    u64 pbase = step_base(ns.seed, kAstroPoissonKey, win_start + s_begin, a);
+    u64 nbase = step_base(ns.seed, kAstroNoiseKey, win_start + s_begin, a);
+    // recording phase (t + 1) % rec_every, advanced by a counter
+    i64 rphase = p.ca_rec ? (win_start + s_begin + 1) % p.rec_every : 1;
+    for (int st = s_begin; st < s_end; ++st) {
+        const i64 t = win_start + st;
+        const R factor = astro_advance_step<R>(rc, ns, s, ((x.mask >> st) & 1u) ? x.sum[st] : static_cast<R>(0.0), a,
+                                               t, pbase, nbase);
+        pbase += kStepAdvance;
+        nbase += kStepAdvance;
+        if (p.ca_rec) {
+            record_ca<R>(p, a, t, rphase == 0, s.Ca);
+            if (++rphase == p.rec_every) rphase = 0;
+        }
+        out.step(st, factor, t == mark, true);
+    }
+    p.Ca[a] = s.Ca;
+    p.IP3[a] = s.IP3;
+    p.h[a] = s.h;
+    out.finish(p, a);
+    return out.any;
 }
 
 // After window `buf` completes: flag the neurons whose a2n rows hold an astrocyte
@@ -326,14 +481,21 @@ __device__ __forceinline__ void push_cells(const WinPtrs<R>& w, u32 n_exc, u32 n
     const u32 lane = threadIdx.x & 31;
     const u64 warp = (static_cast<u64>(blk) * blockDim.x + threadIdx.x) >> 5;
     const u64 n_warps = (static_cast<u64>(n_blk) * blockDim.x) >> 5;
-    {
-        // a warp per active astrocyte: flag its a2n targets for the next window
-        const u32* act = w.astro_active + static_cast<u64>(buf) * w.astro_words;
-        u32* flags = w.sic_flag + static_cast<u64>(nxt) * w.neuron_words;
-        for (u64 wd = warp; wd < w.astro_words; wd += n_warps) {
-            u32 bits = act[wd];
+    // A warp takes one item at a time: first the words of active astrocytes, then each
+    // spike's excitatory, n2a and inhibitory targets as three items.  The items of a
+    // spike go to different warps, because each is a chain of four dependent accesses and
+    // a small network has warps to spare (N = 500: one warp for all three took 7.8k
+    // cycles).
+    const u32* act = w.astro_active + static_cast<u64>(buf) * w.astro_words;
+    u32* flags = w.sic_flag + static_cast<u64>(nxt) * w.neuron_words;
+    const R* vals = w.spk_val + static_cast<u64>(buf) * w.W * n_neurons;
+    const u64 items = w.astro_words + (busy ? 0 : 3 * static_cast<u64>(n));
+    for (u64 item = warp; item < items; item += n_warps) {
+        if (item < w.astro_words) {
+            // flag the a2n targets of the word's active astrocytes for the next window
+            u32 bits = act[item];
             while (bits) {
-                const u32 a = static_cast<u32>(wd * 32) + static_cast<u32>(__ffs(bits) - 1);
+                const u32 a = static_cast<u32>(item * 32) + static_cast<u32>(__ffs(bits) - 1);
                 bits &= bits - 1;
                 for (u32 k = w.fs_rs[a] + lane; k < w.fs_rs[a + 1]; k += 32) {
                     const u32 t = w.fs_dst[k];
@@ -341,22 +503,14 @@ __device__ __forceinline__ void push_cells(const WinPtrs<R>& w, u32 n_exc, u32 n
                     atomicOr(&flags[t >> 5], 1u << (t & 31));
                 }
             }
+            continue;
         }
-    }
-    if (busy) return;
-    const R* vals = w.spk_val + static_cast<u64>(buf) * w.W * n_neurons;
-    for (u64 e = warp; e < n; e += n_warps) {
-        const u32 packed = w.spk_list[static_cast<u64>(buf) * w.cap + e];
+        const u32 e = static_cast<u32>(item - w.astro_words), kind = e % 3;
+        const u32 packed = w.spk_list[static_cast<u64>(buf) * w.cap + e / 3];
         const u32 j = packed >> 5, st = packed & 31u;
         const R v = vals[static_cast<u64>(st) * n_neurons + j];
-        if (j < n_exc) {
-            for (u32 k = w.fe_rs[j] + lane; k < w.fe_rs[j + 1]; k += 32) {
-                const u32 t = w.fe_dst[k];
-                if (t < t_lo || t >= t_hi) continue;
-                const u64 sb = static_cast<u64>(nxt) * n_neurons + t;
-                const u32 slot = atomicAdd(&w.nin_cnt[sb], 1u);
-                if (slot < kInboxSlots) w.nin_ent[sb * kInboxSlots + slot] = Deposit<R>{j, st, v};
-            }
+        if (kind == 1) {
+            if (j >= n_exc) continue;
             for (u32 k = w.fa_rs[j] + lane; k < w.fa_rs[j + 1]; k += 32) {
                 const u32 a = w.fa_astro[k];
                 if (a < a_lo || a >= a_hi) continue;
@@ -364,19 +518,39 @@ __device__ __forceinline__ void push_cells(const WinPtrs<R>& w, u32 n_exc, u32 n
                 const u32 slot = atomicAdd(&w.ain_cnt[sb], 1u);
                 if (slot < kInboxSlots) w.ain_ent[sb * kInboxSlots + slot] = Deposit<R>{w.fa_pos[k], st, v};
             }
+            continue;
         }
         // the inhibitory rows hold local inhibitory ids and read the spike ring by
         // global id (src/astrosim_fused.cu:458-463): neuron j feeds them when j < n_inh
-        if (j < n_inh) {
-            for (u32 k = w.fi_rs[j] + lane; k < w.fi_rs[j + 1]; k += 32) {
-                const u32 t = w.fi_dst[k];
-                if (t < t_lo || t >= t_hi) continue;
-                const u64 sb = static_cast<u64>(nxt) * n_neurons + t;
-                const u32 slot = atomicAdd(&w.nin_cnt[sb], 1u);
-                if (slot < kInboxSlots) w.nin_ent[sb * kInboxSlots + slot] = Deposit<R>{j, st | (1u << 8), v};
-            }
+        const bool inh = kind == 2;
+        if (j >= (inh ? n_inh : n_exc)) continue;
+        const u32* rs = inh ? w.fi_rs : w.fe_rs;
+        const u32* dst = inh ? w.fi_dst : w.fe_dst;
+        const u32 meta = inh ? st | (1u << 8) : st;
+        for (u32 k = rs[j] + lane; k < rs[j + 1]; k += 32) {
+            const u32 t = dst[k];
+            if (t < t_lo || t >= t_hi) continue;
+            const u64 sb = static_cast<u64>(nxt) * n_neurons + t;
+            const u32 slot = atomicAdd(&w.nin_cnt[sb], 1u);
+            if (slot < kInboxSlots) w.nin_ent[sb * kInboxSlots + slot] = Deposit<R>{j, meta, v};
         }
     }
+}
+
+// One block's tile of neurons: the background events of the window that starts at
+// win_start.  `shared`: poisson_bytes of shared memory.
+template <int CELLS>
+__device__ __forceinline__ void draw_events(const NetScalars& ns, u64* events, i64 win_start, int W, const Tile& tile,
+                                            u32* shared) {
+    const u32 j = tile.base + threadIdx.x;
+    if (j >= tile.end) return;
+    const bool exc = tile.kind == kExcCells;
+    poisson_window<CELLS>(ns.seed, win_start, W, j, CELLS == 2 && tile.end - j > blockDim.x, exc ? ns.lambda_exc : ns.lambda_inh,
+                   exc ? ns.lim53_exc : ns.lim53_inh, shared, events);
+}
+// The tiles of the neurons [n_lo, n_hi) for it.
+inline CellTiles event_tiles(u32 n_exc, u32 n_lo, u32 n_hi, int block, int cells) {
+    return cell_tiles(n_exc, n_lo, n_hi, 0, 0, static_cast<u32>(block * cells));
 }
 
 }  // namespace astrosim
