@@ -11,7 +11,7 @@
 #include <utility>
 
 #include "ensemble.cuh"
-#include "window_cells.cuh"
+#include "window_kernels.cuh"
 
 namespace astrosim {
 
@@ -25,26 +25,20 @@ struct alignas(16) NetDesc {
     i64 mark;  // last step of the pre-run (src/astrosim_fused.cu:1066)
 };
 
-// Variants the autotuner chooses from: (block size, minimum resident blocks per SM, cells
-// per thread).  A tile is block * cells consecutive cells of one population of one
+// Variants the autotuner chooses from: (tile size = block size, minimum resident
+// blocks per SM).  A tile is `tile` consecutive cells of one population of one
 // network; each block stages its network's descriptor once, so larger tiles stage
 // less per cell and smaller tiles balance networks of very different sizes better.
-// One cell per thread suits batches that do not fill the chip (see window.cu).
 struct EnsVariant {
-    int block, min_blocks, cells;
+    int tile, min_blocks;
 };
-#ifndef ASTROSIM_FP32_IEEE
-constexpr EnsVariant kEnsVariantsF32[] = {{128, 5, 2}, {128, 6, 2}, {128, 8, 1}, {64, 10, 2}, {64, 12, 2}, {64, 12, 1},
-                                          {256, 2, 2}, {256, 3, 2}, {256, 4, 1}};
-#else
-constexpr EnsVariant kEnsVariantsF32[] = {{128, 6, 1}, {128, 8, 1}, {128, 4, 1}, {64, 12, 1}, {64, 16, 1}, {64, 8, 1},
-                                          {256, 3, 1}, {256, 4, 1}, {256, 2, 1}};
-#endif
-constexpr EnsVariant kEnsVariantsF64[] = {{128, 4, 1}, {128, 5, 1}, {128, 3, 1}, {64, 8, 1}, {64, 10, 1}, {64, 6, 1},
-                                          {256, 2, 1}, {256, 3, 1}, {256, 1, 1}};
+constexpr EnsVariant kEnsVariantsF32[] = {{128, 6}, {128, 8}, {128, 4}, {64, 12}, {64, 16}, {64, 8},
+                                          {256, 3}, {256, 4}, {256, 2}};
+constexpr EnsVariant kEnsVariantsF64[] = {{128, 4}, {128, 5}, {128, 3}, {64, 8}, {64, 10}, {64, 6},
+                                          {256, 2}, {256, 3}, {256, 1}};
 constexpr int kEnsNumVariants = 9;
-constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256, 512};
-int tile_index(int tile) { return tile == 64 ? 0 : tile == 128 ? 1 : tile == 256 ? 2 : 3; }
+constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256};
+int tile_index(int tile) { return tile == 64 ? 0 : (tile == 256 ? 2 : 1); }
 constexpr int kEnsTuneRounds = 2;
 constexpr int kGraphWindows = 10;
 constexpr u32 kPushBlocksPerNet = 4;
@@ -55,8 +49,8 @@ constexpr u32 kTileIndexMask = (1u << kTileKindShift) - 1;
 // One window of one tile (the cells of one block).  UNI: every network shares the constants
 // outside NetScalars, which then come from the kernel parameters (`common`); otherwise
 // each block also stages its network's full constants (`rcs`) into shared memory.
-template <typename R, int BLOCK, int MB, int CELLS, bool UNI>
-__global__ void __launch_bounds__(BLOCK, MB) ens_window_kernel(RunConsts common, const RunConsts* __restrict__ rcs,
+template <typename R, int TILE, int MB, bool UNI>
+__global__ void __launch_bounds__(TILE, MB) ens_window_kernel(RunConsts common, const RunConsts* __restrict__ rcs,
                                                              const NetDesc<R>* __restrict__ descs,
                                                              const u32* __restrict__ tile_net,
                                                              const u32* __restrict__ tile_blk,
@@ -84,16 +78,17 @@ __global__ void __launch_bounds__(BLOCK, MB) ens_window_kernel(RunConsts common,
     __syncthreads();
     const NetDesc<R>& d = *reinterpret_cast<const NetDesc<R>*>(smem);
     const int s_end = static_cast<int>(end - start < W ? end - start : W);
+    extern __shared__ __align__(16) unsigned char shared[];
     const u32 tb = tile_blk[blockIdx.x];
     const int kind = static_cast<int>(tb >> kTileKindShift);
     const u32 first = kind == kInhCells ? d.ns.n_exc : 0;
     const u32 last = kind == kAstroCells ? d.ns.n_astro : (kind == kExcCells ? d.ns.n_exc : d.ns.n_neurons);
-    const Tile tile{kind, first + (tb & kTileIndexMask) * static_cast<u32>(BLOCK * CELLS), last};
+    const Tile tile{kind, first + (tb & kTileIndexMask) * static_cast<u32>(TILE), last};
     if constexpr (UNI) {
-        window_cells<R, CELLS>(common, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tile);
+        window_cells<R>(common, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tile, shared);
     } else {
         const RunConsts& rc = *reinterpret_cast<const RunConsts*>(smem + kDescBytes);
-        window_cells<R, CELLS>(rc, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tile);
+        window_cells<R>(rc, d.ns, d.p, d.w, start, 0, s_end, static_cast<int>(k & 1), d.mark, tile, shared);
     }
 }
 
@@ -145,18 +140,15 @@ template <typename R, bool UNI, int V>
 void launch_ens_window_v(u32 grid, cudaStream_t st, const RunConsts& common, const RunConsts* rcs, const NetDesc<R>* d,
                          const u32* tn, const u32* tb, const i64* win, const i64* stop, int W) {
     constexpr EnsVariant v = std::is_same<R, float>::value ? kEnsVariantsF32[V] : kEnsVariantsF64[V];
-    ens_window_kernel<R, v.block, v.min_blocks, v.cells, UNI>
-        <<<grid, v.block, 0, st>>>(common, rcs, d, tn, tb, win, stop, W);
+    ens_window_kernel<R, v.tile, v.min_blocks, UNI>
+        <<<grid, v.tile, sic_bytes<R>(W, v.tile), st>>>(common, rcs, d, tn, tb, win, stop, W);
 }
 template <typename R, bool UNI, int... V>
 constexpr std::array<EnsLaunchFn<R>, sizeof...(V)> ens_launches(std::integer_sequence<int, V...>) {
     return {&launch_ens_window_v<R, UNI, V>...};
 }
 
-int variant_tile(bool fp32, int v) {
-    const EnsVariant x = fp32 ? kEnsVariantsF32[v] : kEnsVariantsF64[v];
-    return x.block * x.cells;
-}
+int variant_tile(bool fp32, int v) { return fp32 ? kEnsVariantsF32[v].tile : kEnsVariantsF64[v].tile; }
 
 // One window and its push for every network.
 template <typename R>

@@ -2,8 +2,8 @@
 //
 // Each network keeps its own device state exactly as a single Simulation (its own
 // windowed engine buffers).  One window launch covers every cell of every network:
-// a tile table maps each block (64, 128 or 256 threads with one or two cells each: the
-// autotuner times them) to (network, population, tile), and each block reads its network's descriptor (constants and pointers) into shared memory.
+// a tile table maps each block (a tile of 64, 128 or 256 cells: the autotuner times
+// each size with three occupancy targets) to (network, population, tile), and each block reads its network's descriptor (constants and pointers) into shared memory.
 // The constants that differ between networks (NetScalars) sit in the descriptor;
 // when every network shares the rest (the same biology, dt and substeps) those come
 // from the kernel parameters, else each block also stages its network's full
@@ -20,7 +20,7 @@
 
 namespace astrosim {
 
-constexpr int kNumTileSizes = 4;  // tiles of 64, 128, 256 or 512 cells, chosen by the autotuner
+constexpr int kNumTileSizes = 3;  // tiles of 64, 128 or 256 cells, chosen by the autotuner
 
 class Ensemble {
 public:

@@ -11,7 +11,7 @@
 #include <thread>
 
 #include "shard.cuh"
-#include "window_cells.cuh"
+#include "window_kernels.cuh"
 
 namespace astrosim {
 
@@ -26,19 +26,12 @@ ShardPlan shard_plan(u32 n_neurons, u32 n_astro, int rank, int world) {
 
 namespace {
 
-// Cells per thread: two in the FP32 form (a sharded network fills its GPUs).
-template <typename R>
-constexpr int kShardCells = 1;
-#ifndef ASTROSIM_FP32_IEEE
-template <>
-constexpr int kShardCells<float> = 2;
-#endif
-
 // One window of this rank's cells.
 template <typename R, int MB>
 __global__ void __launch_bounds__(128, MB) shard_window_kernel(RunConsts rc, StepPtrs<R> p, WinPtrs<R> w,
                                                                i64 win_start, int buf, i64 mark, CellTiles tiles) {
-    window_cells<R, kShardCells<R>>(rc, net_scalars(rc), p, w, win_start, 0, w.W, buf, mark, tile_of(tiles, blockIdx.x));
+    extern __shared__ __align__(16) unsigned char shared[];
+    window_cells<R>(rc, net_scalars(rc), p, w, win_start, 0, w.W, buf, mark, tile_of(tiles, blockIdx.x), shared);
 }
 
 // The background events of this rank's neurons in the window that starts at win_start.
@@ -119,18 +112,18 @@ Status window_phase(ShardSim& s, i64 k) {
     StepPtrs<R> p = make_ptrs<R>(sim.state_buffers(), sim.network(), rc, sim.raster_steps());
     WinPtrs<R> w = win_ptrs<R>(ws, rc);
     const CellTiles tiles = cell_tiles(rc.n_exc, s.plan.n_lo, s.plan.n_hi, s.plan.a_lo, s.plan.a_hi,
-                                       128 * kShardCells<R>);
+                                       128);
     const u32 grid = total_tiles(tiles);
     const i64 mark = sim.pre_steps() == 0 ? 0 : sim.pre_steps() - 1;
     if (grid == 0) return Status::Ok();
-    constexpr int MB = std::is_same<R, float>::value ? 5 : 4;
+    constexpr int MB = std::is_same<R, float>::value ? 6 : 4;
     const CellTiles draws = event_tiles(rc.n_exc, s.plan.n_lo, s.plan.n_hi, 256, 2);
     if (total_tiles(draws)) {
         shard_draw_kernel<<<total_tiles(draws), 256, poisson_bytes(2, ws.W, 256), sim.stream()>>>(
             net_scalars(rc), w.events, k * ws.W, ws.W, draws);
         AS_CUDA(cudaGetLastError());
     }
-    shard_window_kernel<R, MB><<<grid, 128, 0, sim.stream()>>>(rc, p, w, k * ws.W, static_cast<int>(k & 1), mark,
+    shard_window_kernel<R, MB><<<grid, 128, sic_bytes<R>(ws.W, 128), sim.stream()>>>(rc, p, w, k * ws.W, static_cast<int>(k & 1), mark,
                                                                tiles);
     AS_CUDA(cudaGetLastError());
     return Status::Ok();

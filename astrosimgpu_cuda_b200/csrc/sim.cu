@@ -119,35 +119,6 @@ void fill_stage_constants(RunConsts& rc) {
     rc.f_weight_exc = static_cast<float>(rc.weight_exc);
     rc.f_weight_inh = static_cast<float>(rc.weight_inh);
     rc.f_noise_astro = static_cast<float>(rc.noise_astro);
-    auto twice = [](float x) {
-        u32 b;
-        std::memcpy(&b, &x, sizeof b);
-        return static_cast<u64>(b) << 32 | b;
-    };
-    for (const bool exc : {true, false}) {
-        const NeuronK& k = exc ? rc.pe : rc.pi;
-        AdexPairK& q = exc ? rc.pair_e : rc.pair_i;
-        q.neg_inv_Cm = twice(-k.f_inv_Cm);
-        q.A0 = twice(k.f_A0);
-        q.Eex_c = twice(k.f_Eex_c);
-        q.Ein_c = twice(k.f_Ein_c);
-        q.neg_E_L = twice(-k.f_E_L);
-        q.neg_V_th = twice(-k.f_V_th);
-        q.K1 = twice(k.f_K1);
-        q.K2 = twice(k.f_K2);
-        q.Wa = twice(k.f_Wa);
-        q.neg_inv_tauw = twice(-k.f_inv_tauw);
-        q.psc_ex = twice(k.f_psc_init_ex);
-        q.psc_in = twice(k.f_psc_init_in);
-        q.ex_decay = twice(k.f_ex_decay);
-        q.in_decay = twice(k.f_in_decay);
-        q.V_peak = k.f_V_peak;
-        q.pad_ = 0.0f;
-    }
-    rc.pair_hs = twice(rc.f_h_step);
-    rc.pair_half_hs = twice(0.5f * rc.f_h_step);
-    rc.pair_h6 = twice(rc.f_h6);
-    rc.pair_pad_ = 0;
     rc.pe.ref_steps = static_cast<int>(rc.pe.t_ref / rc.h_step + 0.5);
     rc.pi.ref_steps = static_cast<int>(rc.pi.t_ref / rc.h_step + 0.5);
 }
@@ -266,7 +237,6 @@ Status Simulation::create(const astrosim_config& cfg, const char* biology_json, 
             k.f_ex_decay = h.f_decay[i][0];
             k.f_in_decay = h.f_decay[i][1];
         }
-        fill_stage_constants(rc);  // the pair copies of the decays
     }
 
     pre_steps_ = static_cast<i64>(cfg.pre_ms / cfg.dt + 0.5);

@@ -11,14 +11,6 @@ namespace astrosim { struct WindowState; }
 
 namespace astrosim {
 
-// The FP32 form's neuron constants with the same float in both halves of a 64-bit word,
-// as the two-cell kernels' f32x2 instructions take them (window_pair.cuh).
-struct AdexPairK {
-    u64 neg_inv_Cm, A0, Eex_c, Ein_c, neg_E_L, neg_V_th, K1, K2, Wa, neg_inv_tauw, psc_ex, psc_in, ex_decay, in_decay;
-    float V_peak, pad_;
-};
-static_assert(sizeof(AdexPairK) == 15 * 8, "AdexPairK has no implicit padding");
-
 // Everything the step kernels read that does not change between steps.
 struct RunConsts {
     AstroK ak;
@@ -46,14 +38,12 @@ struct RunConsts {
     double h6;
     float f_h_step, f_h6, f_w_e, f_neg_w_i, f_w_n2a, f_w_a2n;
     float f_weight_astro, f_weight_exc, f_weight_inh, f_noise_astro;
-    AdexPairK pair_e, pair_i;
-    u64 pair_hs, pair_half_hs, pair_h6, pair_pad_;
 };
 // Every byte of RunConsts is a member (the padding is explicit and zero), so two
 // copies built from the same values compare equal bytewise; the batched engine
 // relies on that to find networks that share their constants.
 static_assert(sizeof(RunConsts) == sizeof(AstroK) + 2 * sizeof(NeuronK) + 2 * 8 + 8 * 4 + 16 * 8 + 3 * 8 + 8 +
-                                       5 * 8 + 4 * 4 + 8 + 10 * 4 + 2 * sizeof(AdexPairK) + 4 * 8,
+                                       5 * 8 + 4 * 4 + 8 + 10 * 4,
               "RunConsts has no implicit padding");
 
 // The run constants that differ between the networks of a batch (seed, sizes,

@@ -5,6 +5,7 @@
 
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "model.cuh"
 #include "sim.cuh"
 
@@ -99,13 +100,11 @@ __device__ __forceinline__ AstroRegs<R> load_astro(double Ca, double IP3, R h, d
     return s;
 }
 
-// One step of the astrocyte ODEs: the IP3 kick, then Li-Rinzel RK4 with clamps
+// One step of the astrocyte ODEs after the IP3 kick: Li-Rinzel RK4 with clamps
 // (src/astrosim_fused.cu:255-278); noise held over the stages.  hs is the substep,
 // h6 = hs / 6.
 template <typename R>
-__device__ __forceinline__ void astro_advance(const AstroK& c, AstroRegs<R>& s, R ip3_input, R noise, R hs, R h6,
-                                              int substeps) {
-    if (ip3_input != static_cast<R>(0.0)) s.IP3 += s.delta_IP3 * static_cast<double>(ip3_input);
+__device__ __forceinline__ void astro_advance(const AstroK& c, AstroRegs<R>& s, R noise, R hs, R h6, int substeps) {
     for (int k = 0; k < substeps; ++k) {
         const R ca = static_cast<R>(s.Ca), ip = static_cast<R>(s.IP3), h = s.h;
         R k1c, k1i, k1h, k2c, k2i, k2h, k3c, k3i, k3h, k4c, k4i, k4h;
@@ -124,6 +123,39 @@ __device__ __forceinline__ void astro_advance(const AstroK& c, AstroRegs<R>& s, 
         s.IP3 = s.IP3 < 0.0 ? 0.0 : s.IP3;
     }
 }
+
+#ifndef ASTROSIM_FP32_IEEE
+// astro_advance for the FP32 form with every rounding written out (they are the ones the
+// compiler chose for the plain expressions): Ca and IP3 share two-float instructions
+// between the right-hand sides.
+__device__ __forceinline__ void astro_advance2(const RunConsts& rc, AstroRegs<float>& s, float noise) {
+    const AstroK& c = rc.ak;
+    const f32x2 hs = both(rc.f_h_step), half_hs = both(0.5f * rc.f_h_step);
+    const float half = 0.5f * rc.f_h_step;
+    int left = rc.substeps;
+    do {
+        auto rhs = [&](f32x2 y, float h, float& dh) {
+            float dCa, dIP3;
+            astro_rhs_fast(c, s.Ct, s.I0, s.tI, s.inv_tI, lo2(y), hi2(y), h, noise, dCa, dIP3, dh);
+            return pack2(dCa, dIP3);
+        };
+        const f32x2 y = pack2(static_cast<float>(s.Ca), static_cast<float>(s.IP3));
+        const float h = s.h;
+        float h1, h2, h3, h4;
+        const f32x2 k1 = rhs(y, h, h1);
+        const f32x2 k2 = rhs(fma2(half_hs, k1, y), fmaf(half, h1, h), h2);
+        const f32x2 k3 = rhs(fma2(half_hs, k2, y), fmaf(half, h2, h), h3);
+        const f32x2 k4 = rhs(fma2(hs, k3, y), fmaf(rc.f_h_step, h3, h), h4);
+        const f32x2 d = rk4_sum(both(rc.f_h6), k1, k2, k3, k4);
+        s.Ca += static_cast<double>(lo2(d));
+        s.IP3 += static_cast<double>(hi2(d));
+        const float hn = fmaf(rc.f_h6, fmaf(2.0f, h3, fmaf(2.0f, h2, h1)) + h4, h);
+        s.Ca = s.Ca < 0.0 ? 0.0 : (s.Ca > s.Ca_tot ? s.Ca_tot : s.Ca);
+        s.h = hn < 0.0f ? 0.0f : (hn > 1.0f ? 1.0f : hn);
+        s.IP3 = s.IP3 < 0.0 ? 0.0 : s.IP3;
+    } while (--left);
+}
+#endif
 
 // rng_poisson_at out of line, for the window kernels' rare exact draws: its normal
 // approximation inlines a double log, cos and sqrt that the common step never runs.
@@ -174,8 +206,12 @@ __device__ __forceinline__ R astro_advance_step(const RunConsts& rc, const NetSc
             noise = rc.noise_astro * (sqrt(-2.0 * log(u1)) * cos(kTwoPi * u2));
         }
     }
-    astro_advance<R>(rc.ak, s, ip3_input, noise, as_r<R>(rc.h_step, rc.f_h_step), as_r<R>(rc.h6, rc.f_h6),
-                     rc.substeps);
+    if (ip3_input != static_cast<R>(0.0)) s.IP3 += s.delta_IP3 * static_cast<double>(ip3_input);
+#ifndef ASTROSIM_FP32_IEEE
+    if constexpr (std::is_same<R, float>::value) astro_advance2(rc, s, noise);
+    else
+#endif
+        astro_advance<R>(rc.ak, s, noise, as_r<R>(rc.h_step, rc.f_h_step), as_r<R>(rc.h6, rc.f_h6), rc.substeps);
     return sic_factor<R>(rc, s.Ca);
 }
 
@@ -314,6 +350,69 @@ __device__ __forceinline__ bool neuron_ode_step(const RunConsts& rc, const Neuro
     n.refr = refractory;
     return spiked;
 }
+
+#ifndef ASTROSIM_FP32_IEEE
+// The FP32 form's neuron between steps: the conductances and their drives as
+// (excitatory, inhibitory) pairs.
+struct NeuronRegs2 {
+    double V, w;
+    f32x2 g, dg;
+    int refr;
+};
+
+// neuron_ode_step for the FP32 form with every rounding written out (they are the ones
+// the compiler chose for the plain expressions).  The two conductances share two-float
+// instructions, and so do V and w between the right-hand sides (N = 1e6: 80 M warp
+// instructions per window instead of 97 M, 95 us instead of 105).  Two cells per thread
+// issue fewer still (61 M) but with half the warps and twice the registers took the same
+// time at N = 1e6 and up to 1.5 times as long at N = 5003.  `iext_c` = C0 + I_ext / C_m.  Returns whether it spiked.
+__device__ __forceinline__ bool neuron_ode_step2(const RunConsts& rc, const NeuronK& pk, NeuronRegs2& n,
+                                                 const double* V_reset, const double* b, f32x2 input, float iext_c) {
+    const f32x2 decay = pack2(pk.f_ex_decay, pk.f_in_decay);
+    const f32x2 hs = both(rc.f_h_step), half_hs = both(0.5f * rc.f_h_step);
+    n.dg = fma2(input, pack2(pk.f_psc_init_ex, pk.f_psc_init_in), n.dg);
+    bool spiked = false;
+    int left = rc.substeps;
+    do {
+        const f32x2 g_next = mul2(decay, fma2(hs, n.dg, n.g));
+        const f32x2 g_mid = mul2(both(0.5f), add2(n.g, g_next));
+        const AdexCoef c1 = adex_coef(pk, lo2(n.g), hi2(n.g), iext_c);
+        if (n.refr > 0) {  // clamped: V at its reset value, w by an Euler step
+            n.V = *V_reset;
+            float dV, dw;
+            adex_rhs_folded(pk, c1, static_cast<float>(n.V), static_cast<float>(n.w), dV, dw);
+            n.w += static_cast<double>(rc.f_h_step * dw);
+            --n.refr;
+        } else {
+            const AdexCoef cm = adex_coef(pk, lo2(g_mid), hi2(g_mid), iext_c);
+            const AdexCoef c4 = adex_coef(pk, lo2(g_next), hi2(g_next), iext_c);
+            auto rhs = [&](const AdexCoef& c, f32x2 y) {
+                float dV, dw;
+                adex_rhs_folded(pk, c, lo2(y), hi2(y), dV, dw);
+                return pack2(dV, dw);
+            };
+            const f32x2 y = pack2(static_cast<float>(n.V), static_cast<float>(n.w));
+            const f32x2 k1 = rhs(c1, y);
+            const f32x2 k2 = rhs(cm, fma2(half_hs, k1, y));
+            const f32x2 k3 = rhs(cm, fma2(half_hs, k2, y));
+            const f32x2 k4 = rhs(c4, fma2(hs, k3, y));
+            const f32x2 d = rk4_sum(both(rc.f_h6), k1, k2, k3, k4);
+            n.V += static_cast<double>(lo2(d));
+            n.w += static_cast<double>(hi2(d));
+            if (n.V >= pk.V_peak) {  // threshold test in double
+                n.V = *V_reset;
+                n.w += *b;
+                n.refr = pk.ref_steps;
+                spiked = true;
+            }
+        }
+        n.g = g_next;
+        n.dg = mul2(decay, n.dg);
+    } while (--left);
+    return spiked;
+}
+
+#endif  // ASTROSIM_FP32_IEEE
 
 // Tsodyks-Markram update of a presynaptic neuron at its spike (src/astrosim_fused.cu:564-579);
 // returns the multiplier its outgoing synapses carry.  Every operation's rounding is

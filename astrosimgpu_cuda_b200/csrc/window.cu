@@ -13,22 +13,23 @@
 #include <type_traits>
 #include <utility>
 
-#include "window_cells.cuh"
+#include "window_kernels.cuh"
 
 namespace astrosim {
 
 namespace {
 
 // Block and MinBlocks are the block size and the launch-bounds occupancy target
-// (resident blocks per SM), Cells the cells per thread: the autotuner (window_launch) times the instantiated
+// (resident blocks per SM): the autotuner (window_launch) times the instantiated
 // pairs on the first windows of a run and keeps the fastest.  The per-cell
 // arithmetic is the same in every instantiation; the kernel indexes cells by
 // blockDim.x, so Block = 1024 with MinBlocks = 1 serves any other block size.
-template <typename R, int Block, int MinBlocks, int Cells>
+template <typename R, int Block, int MinBlocks>
 __global__ void __launch_bounds__(Block, MinBlocks) window_kernel(RunConsts rc, StepPtrs<R> p, WinPtrs<R> w,
                                                                   i64 win_start, int s_begin, int s_end, int buf,
                                                                   i64 mark, CellTiles tiles) {
-    window_cells<R, Cells>(rc, net_scalars(rc), p, w, win_start, s_begin, s_end, buf, mark, tile_of(tiles, blockIdx.x));
+    extern __shared__ __align__(16) unsigned char shared[];
+    window_cells<R>(rc, net_scalars(rc), p, w, win_start, s_begin, s_end, buf, mark, tile_of(tiles, blockIdx.x), shared);
 }
 
 // The first push_blocks blocks deliver window `buf`'s spikes; the others draw the
@@ -74,6 +75,15 @@ __global__ void edge_rows_kernel(const u32* rs, u32 n_rows, u32* row_of_edge) {
     for (u32 k = rs[r] + (threadIdx.x & 31u); k < end; k += 32) row_of_edge[k] = static_cast<u32>(r);
 }
 
+// The same, each entry also naming its place in the row: (row + row0) << 5 | min(place, 31).
+__global__ void edge_places_kernel(const u32* rs, u32 n_rows, u32 row0, u32* place_of_edge) {
+    const u64 r = (static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (r >= n_rows) return;
+    const u32 start = rs[r], end = rs[r + 1];
+    for (u32 k = start + (threadIdx.x & 31u); k < end; k += 32)
+        place_of_edge[k] = (static_cast<u32>(r) + row0) << 5 | min(k - start, 31u);
+}
+
 __global__ void iota_kernel(u32* v, u64 n) {
     const u64 i = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) v[i] = static_cast<u32>(i);
@@ -110,8 +120,9 @@ __global__ void add_offset_kernel(u32* v, u64 n, u32 off) {
 // depend on; positions let e2a deposits name their place in the target row.  Row r
 // of `c` is target row0 + r (a network that keeps only its owned cells' rows), and
 // the forward lists hold target ids.
+// With `places` an entry is target << 5 | min(place in the target's row, 31).
 Status invert_csr(const DeviceCSR& c, u32 row0, u32 n_sources, DevBuf<u32>& rs, DevBuf<u32>& dst, DevBuf<u32>* pos,
-                  cudaStream_t st) {
+                  bool places, cudaStream_t st) {
     const u64 n = c.n_edges;
     AS_TRY(rs.alloc(static_cast<size_t>(n_sources) + 1));
     AS_TRY(dst.alloc(n));
@@ -123,8 +134,9 @@ Status invert_csr(const DeviceCSR& c, u32 row0, u32 n_sources, DevBuf<u32>& rs, 
     DevBuf<u32> row_of, keys_out;
     AS_TRY(row_of.alloc(n));
     AS_TRY(keys_out.alloc(n));
-    edge_rows_kernel<<<ceil_div(static_cast<u64>(c.n_targets) * 32, 256), 256, 0, st>>>(c.row_start.get(), c.n_targets,
-                                                                                     row_of.get());
+    const u32 row_blocks = ceil_div(static_cast<u64>(c.n_targets) * 32, 256);
+    if (places) edge_places_kernel<<<row_blocks, 256, 0, st>>>(c.row_start.get(), c.n_targets, row0, row_of.get());
+    else edge_rows_kernel<<<row_blocks, 256, 0, st>>>(c.row_start.get(), c.n_targets, row_of.get());
     AS_CUDA(cudaGetLastError());
     int end_bit = 1;
     while (end_bit < 32 && (1ull << end_bit) < static_cast<u64>(n_sources) + 1) ++end_bit;
@@ -141,7 +153,7 @@ Status invert_csr(const DeviceCSR& c, u32 row0, u32 n_sources, DevBuf<u32>& rs, 
                                                 n, 0, end_bit, st));
         lower_bound_rows_kernel<<<ceil_div(static_cast<u64>(n_sources) + 1, 256), 256, 0, st>>>(keys_out.get(), n,
                                                                                               n_sources, rs.get());
-        if (row0) add_offset_kernel<<<ceil_div(n, 256), 256, 0, st>>>(dst.get(), n, row0);
+        if (row0 && !places) add_offset_kernel<<<ceil_div(n, 256), 256, 0, st>>>(dst.get(), n, row0);
         AS_CUDA(cudaGetLastError());
         AS_CUDA(cudaStreamSynchronize(st));
         return Status::Ok();
@@ -194,11 +206,11 @@ Status window_setup(const RunConsts& rc, Network& net, bool fp32, WindowState& w
         }
     } else {
         net.drop_forward();
-        AS_TRY(invert_csr(net.exc, net.own.n_lo, rc.n_exc, ws.fwd.exc_rs, ws.fwd.exc_dst, nullptr, st));
-        AS_TRY(invert_csr(net.inh, net.own.n_lo, net.sz.n_inh, ws.fwd.inh_rs, ws.fwd.inh_dst, nullptr, st));
+        AS_TRY(invert_csr(net.exc, net.own.n_lo, rc.n_exc, ws.fwd.exc_rs, ws.fwd.exc_dst, nullptr, false, st));
+        AS_TRY(invert_csr(net.inh, net.own.n_lo, net.sz.n_inh, ws.fwd.inh_rs, ws.fwd.inh_dst, nullptr, false, st));
     }
-    AS_TRY(invert_csr(net.e2a, net.own.a_lo, rc.n_exc, ws.fwd.e2a_rs, ws.fwd.e2a_astro, &ws.fwd.e2a_pos, st));
-    AS_TRY(invert_csr(net.sic, net.own.n_lo, rc.n_astro, ws.fwd.sic_rs, ws.fwd.sic_dst, nullptr, st));
+    AS_TRY(invert_csr(net.e2a, net.own.a_lo, rc.n_exc, ws.fwd.e2a_rs, ws.fwd.e2a_astro, &ws.fwd.e2a_pos, false, st));
+    AS_TRY(invert_csr(net.sic, net.own.n_lo, rc.n_astro, ws.fwd.sic_rs, ws.fwd.sic_dst, nullptr, true, st));
     // Windows with more spikes than this use the pull gather instead of deposits.
     // ASTROSIM_PUSH_LIMIT overrides it (the tests force the pull path with 0).
     ws.push_limit = static_cast<u32>(std::max<u64>(1024, nN / 50));
@@ -214,7 +226,7 @@ Status window_setup(const RunConsts& rc, Network& net, bool fp32, WindowState& w
     AS_TRY(ws.spk_count.alloc_zero(2, st));
     AS_TRY(ws.sic_win.alloc_zero(2 * nA * ws.W * rb, st));
     AS_TRY(ws.astro_active.alloc_zero(2 * ((nA + 31) / 32), st));
-    AS_TRY(ws.sic_flag.alloc_zero(2 * ((nN + 31) / 32), st));
+    AS_TRY(ws.sic_pos.alloc_zero(2 * nN, st));
     AS_TRY(ws.mode.alloc_zero(2, st));
     AS_TRY(ws.events.alloc(nN));
     AS_CUDA(cudaStreamSynchronize(st));
@@ -223,23 +235,16 @@ Status window_setup(const RunConsts& rc, Network& net, bool fp32, WindowState& w
 
 namespace {
 
-// Variants the autotuner chooses from: (block size, minimum resident blocks per SM, cells
-// per thread).  The FP32 form comes with two cells per thread at two register budgets, the
-// faster ones for networks that fill the chip, and with one (N = 500: 14.9 us per window
-// against 19.4 with two, whose warps are half as many and longer); the FP64 form with
-// three register budgets.
+// Variants the autotuner chooses from: (block size, minimum resident blocks per SM).
+// Each block size comes with three occupancy targets (the same threads per SM as
+// the 128-thread entries), trading registers (and a few spills) for occupancy.
 struct Variant {
-    int block, min_blocks, cells;
+    int block, min_blocks;
 };
-#ifndef ASTROSIM_FP32_IEEE
-constexpr Variant kVariantsF32[] = {{128, 5, 2}, {128, 6, 2}, {128, 8, 1}, {64, 10, 2}, {64, 12, 2}, {64, 12, 1},
-                                    {256, 2, 2}, {256, 3, 2}, {256, 4, 1}};
-#else
-constexpr Variant kVariantsF32[] = {{128, 6, 1}, {128, 8, 1}, {128, 4, 1}, {64, 12, 1}, {64, 16, 1}, {64, 8, 1},
-                                    {256, 3, 1}, {256, 4, 1}, {256, 2, 1}};
-#endif
-constexpr Variant kVariantsF64[] = {{128, 4, 1}, {128, 5, 1}, {128, 3, 1}, {64, 8, 1}, {64, 10, 1}, {64, 6, 1},
-                                    {256, 2, 1}, {256, 3, 1}, {256, 1, 1}};
+constexpr Variant kVariantsF32[] = {{128, 6}, {128, 8}, {128, 4}, {64, 12}, {64, 16}, {64, 8},
+                                    {256, 3}, {256, 4}, {256, 2}};
+constexpr Variant kVariantsF64[] = {{128, 4}, {128, 5}, {128, 3}, {64, 8}, {64, 10}, {64, 6},
+                                    {256, 2}, {256, 3}, {256, 1}};
 constexpr int kNumVariants = 9;
 constexpr int kVariantsPerBlock = 3;
 constexpr int kTuneRounds = 2;
@@ -268,11 +273,17 @@ void variant_range(int block, int* first, int* count) {
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int> g_tuned;  // (precision, log2 size bucket, requested block) -> variant
 
-template <typename R, int B, int M, int C>
+template <typename R, int B, int M>
 cudaError_t launch_one(cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p, const WinPtrs<R>& w, i64 start,
                        int s0, int s1, int buf, i64 mark, int block) {
-    const CellTiles tiles = cell_tiles(rc.n_exc, 0, rc.n_neurons, 0, rc.n_astro, static_cast<u32>(block * C));
-    window_kernel<R, B, M, C><<<total_tiles(tiles), block, 0, st>>>(rc, p, w, start, s0, s1, buf, mark, tiles);
+    const CellTiles tiles = cell_tiles(rc.n_exc, 0, rc.n_neurons, 0, rc.n_astro, static_cast<u32>(block));
+    const size_t smem = sic_bytes<R>(w.W, block);
+    if (smem > 48 * 1024) {  // large blocks of the generic instantiation
+        const cudaError_t e = cudaFuncSetAttribute(window_kernel<R, B, M>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+    }
+    window_kernel<R, B, M><<<total_tiles(tiles), block, smem, st>>>(rc, p, w, start, s0, s1, buf, mark, tiles);
     return cudaGetLastError();
 }
 
@@ -282,7 +293,7 @@ using LaunchFn = cudaError_t (*)(cudaStream_t, const RunConsts&, const StepPtrs<
 template <typename R, int V>
 constexpr LaunchFn<R> variant_launch() {
     constexpr Variant v = std::is_same<R, float>::value ? kVariantsF32[V] : kVariantsF64[V];
-    return &launch_one<R, v.block, v.min_blocks, v.cells>;
+    return &launch_one<R, v.block, v.min_blocks>;
 }
 template <typename R, int... V>
 constexpr std::array<LaunchFn<R>, sizeof...(V)> variant_launches(std::integer_sequence<int, V...>) {
@@ -295,7 +306,7 @@ template <typename R>
 cudaError_t launch_window(int variant, int block, cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p,
                           const WinPtrs<R>& w, i64 start, int s0, int s1, int buf, i64 mark) {
     static constexpr auto table = variant_launches<R>(std::make_integer_sequence<int, kNumVariants>());
-    if (variant < 0) return launch_one<R, 1024, 1, 1>(st, rc, p, w, start, s0, s1, buf, mark, block);
+    if (variant < 0) return launch_one<R, 1024, 1>(st, rc, p, w, start, s0, s1, buf, mark, block);
     const Variant v = std::is_same<R, float>::value ? kVariantsF32[variant] : kVariantsF64[variant];
     return table[variant](st, rc, p, w, start, s0, s1, buf, mark, v.block);
 }

@@ -13,10 +13,10 @@
 //   - pull (a busy window, or a target whose slots overflowed): the target walks its
 //     CSR rows against the previous window's per-neuron spike words, exactly like
 //     the per-step gather.
-// SIC factors are pulled through a per-window "astrocyte active" bitmask, by the
-// neurons that the push flagged: those whose a2n row holds an astrocyte that was
-// active (the push walks each active astrocyte's forward a2n list), so a window
-// without active astrocytes costs every other neuron one flag-word read.
+// SIC factors are pulled by the neurons whose a2n row holds an astrocyte that was active:
+// the push walks each active astrocyte's forward a2n list and marks its position in each
+// target's row, so that a neuron reads its marked positions only, and a neuron without
+// any one word.
 // The launch that pushes a window's spikes also draws the next window's background events
 // (poisson_window.cuh).
 #pragma once
@@ -42,7 +42,7 @@ struct ForwardCSR {
     DevBuf<u32> exc_rs, exc_dst;            // excitatory source -> neuron targets
     DevBuf<u32> inh_rs, inh_dst;            // stored inhibitory id -> neuron targets
     DevBuf<u32> e2a_rs, e2a_astro, e2a_pos; // excitatory source -> (astrocyte, position in its row)
-    DevBuf<u32> sic_rs, sic_dst;            // astrocyte -> neurons whose a2n rows hold it
+    DevBuf<u32> sic_rs, sic_dst;            // astrocyte -> (neuron << 5 | position in its a2n row, at most 31)
     u32 max_fanout = 0;
 };
 
@@ -58,7 +58,7 @@ struct WindowState {
     DevBuf<u32> spk_count;                    // [2]
     DevBuf<unsigned char> sic_win;            // [2][n_astro][W] real
     DevBuf<u32> astro_active;                 // [2][ceil(n_astro / 32)]
-    DevBuf<u32> sic_flag;                     // [2][ceil(n_neurons / 32)]: a2n row holds an active astrocyte
+    DevBuf<u32> sic_pos;                      // [2][n_neurons]: positions of active astrocytes in the a2n row
     DevBuf<int> mode;                         // [2]: 0 push, 1 pull
     DevBuf<u64> events;                       // background event counts of one window (poisson_window.cuh)
     i64 events_window = -1;                   // the window whose counts `events` holds (single-network engine)

@@ -1,6 +1,6 @@
 """Edges of the window kernels' tiles and of the background draws: network sizes around
-one and two tiles of every block size (so that a thread has one cell, two, or a second
-one past its population's end), background rates around the limits of the window-wide
+one and two tiles of every block size (so that blocks and warps are partly
+empty), background rates around the limits of the window-wide
 draw, and the long windows of small steps.  The per-step path draws and rounds every step
 by itself, and every result must equal it bit for bit."""
 import numpy as np
