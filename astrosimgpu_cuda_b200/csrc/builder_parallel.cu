@@ -12,9 +12,10 @@
 //  1. Pools: each post's pool is 5 draws unless a duplicate forces a redraw;
 //     offsets are found by a fixed-point iteration (each round fixes at least the
 //     first misplaced post).
-//  2. Skip cache: floor(log1p(-u) / log1p(-p)) for every tape position the walks
-//     can reach, computed once; ambiguous values (quotient within a few ulps of an
-//     integer) are settled with the host C library that the reference uses.
+//  2. Draw cache: for every tape position the walks can reach, its skip
+//     floor(log1p(-u) / log1p(-p)), its third-factor test and its pool pick in one
+//     word, computed once (walk_chunked.cuh); ambiguous skips (quotient within a few
+//     ulps of an integer) are settled with the host C library that the reference uses.
 //  3. For each walk section (E block, I block, inhibitory pres), the section's
 //     tape is cut into chunks.  For each chunk, walks start from EVERY candidate
 //     entry position in [T, T + delta) -- the chunk's first pre start must be one
@@ -113,14 +114,13 @@ __global__ void diff_kernel(const u64* a, const u64* b, u64 n, int* flag) {
     if (i < n && a[i] != b[i]) *flag = 1;
 }
 
-// ---------------------------------------------------------------- skip cache
-__global__ void skip_cache_kernel(u64 seed, double L, u64 base, u64 n, u32* cache, AmbiguityLog amb) {
+// ---------------------------------------------------------------- draw cache
+__global__ void draw_cache_kernel(u64 seed, double L, u64 base, u64 n, u32 take, u32* cache, AmbiguityLog amb) {
     const u64 stride = static_cast<u64>(gridDim.x) * blockDim.x;
     const SkipTable none{};
-    for (u64 i = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const double g = skip_value(seed, L, base + i, none, amb);
-        cache[i] = g >= 4294967295.0 ? 0xFFFFFFFFu : static_cast<u32>(g);
-    }
+    for (u64 i = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+        cache[i] = draw_word(rng_bits(seed, kSetupStream, base + i) >> 11, skip_value(seed, L, base + i, none, amb),
+                             take);
 }
 
 // ---------------------------------------------------------------- chunk tables
@@ -303,20 +303,45 @@ __global__ void __launch_bounds__(128) swarm_kernel(Sec s, u64 sec_start, u32 ch
     }
 }
 
+// The kernels whose lanes walk long stretches (walk_stretch): `lanes` of each warp walk,
+// each with a tape ring of its own in dynamic shared memory.
+constexpr u32 kWalkBlock = 64;
+inline size_t ring_bytes(u32 lanes) { return static_cast<size_t>(kWalkBlock / 32) * lanes * kRingWords * sizeof(u32); }
+inline u32 walk_blocks(u64 walks, u32 lanes) { return std::max<u32>(1, ceil_div(walks, kWalkBlock / 32 * lanes)); }
+struct Walker {
+    u32 walk;    // this lane's walk
+    bool walks;  // false for the lanes past `lanes`
+    u32* ring;
+    __device__ __forceinline__ explicit Walker(u32 lanes) {
+        extern __shared__ __align__(16) u32 rings[];
+        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        walks = lane < lanes;
+        walk = (blockIdx.x * (kWalkBlock / 32) + warp) * lanes + lane;
+        ring = rings + (warp * lanes + (walks ? lane : 0)) * kRingWords;
+    }
+};
+
 // The walks a warp handed off, to the chunk end without claims.
-__global__ void swarm_continue_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, const SwarmCont* cont,
-                                      const unsigned* n_cont, unsigned cont_cap, SwarmRec rec) {
-    const u32 k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= min(*n_cont, cont_cap)) return;
-    const SwarmCont q = cont[k];
+__global__ void __launch_bounds__(kWalkBlock) swarm_continue_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta,
+                                                                    const SwarmCont* cont, const unsigned* n_cont,
+                                                                    unsigned cont_cap, SwarmRec rec, u32 lanes) {
+    const Walker me(lanes);
+    const u32 k = me.walk;
+    const bool mine = me.walks && k < min(*n_cont, cont_cap);
+    SwarmCont q{0, 0, 0, 0, 0};
+    if (mine) q = cont[k];
     const u64 T1 = sec_start + static_cast<u64>(q.chunk + 1) * chunk_len;
     u64 c = q.c;
     u32 cnt = q.cnt;
-    NoVisit nv;
-    while (c < T1) {
-        c = walk_pre(s, c, kNoSelf, nv);
-        ++cnt;
-    }
+    walk_stretch(
+        s, c, mine && c < T1, me.ring,
+        [&](u64 start) {
+            c = start;
+            ++cnt;
+            return c < T1;
+        },
+        [] { return kNoSelf; });
+    if (!mine) return;
     const u64 r = static_cast<u64>(q.chunk) * delta + q.w;
     rec.par[r] = -1;
     rec.mycnt[r] = cnt;
@@ -408,19 +433,26 @@ __global__ void chunk_entry_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delt
 }
 
 // One thread per chunk writes the start of every pre that begins in the chunk.
-__global__ void materialize_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 n_chunks, const u64* c_entry,
-                                   const u64* c_g0, u64 limit, u64* orbit) {
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_chunks) return;
-    u64 idx = c_g0[i];
-    if (idx >= limit) return;
+__global__ void __launch_bounds__(kWalkBlock) materialize_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 n_chunks,
+                                                                 const u64* c_entry, const u64* c_g0, u64 limit,
+                                                                 u64* orbit, u32 lanes) {
+    const Walker me(lanes);
+    const u32 i = me.walk;
+    const bool mine = me.walks && i < n_chunks;
+    u64 idx = mine ? c_g0[i] : limit;
     const u64 T1 = sec_start + static_cast<u64>(i + 1) * chunk_len;
-    u64 c = c_entry[i];
-    NoVisit nv;
-    while (c < T1 && idx < limit) {
-        orbit[idx++] = c;
-        c = walk_pre(s, c, kNoSelf, nv);
-    }
+    u64 c = mine ? c_entry[i] : 0;
+    const bool live = idx < limit && c < T1;
+    if (live) orbit[idx++] = c;
+    walk_stretch(
+        s, c, live && idx < limit, me.ring,
+        [&](u64 start) {
+            c = start;
+            if (c >= T1 || idx >= limit) return false;
+            orbit[idx++] = c;
+            return idx < limit;
+        },
+        [] { return kNoSelf; });
     if (idx < limit && i + 1 < n_chunks && c != c_entry[i + 1]) atomicOr(s.err, kErrOrbit);
 }
 
@@ -495,13 +527,13 @@ __device__ __forceinline__ long long find_in_orbit(const u64* orbit, u64 n, u64 
 // The exact walk from pre start c with true index r, applying the autapse rule
 // with true indices, until it lands on a start of the table orbit, the section's
 // last pre ends, or it has recorded `cap` starts (then it stops where it stands and
-// can be continued from there).
-__device__ __forceinline__ void remerge_from(const Sec& s, u64 c, long long r, const u64* orbit, u64 n_orbit,
-                                             u64 n_pres, u32 cap, u64* starts, Remerge& out) {
+// can be continued from there).  Every lane of the warp takes part (`live`: has a walk).
+__device__ __forceinline__ void remerge_from(const Sec& s, bool live, u64 c, long long r, const u64* orbit,
+                                             u64 n_orbit, u64 n_pres, u32 cap, u64* starts, u32* ring, Remerge& out) {
     out = Remerge{-1, 0, 0, 0, 0, 0, 0, 0, 0};
-    starts[out.m++] = c;
     u64 from = 0;
-    {
+    if (live) {
+        starts[out.m++] = c;
         u64 lo = 0, hi = n_orbit;  // c's lower bound in the orbit, once
         while (lo < hi) {
             const u64 mid = (lo + hi) >> 1;
@@ -509,55 +541,58 @@ __device__ __forceinline__ void remerge_from(const Sec& s, u64 c, long long r, c
         }
         from = lo;
     }
-    for (;;) {
-        c = walk_pre_end(s, c, static_cast<u32>(r));
-        ++r;
-        if (r >= static_cast<long long>(n_pres)) {
-            out.end = c;
-            out.ok = 1;
-            return;
-        }
-        const long long k = find_in_orbit(orbit, n_orbit, c, from);
-        if (k >= 0) {
-            out.k = k;
-            out.shift = r - k;
-            out.ok = 1;
-            return;
-        }
-        if (out.m >= cap) {
-            out.capped = 1;
-            out.c_next = c;
-            out.r_next = r;
-            return;
-        }
-        starts[out.m++] = c;
-    }
+    walk_stretch(
+        s, c, live, ring,
+        [&](u64 start) {
+            ++r;
+            if (r >= static_cast<long long>(n_pres)) {
+                out.end = start;
+                out.ok = 1;
+                return false;
+            }
+            const long long k = find_in_orbit(orbit, n_orbit, start, from);
+            if (k >= 0) {
+                out.k = k;
+                out.shift = r - k;
+                out.ok = 1;
+                return false;
+            }
+            if (out.m >= cap) {
+                out.capped = 1;
+                out.c_next = start;
+                out.r_next = r;
+                return false;
+            }
+            starts[out.m++] = start;
+            return true;
+        },
+        [&] { return static_cast<u32>(r); });
 }
 
 // For each hazard, assume it is real (true index = r + d) and walk exactly from
 // there (remerge_from) with at most max_explicit starts.  Most walks rejoin within a
 // few pres; the host continues a capped walk only when its replay reaches it.
-__global__ void remerge_kernel(Sec s, const Hazard* hz, u32 n_hz, const u64* orbit, u64 n_orbit, u64 n_pres,
-                               u32 max_explicit, u64* expl, Remerge* res) {
-    const u32 h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= n_hz) return;
-    const long long r = static_cast<long long>(hz[h].r) + hz[h].d;
-    if (r < 0 || r >= static_cast<long long>(n_pres)) {
-        res[h] = Remerge{-1, 0, 0, 0, 0, 0, 0, 0, 0};
-        return;
-    }
+__global__ void __launch_bounds__(kWalkBlock) remerge_kernel(Sec s, const Hazard* hz, u32 n_hz, const u64* orbit,
+                                                             u64 n_orbit, u64 n_pres, u32 max_explicit, u64* expl,
+                                                             Remerge* res, u32 lanes) {
+    const Walker me(lanes);
+    const u32 h = me.walk;
+    const bool mine = me.walks && h < n_hz;
+    const long long r = mine ? static_cast<long long>(hz[h].r) + hz[h].d : -1;
+    const bool live = r >= 0 && r < static_cast<long long>(n_pres);
     Remerge out;
-    remerge_from(s, orbit[hz[h].r], r, orbit, n_orbit, n_pres, max_explicit, expl + static_cast<u64>(h) * max_explicit,
-                 out);
-    res[h] = out;
+    remerge_from(s, live, live ? orbit[hz[h].r] : s.cache_base, r, orbit, n_orbit, n_pres, max_explicit,
+                 expl + static_cast<u64>(h) * max_explicit, me.ring, out);
+    if (mine) res[h] = out;
 }
 
-// One capped walk continued from where it stopped.
-__global__ void remerge_continue_kernel(Sec s, u64 c, long long r, const u64* orbit, u64 n_orbit, u64 n_pres, u32 cap,
-                                        u64* starts, Remerge* res) {
+// One capped walk continued from where it stopped (one warp, its first lane walks).
+__global__ void __launch_bounds__(32) remerge_continue_kernel(Sec s, u64 c, long long r, const u64* orbit, u64 n_orbit,
+                                                              u64 n_pres, u32 cap, u64* starts, Remerge* res) {
+    __shared__ __align__(16) u32 ring[kRingWords];
     Remerge out;
-    remerge_from(s, c, r, orbit, n_orbit, n_pres, cap, starts, out);
-    *res = out;
+    remerge_from(s, threadIdx.x == 0, c, r, orbit, n_orbit, n_pres, cap, starts, ring, out);
+    if (threadIdx.x == 0) *res = out;
 }
 
 // The spliced orbit: piece p covers true indices [t_start[p], t_start[p] + len) and
@@ -871,8 +906,9 @@ Status chunk_tables(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks
     swarm_kernel<<<blocks, 128, 0, st>>>(s, sec_start, chunk_len, delta, n_chunks, handoff, counters.get(),
                                          tables.get(), rec, cont.get(), counters.get() + 1, cont_cap);
     AS_CUDA(cudaGetLastError());
-    swarm_continue_kernel<<<ceil_div(cont_cap, 128), 128, 0, st>>>(s, sec_start, chunk_len, delta, cont.get(),
-                                                                  counters.get() + 1, cont_cap, rec);
+    const u32 lanes = walking_lanes(cont_cap, sm_count() * 4);
+    swarm_continue_kernel<<<walk_blocks(cont_cap, lanes), kWalkBlock, ring_bytes(lanes), st>>>(
+        s, sec_start, chunk_len, delta, cont.get(), counters.get() + 1, cont_cap, rec, lanes);
     AS_CUDA(cudaGetLastError());
     swarm_resolve_kernel<<<ceil_div(n, 256), 256, 0, st>>>(delta, n, rec, s.err, t_exit, t_cnt);
     AS_CUDA(cudaGetLastError());
@@ -976,9 +1012,9 @@ Status section_orbit(const SectionPlan& P, Sec s, u64 start, DevBuf<int>& err, D
         }
         DevBuf<u64> forbit;
         AS_TRY(forbit.alloc(target));
-        materialize_kernel<<<ceil_div(used_chunks, 128), 128, 0, st>>>(s, start, chunk_len, used_chunks,
-                                                                       c_entry.get(), c_g0.get(), target,
-                                                                       forbit.get());
+        const u32 lanes = walking_lanes(used_chunks, sm_count() * 4);
+        materialize_kernel<<<walk_blocks(used_chunks, lanes), kWalkBlock, ring_bytes(lanes), st>>>(
+            s, start, chunk_len, used_chunks, c_entry.get(), c_g0.get(), target, forbit.get(), lanes);
         AS_CUDA(cudaGetLastError());
         AS_TRY(read_err(err, &herr, st));
         if (herr & kErrDelta) {
@@ -1028,8 +1064,10 @@ Status section_orbit(const SectionPlan& P, Sec s, u64 start, DevBuf<int>& err, D
         std::vector<Remerge> rr(n_hz);
         if (n_hz) {
             AS_CUDA(cudaMemcpyAsync(hz_sorted.get(), hh.data(), n_hz * sizeof(Hazard), cudaMemcpyHostToDevice, st));
-            remerge_kernel<<<ceil_div(n_hz, 64), 64, 0, st>>>(s, hz_sorted.get(), n_hz, forbit.get(), target, P.n_pres,
-                                                             max_explicit, expl.get(), rm.get());
+            const u32 walk_lanes = walking_lanes(n_hz, sm_count() * 4);
+            remerge_kernel<<<walk_blocks(n_hz, walk_lanes), kWalkBlock, ring_bytes(walk_lanes), st>>>(
+                s, hz_sorted.get(), n_hz, forbit.get(), target, P.n_pres, max_explicit, expl.get(), rm.get(),
+                walk_lanes);
             AS_CUDA(cudaGetLastError());
             AS_TRY(to_host(rr.data(), rm.get(), n_hz, st));
             AS_TRY(read_err(err, &herr, st));
@@ -1062,7 +1100,7 @@ Status section_orbit(const SectionPlan& P, Sec s, u64 start, DevBuf<int>& err, D
             for (u32 cap = 4096; m.capped; cap = std::min<u32>(cap * 8, 1u << 24)) {
                 DevBuf<u64> buf;
                 AS_TRY(buf.alloc(cap));
-                remerge_continue_kernel<<<1, 1, 0, st>>>(s, m.c_next, m.r_next, forbit.get(), target, P.n_pres, cap,
+                remerge_continue_kernel<<<1, 32, 0, st>>>(s, m.c_next, m.r_next, forbit.get(), target, P.n_pres, cap,
                                                          buf.get(), cont_res.get());
                 AS_CUDA(cudaGetLastError());
                 Remerge m2{};
@@ -1169,7 +1207,8 @@ Status build_parallel(const Sizes& sz, u64 seed, u64 c0, Network& net, cudaStrea
     prefix_new.release();
     pc.mark("pools");
 
-    // ---- 2. skip cache over every tape position the three sections can reach
+    // ---- 2. draw cache over every tape position the three sections can reach
+    if (nN >= kSkipMax) return make_error(ASTROSIM_ERR_OUT_OF_MEMORY, "%u neurons need a draw cache of over 100 GB", nN);
     const double ne = sz.n_exc, ni = sz.n_inh, nn = nN, p = sz.p;
     SectionPlan plans[3] = {
         {"E block", sz.n_exc, 0, 1, sz.n_exc, 1.0 + p * ne * (2.0 + kPThird), 32768, 384, 1, 0, true, 16384, 4},
@@ -1180,7 +1219,7 @@ Status build_parallel(const Sizes& sz, u64 seed, u64 c0, Network& net, cudaStrea
     for (const auto& P : plans) est_total += static_cast<double>(P.n_pres) * P.draws_per_pre;
     const u64 cache_len = static_cast<u64>(est_total * 1.12) + 64ull * 65536 + 1000000;
     DevBuf<u32> cache;
-    AS_TRY(cache.alloc(cache_len));
+    AS_TRY(cache.alloc(cache_words(cache_len)));
     const double L = std::log1p(-p);  // host value, as the reference computes it (src/astrosim_fused.cu:622)
     {
         DevBuf<u64> amb_pos;
@@ -1191,7 +1230,7 @@ Status build_parallel(const Sizes& sz, u64 seed, u64 c0, Network& net, cudaStrea
         AS_TRY(amb_val.alloc(amb_cap));
         AS_TRY(amb_n.alloc_zero(1, st));
         AmbiguityLog amb{amb_pos.get(), amb_val.get(), amb_n.get(), amb_cap};
-        skip_cache_kernel<<<sm_count() * 16, 256, 0, st>>>(seed, L, pools_end, cache_len, cache.get(), amb);
+        draw_cache_kernel<<<sm_count() * 16, 256, 0, st>>>(seed, L, pools_end, cache_len, take, cache.get(), amb);
         AS_CUDA(cudaGetLastError());
         unsigned n_amb = 0;
         AS_TRY(to_host(&n_amb, amb_n.get(), 1, st));
@@ -1199,14 +1238,13 @@ Status build_parallel(const Sizes& sz, u64 seed, u64 c0, Network& net, cudaStrea
         std::vector<u64> pos(n_amb);
         if (n_amb) AS_TRY(to_host(pos.data(), amb_pos.get(), n_amb, st));
         for (u64 t : pos) {  // settle with the host formula
-            const double g = skip_value_host(seed, L, t);
-            const u32 v = g >= 4294967295.0 ? 0xFFFFFFFFu : static_cast<u32>(g);
+            const u32 v = draw_word(rng_bits(seed, kSetupStream, t) >> 11, skip_value_host(seed, L, t), take);
             AS_CUDA(cudaMemcpyAsync(cache.get() + (t - pools_end), &v, sizeof(u32), cudaMemcpyHostToDevice, st));
             AS_CUDA(cudaStreamSynchronize(st));
         }
     }
 
-    pc.mark("skip cache");
+    pc.mark("draw cache");
     // ---- 3-4. every pre's start, section by section
     Sec s{};
     s.seed = seed;
