@@ -16,22 +16,21 @@
 //     floor(log1p(-u) / log1p(-p)), its third-factor test and its pool pick in one
 //     word, computed once (walk_chunked.cuh); ambiguous skips (quotient within a few
 //     ulps of an integer) are settled with the host C library that the reference uses.
-//  3. For each walk section (E block, I block, inhibitory pres), the section's
-//     tape is cut into chunks.  For each chunk, walks start from EVERY candidate
-//     entry position in [T, T + delta) -- the chunk's first pre start must be one
-//     of them -- and merge when they land on the same pre start (a claim table):
-//     one CTA per short chunk, all candidates at once; persistent warp swarms for
-//     long chunks.  That gives an exact table: entry -> (exit, pres started).
-//     Tables are composed (groups in parallel, then one thread over the groups),
-//     which yields every chunk's true entry, and one thread per chunk then writes
-//     every pre's start ("orbit").
-//  4. The transfer tables ignore one index-dependent rule: in the E block a pre
+//  3. For each walk section (E block, I block, inhibitory pres): the length of the pre
+//     that would start at each tape position (walk_chunked.cuh), in parallel.  The
+//     section's tape is cut into chunks; from EVERY candidate entry position in
+//     [T, T + delta) of a chunk -- its first pre start must be one of them -- a thread
+//     follows the lengths to the chunk's end: an exact table entry -> (exit, pres
+//     started).  Tables are composed (groups in parallel, then one thread over the
+//     groups), which yields every chunk's true entry, and one thread per chunk then
+//     writes every pre's start ("orbit").
+//  4. The lengths ignore one index-dependent rule: in the E block a pre
 //     that lands on its own index skips its P_THIRD draws (no autapses).  Such
 //     landings are rare (about 80 per network) but shift the stream, so: every
-//     pre whose walk lands within +-K of its own index is a hazard; for each hazard
-//     a speculative exact walk from that point runs until it rejoins the table
-//     orbit; the host then replays the hazards in order with the running index
-//     shift and splices the true orbit.
+//     pre whose walk lands within +-K of its own index is a hazard; one block then
+//     replays the hazards in order with the running index shift: from each one that
+//     is an autapse it follows the lengths, checking batches of pres for further
+//     autapses, until it rejoins the table orbit, and splices the true orbit.
 //  5. Count and emit: one thread per pre walks its row again (exact rules,
 //     including autapses), first counting, then writing edges at scanned offsets.
 //     The lists are in emission order (the two excitatory blocks interleaved by pre,
@@ -59,17 +58,14 @@ namespace astrosim {
 
 namespace {
 
-constexpr u32 kHashSlots = 4096;  // per-CTA claim table (32 KB of shared memory)
-constexpr unsigned long long kEmpty = ~0ull;
-constexpr u32 kGroup = 64;  // chunks composed per group
-constexpr u32 kMaxDelta = 512;  // candidate entries (walkers) per chunk
-// A section with fewer than target_chunks() (8 per SM) chunks of its planned length
+constexpr u32 kMaxDelta = kMaxPre;  // candidate entries per chunk
+// A section with fewer than target_chunks() (8 per SM) chunks of kChunkLen positions
 // runs with shorter chunks, down to kMinChunkLen (4 x kMaxDelta): the table and orbit
-// passes walk one chunk per thread, position after position, so on small networks
+// passes follow one chunk per thread, pre after pre, so on small networks
 // the chunk length, not the network, sets their time.  The chunking never changes
 // the result, only how the walk is split.
 inline u32 target_chunks() { return sm_count() * 8; }
-constexpr u32 kMinChunkLen = 2048;
+constexpr u32 kMinChunkLen = 2048, kChunkLen = 16384;
 
 // ---------------------------------------------------------------- pools
 __global__ void pool_pass_kernel(u64 seed, u32 n_neurons, u32 n_astro, u32 take, u64 base, const u64* prefix,
@@ -123,259 +119,69 @@ __global__ void draw_cache_kernel(u64 seed, double L, u64 base, u64 n, u32 take,
                              take);
 }
 
-// ---------------------------------------------------------------- chunk tables
-__global__ void table_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u64* t_exit, u32* t_cnt) {
-    __shared__ unsigned long long hash[kHashSlots];
-    __shared__ int par[kMaxDelta];
-    __shared__ u32 mycnt[kMaxDelta], pcnt[kMaxDelta];
-    __shared__ unsigned long long ex[kMaxDelta];
-    for (u32 i = threadIdx.x; i < kHashSlots; i += blockDim.x) hash[i] = kEmpty;
+// ---------------------------------------------------------------- pre lengths and chunk tables
+// lens[i]: the length of the pre that starts at tape position start + i (0: it leaves the
+// cache, kLongPre: it is too long).  One tile of positions per block, its words and jumps
+// in shared memory: 56 KB for 4096 positions and the words a pre may reach past them.
+// Bound by the shared-memory reads of the jumps.
+constexpr u32 kLenTile = 4096, kLenBlock = 512;
+constexpr u32 kLenWords = kLenTile + kWordsAhead + 64, kLenJumps = kLenTile + kJumpsAhead;
+constexpr size_t kLenShared = (kLenWords + 2 * kLenJumps + 64) * sizeof(u32);
+
+__global__ void __launch_bounds__(kLenBlock) pre_length_kernel(Sec s, u64 start, u64 n, u16* lens) {
+    extern __shared__ u32 words[];
+    u32* jumps4 = words + kLenWords;
+    u32* jumps16 = jumps4 + kLenJumps + 48;
+    const u64 tile = static_cast<u64>(blockIdx.x) * kLenTile;
+    for (u32 i = threadIdx.x; i < kLenWords; i += kLenBlock) words[i] = peek(s, start + tile + i);
     __syncthreads();
-    const u64 T0 = sec_start + static_cast<u64>(blockIdx.x) * chunk_len;
-    const u64 T1 = T0 + chunk_len;
+    for (u32 i = threadIdx.x; i < kLenJumps + 36; i += kLenBlock) jumps4[i] = jump4(s, words, i);
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < kLenJumps; i += kLenBlock) jumps16[i] = jump16(jumps4, i);
+    __syncthreads();
+    const u64 end = s.cache_base + s.cache_len;
+    for (u32 i = threadIdx.x; i < kLenTile && tile + i < n; i += kLenBlock) {
+        const u32 len = pre_length(s, words, jumps4, jumps16, i);
+        lens[tile + i] = static_cast<u16>(start + tile + i + len > end ? 0u : len);
+    }
+}
+
+// A chunk's lengths into shared memory (chunk_len is a multiple of 8, chunks are 16-byte aligned).
+__device__ __forceinline__ void stage_lengths(const u16* lens, u32 chunk, u32 chunk_len, u16* shared) {
+    const uint4* from = reinterpret_cast<const uint4*>(lens + static_cast<u64>(chunk) * chunk_len);
+    uint4* to = reinterpret_cast<uint4*>(shared);
+    for (u32 i = threadIdx.x; i < chunk_len / 8; i += blockDim.x) to[i] = from[i];
+    __syncthreads();
+}
+
+// One block per chunk, one thread per candidate entry: t_exit/t_cnt[chunk * delta + d] for
+// the walk from tape position sec_start + chunk * chunk_len + d.
+__global__ void table_kernel(Sec s, const u16* lens, u64 sec_start, u32 chunk_len, u32 delta, u64* t_exit, u32* t_cnt) {
+    extern __shared__ __align__(16) u16 len[];
+    stage_lengths(lens, blockIdx.x, chunk_len, len);
     const u32 w = threadIdx.x;
-    if (w < delta) {
-        u64 c = T0 + w;
-        u32 cnt = 0, pc = 0;
-        int p = -1;
-        NoVisit nv;
-        while (c < T1) {
-            const u32 key = static_cast<u32>(c - T0);
-            u32 slot = (key * 2654435761u) & (kHashSlots - 1);
-            const unsigned long long mine =
-                (static_cast<unsigned long long>(key) << 32) | (static_cast<unsigned long long>(w) << 22) | cnt;
-            bool stop = false;
-            for (u32 probe = 0;; ++probe) {
-                const unsigned long long old = atomicCAS(&hash[slot], kEmpty, mine);
-                if (old == kEmpty) break;  // claimed: this walk continues from here
-                if (static_cast<u32>(old >> 32) == key) {  // another walk was here: follow it
-                    p = static_cast<int>((old >> 22) & 0x3FFu);
-                    pc = static_cast<u32>(old & 0x3FFFFFu);
-                    stop = true;
-                    break;
-                }
-                slot = (slot + 1) & (kHashSlots - 1);
-                if (probe + 1 >= kHashSlots) {
-                    atomicOr(s.err, kErrHash);
-                    stop = true;
-                    break;
-                }
-            }
-            if (stop) break;
-            c = walk_pre(s, c, kNoSelf, nv);
-            ++cnt;
-        }
-        par[w] = p;
-        mycnt[w] = cnt;
-        pcnt[w] = pc;
-        ex[w] = c;
-    }
-    __syncthreads();
-    if (w < delta) {
-        // pres from my candidate = sum over the merge chain of (mine before the merge - the
-        // claimer's count at the merge point) + the root's full count
-        long long total = 0;
-        int x = static_cast<int>(w);
-        for (u32 guard = 0; par[x] >= 0 && guard < kMaxDelta; ++guard) {
-            total += static_cast<long long>(mycnt[x]) - static_cast<long long>(pcnt[x]);
-            x = par[x];
-        }
-        total += mycnt[x];
-        t_exit[static_cast<u64>(blockIdx.x) * delta + w] = ex[x];
-        t_cnt[static_cast<u64>(blockIdx.x) * delta + w] = static_cast<u32>(total);
-    }
-}
-
-// ---------------------------------------------------------------- chunk tables by warp swarms
-// The same tables from persistent warps.  In the one-CTA-per-chunk form above, the
-// walk that never merges holds its CTA (delta threads, 42 KB of shared memory) for
-// the whole chunk, so an SM keeps only 5 chunks in flight and, late in each chunk,
-// walks 5-10 chains.  Here a warp takes a chunk, its lanes take the candidates a few
-// at a time (a lane whose walk merged or left the chunk takes the next candidate),
-// claims go to a per-warp table in global memory, and once every candidate has
-// started and at most `handoff` walks remain, the warp hands them to a
-// one-thread-per-walk kernel and takes the next chunk.  A walk's exit and count are
-// the same whoever it merges into, so the tables are identical.
-constexpr u32 kSwarmSlots = 4096;  // claim slots per warp (32 KB of global memory)
-constexpr u32 kSwarmIdle = 0xFFFFFFFFu;
-
-struct SwarmRec {
-    int* par;     // walk this one merged into, -1 for a walk that reached the chunk end
-    u32* mycnt;   // pres walked before merging (or in all)
-    u32* pcnt;    // the merged-into walk's count where they met
-    u64* ex;      // where the walk stopped
-};
-
-struct SwarmCont {
-    u32 chunk, w;
-    u64 c;
-    u32 cnt, pad_;
-};
-
-__global__ void __launch_bounds__(128) swarm_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks,
-                                                    u32 handoff, unsigned* next_chunk, unsigned long long* tables,
-                                                    SwarmRec rec, SwarmCont* cont, unsigned* n_cont,
-                                                    unsigned cont_cap) {
-    const u32 lane = threadIdx.x & 31u;
-    const u64 warp = (static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    unsigned long long* tab = tables + warp * kSwarmSlots;
-    NoVisit nv;
-    for (;;) {
-        u32 chunk = 0;
-        if (lane == 0) chunk = atomicAdd(next_chunk, 1u);
-        chunk = __shfl_sync(0xffffffffu, chunk, 0);
-        if (chunk >= n_chunks) return;
-        for (u32 i = lane; i < kSwarmSlots; i += 32) tab[i] = kEmpty;
-        __threadfence();  // the cleared slots are in place before any lane's first claim
-        __syncwarp();
-        const u64 T0 = sec_start + static_cast<u64>(chunk) * chunk_len, T1 = T0 + chunk_len;
-        const u64 rb = static_cast<u64>(chunk) * delta;
-        u32 w = lane < delta ? lane : kSwarmIdle;
-        u64 c = T0 + lane;
-        u32 cnt = 0;
-        u32 next = min(32u, delta);
-        for (;;) {
-            bool claimed = false;
-            if (w != kSwarmIdle) {
-                if (c >= T1) {  // reached the chunk end
-                    rec.par[rb + w] = -1;
-                    rec.mycnt[rb + w] = cnt;
-                    rec.ex[rb + w] = c;
-                    w = kSwarmIdle;
-                } else {
-                    const u32 key = static_cast<u32>(c - T0);
-                    u32 slot = (key * 2654435761u) & (kSwarmSlots - 1);
-                    const unsigned long long mine = (static_cast<unsigned long long>(key) << 32) |
-                                                    (static_cast<unsigned long long>(w) << 22) | cnt;
-                    for (u32 probe = 0;; ++probe) {
-                        const unsigned long long old = atomicCAS(&tab[slot], kEmpty, mine);
-                        if (old == kEmpty) {  // claimed: this walk continues from here
-                            claimed = true;
-                            break;
-                        }
-                        if (static_cast<u32>(old >> 32) == key) {  // another walk was here: follow it
-                            rec.par[rb + w] = static_cast<int>((old >> 22) & 0x3FFu);
-                            rec.pcnt[rb + w] = static_cast<u32>(old & 0x3FFFFFu);
-                            rec.mycnt[rb + w] = cnt;
-                            rec.ex[rb + w] = c;
-                            w = kSwarmIdle;
-                            break;
-                        }
-                        slot = (slot + 1) & (kSwarmSlots - 1);
-                        if (probe + 1 >= kSwarmSlots) {  // table full: the host retries with shorter chunks
-                            atomicOr(s.err, kErrHash);
-                            rec.par[rb + w] = -1;
-                            rec.mycnt[rb + w] = cnt;
-                            rec.ex[rb + w] = c;
-                            w = kSwarmIdle;
-                            break;
-                        }
-                    }
-                }
-            }
-            // idle lanes take the next candidates (they claim their start in the next round)
-            const unsigned idle = __ballot_sync(0xffffffffu, w == kSwarmIdle);
-            if (next < delta && idle) {
-                const u32 rank = __popc(idle & ((1u << lane) - 1u));
-                if (w == kSwarmIdle && next + rank < delta) {
-                    w = next + rank;
-                    c = T0 + w;
-                    cnt = 0;
-                }
-                next = min(delta, next + static_cast<u32>(__popc(idle)));
-            }
-            const unsigned live = __ballot_sync(0xffffffffu, w != kSwarmIdle);
-            if (live == 0) break;
-            if (next >= delta && static_cast<u32>(__popc(live)) <= handoff) {
-                if (w != kSwarmIdle) {
-                    const unsigned k = atomicAdd(n_cont, 1u);
-                    if (k < cont_cap) cont[k] = SwarmCont{chunk, w, c, cnt, 0u};
-                    else atomicOr(s.err, kErrOrbit);
-                }
-                break;
-            }
-            if (claimed) {
-                c = walk_pre(s, c, kNoSelf, nv);
-                ++cnt;
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// The kernels whose lanes walk long stretches (walk_stretch): `lanes` of each warp walk,
-// each with a tape ring of its own in dynamic shared memory.
-constexpr u32 kWalkBlock = 64;
-inline size_t ring_bytes(u32 lanes) { return static_cast<size_t>(kWalkBlock / 32) * lanes * kRingWords * sizeof(u32); }
-inline u32 walk_blocks(u64 walks, u32 lanes) { return std::max<u32>(1, ceil_div(walks, kWalkBlock / 32 * lanes)); }
-struct Walker {
-    u32 walk;    // this lane's walk
-    bool walks;  // false for the lanes past `lanes`
-    u32* ring;
-    __device__ __forceinline__ explicit Walker(u32 lanes) {
-        extern __shared__ __align__(16) u32 rings[];
-        const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        walks = lane < lanes;
-        walk = (blockIdx.x * (kWalkBlock / 32) + warp) * lanes + lane;
-        ring = rings + (warp * lanes + (walks ? lane : 0)) * kRingWords;
-    }
-};
-
-// The walks a warp handed off, to the chunk end without claims.
-__global__ void __launch_bounds__(kWalkBlock) swarm_continue_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta,
-                                                                    const SwarmCont* cont, const unsigned* n_cont,
-                                                                    unsigned cont_cap, SwarmRec rec, u32 lanes) {
-    const Walker me(lanes);
-    const u32 k = me.walk;
-    const bool mine = me.walks && k < min(*n_cont, cont_cap);
-    SwarmCont q{0, 0, 0, 0, 0};
-    if (mine) q = cont[k];
-    const u64 T1 = sec_start + static_cast<u64>(q.chunk + 1) * chunk_len;
-    u64 c = q.c;
-    u32 cnt = q.cnt;
-    walk_stretch(
-        s, c, mine && c < T1, me.ring,
-        [&](u64 start) {
-            c = start;
-            ++cnt;
-            return c < T1;
-        },
-        [] { return kNoSelf; });
-    if (!mine) return;
-    const u64 r = static_cast<u64>(q.chunk) * delta + q.w;
-    rec.par[r] = -1;
-    rec.mycnt[r] = cnt;
-    rec.ex[r] = c;
-}
-
-// Exit and pre count of every candidate: along its merge chain, the sum of (pres
-// before the merge - the merged-into walk's count there), plus the last walk's count.
-__global__ void swarm_resolve_kernel(u32 delta, u64 n, SwarmRec rec, int* err, u64* t_exit, u32* t_cnt) {
-    const u64 i = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const u64 base = i - i % delta;
-    u64 x = i;
-    long long total = 0;
-    for (u32 guard = 0; rec.par[x] >= 0; ++guard) {
-        if (guard >= delta) {  // merges point to earlier claims, so chains cannot cycle
-            atomicOr(err, kErrOrbit);
+    if (w >= delta) return;
+    u32 c = w, cnt = 0;
+    while (c < chunk_len) {
+        const u32 l = len[c];
+        if (l == 0 || l == kLongPre) {
+            atomicOr(s.err, l ? kErrDelta : kErrCache);
             break;
         }
-        total += static_cast<long long>(rec.mycnt[x]) - static_cast<long long>(rec.pcnt[x]);
-        x = base + static_cast<u32>(rec.par[x]);
+        c += l;
+        ++cnt;
     }
-    total += rec.mycnt[x];
-    t_exit[i] = rec.ex[x];
-    t_cnt[i] = static_cast<u32>(total);
+    t_exit[static_cast<u64>(blockIdx.x) * delta + w] = sec_start + static_cast<u64>(blockIdx.x) * chunk_len + c;
+    t_cnt[static_cast<u64>(blockIdx.x) * delta + w] = cnt;
 }
 
-// Composes the tables of kGroup consecutive chunks: thread d follows candidate d.
-__global__ void group_compose_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks, const u64* t_exit,
-                                     const u32* t_cnt, u64* g_exit, u64* g_cnt) {
+// Composes the tables of `group` consecutive chunks: thread d follows candidate d.
+__global__ void group_compose_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks, u32 group,
+                                     const u64* t_exit, const u32* t_cnt, u64* g_exit, u64* g_cnt) {
     const u32 g = blockIdx.x, d = threadIdx.x;
     if (d >= delta) return;
-    const u32 c0 = g * kGroup;
-    const u32 c1 = min(c0 + kGroup, n_chunks);
+    const u32 c0 = g * group;
+    const u32 c1 = min(c0 + group, n_chunks);
     u64 x = d, cnt = 0, e = 0;
     for (u32 i = c0; i < c1; ++i) {
         if (x >= delta) {
@@ -391,15 +197,16 @@ __global__ void group_compose_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 de
 }
 
 // One thread over the groups: the true entry and pre index of every group, up to
-// the group where `target` pres are reached.
-__global__ void top_compose_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_groups, const u64* g_exit,
-                                   const u64* g_cnt, u64 target, u64* g_entry, u64* g_g0, u32* end_group) {
+// the group where `target` pres are reached (*end_group, n_groups if they are not).
+__global__ void top_compose_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_groups, u32 group,
+                                   const u64* g_exit, const u64* g_cnt, u64 target, u64* g_entry, u64* g_g0,
+                                   u32* end_group) {
     u64 e = sec_start, cnt = 0;
     u32 g = 0;
     for (; g < n_groups; ++g) {
         g_entry[g] = e;
         g_g0[g] = cnt;
-        const u64 d = e - (sec_start + static_cast<u64>(g) * kGroup * chunk_len);
+        const u64 d = e - (sec_start + static_cast<u64>(g) * group * chunk_len);
         if (d >= delta) {
             atomicOr(s.err, kErrDelta);
             break;
@@ -411,49 +218,52 @@ __global__ void top_compose_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delt
     *end_group = g;
 }
 
-// Per group: the entry and first pre index of each of its chunks.
-__global__ void chunk_entry_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks, u32 n_groups,
+// Per group: the entry and first pre index of each of its chunks (a first index of all
+// ones for the chunks after the end group, which start no pre that is needed).
+__global__ void chunk_entry_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks, u32 n_groups, u32 group,
                                    const u64* t_exit, const u32* t_cnt, const u64* g_entry, const u64* g_g0,
-                                   u64* c_entry, u64* c_g0) {
+                                   const u32* end_group, u64* c_entry, u64* c_g0) {
     const u32 g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n_groups) return;
-    u64 e = g_entry[g], cnt = g_g0[g];
-    const u32 c0 = g * kGroup, c1 = min(c0 + kGroup, n_chunks);
+    const u32 c0 = g * group, c1 = min(c0 + group, n_chunks);
+    bool known = g <= *end_group;
+    u64 e = known ? g_entry[g] : 0, cnt = known ? g_g0[g] : ~u64(0);
     for (u32 i = c0; i < c1; ++i) {
-        c_entry[i] = e;
-        c_g0[i] = cnt;
         const u64 d = e - (sec_start + static_cast<u64>(i) * chunk_len);
-        if (d >= delta) {
+        if (known && d >= delta) {
             atomicOr(s.err, kErrDelta);
-            return;
+            known = false;
         }
+        c_entry[i] = e;
+        c_g0[i] = known ? cnt : ~u64(0);
+        if (!known) continue;
         cnt += t_cnt[static_cast<u64>(i) * delta + d];
         e = t_exit[static_cast<u64>(i) * delta + d];
     }
 }
 
-// One thread per chunk writes the start of every pre that begins in the chunk.
-__global__ void __launch_bounds__(kWalkBlock) materialize_kernel(Sec s, u64 sec_start, u32 chunk_len, u32 n_chunks,
-                                                                 const u64* c_entry, const u64* c_g0, u64 limit,
-                                                                 u64* orbit, u32 lanes) {
-    const Walker me(lanes);
-    const u32 i = me.walk;
-    const bool mine = me.walks && i < n_chunks;
-    u64 idx = mine ? c_g0[i] : limit;
-    const u64 T1 = sec_start + static_cast<u64>(i + 1) * chunk_len;
-    u64 c = mine ? c_entry[i] : 0;
-    const bool live = idx < limit && c < T1;
-    if (live) orbit[idx++] = c;
-    walk_stretch(
-        s, c, live && idx < limit, me.ring,
-        [&](u64 start) {
-            c = start;
-            if (c >= T1 || idx >= limit) return false;
-            orbit[idx++] = c;
-            return idx < limit;
-        },
-        [] { return kNoSelf; });
-    if (idx < limit && i + 1 < n_chunks && c != c_entry[i + 1]) atomicOr(s.err, kErrOrbit);
+// One block per chunk; its first thread writes the start of every pre that begins in the
+// chunk, up to pre `limit`, and the end of pre `last`.
+__global__ void materialize_kernel(Sec s, const u16* lens, u64 sec_start, u32 chunk_len, u32 n_chunks,
+                                   const u64* c_entry, const u64* c_g0, u64 limit, u64 last, u64* orbit, u64* end) {
+    extern __shared__ __align__(16) u16 len[];
+    const u32 i = blockIdx.x;
+    u64 idx = c_g0[i];
+    if (idx >= limit) return;
+    stage_lengths(lens, i, chunk_len, len);
+    if (threadIdx.x) return;
+    const u64 T0 = sec_start + static_cast<u64>(i) * chunk_len;
+    u32 c = static_cast<u32>(c_entry[i] - T0);
+    while (c < chunk_len && idx < limit) {
+        const u32 l = len[c];
+        if (l == 0 || l == kLongPre) return;  // the table pass flagged it
+        orbit[idx] = T0 + c;
+        c += l;
+        if (idx == last) *end = T0 + c;
+        ++idx;
+    }
+    if (idx < limit && i + 1 < n_chunks && c_g0[i + 1] != ~u64(0) && T0 + c != c_entry[i + 1])
+        atomicOr(s.err, kErrOrbit);
 }
 
 // ---------------------------------------------------------------- autapse hazards (E block)
@@ -477,32 +287,18 @@ struct HazardVisit {
     }
 };
 
-__global__ void hazard_kernel(Sec s, const u64* orbit, u64 n, int K, Hazard* out, unsigned* count, unsigned cap) {
+__global__ void hazard_kernel(Sec s, const u64* orbit, u64 n, int K, Hazard* out, unsigned* count, unsigned cap,
+                              const u32* end_group, u32 n_groups) {
     const u64 r = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (r >= n) return;
+    if (r >= n || *s.err || *end_group >= n_groups) return;  // no complete table orbit
     HazardVisit v{static_cast<u32>(r), K, out, count, cap};
     walk_pre(s, orbit[r], kNoSelf, v);
 }
 
-struct Remerge {
-    long long k;       // table-orbit index where the exact walk rejoins (-1: section ended first)
-    long long shift;   // true index - table index after rejoining
-    u32 m;             // explicit pre starts recorded
-    u32 ok;            // the walk rejoined or reached the section's end
-    u64 end;           // section end when the walk reached the last pre
-    // a walk that recorded its cap of starts first (ok == 0, capped == 1): the start
-    // and true index of its next pre, from which it can be continued
-    u64 c_next;
-    long long r_next;
-    u32 capped;
-    u32 pad_;
-};
-
-// Index of c in the sorted orbit, or -1.  `from` is a lower bound of where c can be
-// (the previous query's answer: a walk's queries only move forward); the search
-// gallops from there, so a walk that keeps pace with the orbit costs one or two
-// loads per query instead of a full binary search.  `from` becomes c's lower bound.
-__device__ __forceinline__ long long find_in_orbit(const u64* orbit, u64 n, u64 c, u64& from) {
+// Index of c in the sorted orbit, or -1.  `from` is a lower bound of where c can be; the
+// search gallops from there, so a walk that keeps pace with the orbit costs one or two
+// loads per query instead of a full binary search.
+__device__ __forceinline__ long long find_in_orbit(const u64* orbit, u64 n, u64 c, u64 from) {
     u64 lo = from, hi = n;
     if (lo < n && orbit[lo] < c) {
         u64 step = 1;
@@ -520,79 +316,7 @@ __device__ __forceinline__ long long find_in_orbit(const u64* orbit, u64 n, u64 
         const u64 mid = (lo + hi) >> 1;
         if (orbit[mid] < c) lo = mid + 1; else hi = mid;
     }
-    from = lo;
     return (lo < n && orbit[lo] == c) ? static_cast<long long>(lo) : -1;
-}
-
-// The exact walk from pre start c with true index r, applying the autapse rule
-// with true indices, until it lands on a start of the table orbit, the section's
-// last pre ends, or it has recorded `cap` starts (then it stops where it stands and
-// can be continued from there).  Every lane of the warp takes part (`live`: has a walk).
-__device__ __forceinline__ void remerge_from(const Sec& s, bool live, u64 c, long long r, const u64* orbit,
-                                             u64 n_orbit, u64 n_pres, u32 cap, u64* starts, u32* ring, Remerge& out) {
-    out = Remerge{-1, 0, 0, 0, 0, 0, 0, 0, 0};
-    u64 from = 0;
-    if (live) {
-        starts[out.m++] = c;
-        u64 lo = 0, hi = n_orbit;  // c's lower bound in the orbit, once
-        while (lo < hi) {
-            const u64 mid = (lo + hi) >> 1;
-            if (orbit[mid] < c) lo = mid + 1; else hi = mid;
-        }
-        from = lo;
-    }
-    walk_stretch(
-        s, c, live, ring,
-        [&](u64 start) {
-            ++r;
-            if (r >= static_cast<long long>(n_pres)) {
-                out.end = start;
-                out.ok = 1;
-                return false;
-            }
-            const long long k = find_in_orbit(orbit, n_orbit, start, from);
-            if (k >= 0) {
-                out.k = k;
-                out.shift = r - k;
-                out.ok = 1;
-                return false;
-            }
-            if (out.m >= cap) {
-                out.capped = 1;
-                out.c_next = start;
-                out.r_next = r;
-                return false;
-            }
-            starts[out.m++] = start;
-            return true;
-        },
-        [&] { return static_cast<u32>(r); });
-}
-
-// For each hazard, assume it is real (true index = r + d) and walk exactly from
-// there (remerge_from) with at most max_explicit starts.  Most walks rejoin within a
-// few pres; the host continues a capped walk only when its replay reaches it.
-__global__ void __launch_bounds__(kWalkBlock) remerge_kernel(Sec s, const Hazard* hz, u32 n_hz, const u64* orbit,
-                                                             u64 n_orbit, u64 n_pres, u32 max_explicit, u64* expl,
-                                                             Remerge* res, u32 lanes) {
-    const Walker me(lanes);
-    const u32 h = me.walk;
-    const bool mine = me.walks && h < n_hz;
-    const long long r = mine ? static_cast<long long>(hz[h].r) + hz[h].d : -1;
-    const bool live = r >= 0 && r < static_cast<long long>(n_pres);
-    Remerge out;
-    remerge_from(s, live, live ? orbit[hz[h].r] : s.cache_base, r, orbit, n_orbit, n_pres, max_explicit,
-                 expl + static_cast<u64>(h) * max_explicit, me.ring, out);
-    if (mine) res[h] = out;
-}
-
-// One capped walk continued from where it stopped (one warp, its first lane walks).
-__global__ void __launch_bounds__(32) remerge_continue_kernel(Sec s, u64 c, long long r, const u64* orbit, u64 n_orbit,
-                                                              u64 n_pres, u32 cap, u64* starts, Remerge* res) {
-    __shared__ __align__(16) u32 ring[kRingWords];
-    Remerge out;
-    remerge_from(s, threadIdx.x == 0, c, r, orbit, n_orbit, n_pres, cap, starts, ring, out);
-    if (threadIdx.x == 0) *res = out;
 }
 
 // The spliced orbit: piece p covers true indices [t_start[p], t_start[p] + len) and
@@ -602,16 +326,238 @@ struct OrbitPiece {
     u64 t_start, len;
 };
 
-__global__ void splice_orbit_kernel(const OrbitPiece* pieces, u32 n_pieces, u64 n, u64* dst) {
+struct Replay {
+    u64 end;         // tape position after the section
+    u32 n_pieces;
+    u32 retry;       // the shift left the hazards' range, or the table orbit was too short for it
+    u32 full;        // more pieces than their table holds
+    u32 pad_;
+};
+
+constexpr u32 kReplayOrbit = 64;  // table starts that the replay keeps around its walk
+
+// The first of the kReplayOrbit ascending entries that is not below c (the last is not).
+__device__ __forceinline__ u32 lower_bound_near(const u64* entries, u64 c) {
+    u32 lo = 0, hi = kReplayOrbit - 1;
+    while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if (entries[mid] < c) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// The replay of the E block's autapses in order (one block).  On the table orbit with
+// running shift d (true index - table index) the next autapse is the next hazard that
+// lands d from its table index.  From there the walk leaves the table orbit: its pres are
+// taken in batches of up to 32 (4 in the first, which most walks rejoin in), whose starts
+// follow from the lengths; a lane walks each pre in full for a landing on its true index
+// and looks its start up in the table orbit.  The first of the two ends the batch: an
+// autapse sends the walk on from that pre's exact end, a start on the table orbit ends
+// it.  (Walks rejoin after a median of 2 pres, some after hundreds.)  What bounds it is
+// latency: the load of the window and a lane's walk of about a hundred words.  512 threads
+// load, look through the hazards in shared memory and through the table starts around the
+// walk: 1.5 ms at N = 1e3, 3.0 ms at N = 3e5; 128 threads that read hazards and table
+// starts from global memory took 2.8 and 6.3 ms.
+constexpr u32 kReplayBlock = 512, kReplayBatch = 32, kReplayWindow = 8192;
+constexpr u32 kReplayWords = kReplayWindow + kWordsAhead;
+constexpr u32 kReplayHazards = 6144;  // hazards kept in shared memory (5200 expected), all or none
+constexpr size_t kReplayShared = kReplayWords * sizeof(u32) + kReplayWindow * sizeof(u16) + kReplayHazards * sizeof(Hazard);
+
+__global__ void __launch_bounds__(kReplayBlock) replay_kernel(Sec s, const u16* lens, u64 sec_start, u64 n_lens,
+                                                              const Hazard* hz, const unsigned* n_hz_ptr,
+                                                              unsigned hz_cap, const u64* orbit, u64 n_orbit,
+                                                              u64 n_pres, int K, const u32* end_group, u32 n_groups,
+                                                              u64* starts, OrbitPiece* pieces, u32 piece_cap,
+                                                              Replay* out) {
+    extern __shared__ __align__(16) u32 words[];
+    u16* len = reinterpret_cast<u16*>(words + kReplayWords);
+    Hazard* near_hz = reinterpret_cast<Hazard*>(len + kReplayWindow);
+    __shared__ u64 batch[kReplayBatch + 1];  // the batch's starts, and where it ends
+    __shared__ u64 near_orbit[kReplayOrbit];
+    __shared__ u32 n_batch;
+    __shared__ unsigned best;
+    __shared__ u64 merge_k, auto_end;
+    __shared__ u32 merge_at, auto_at, past_lens;
+    Replay res{0, 0, 0, 0, 0};
+    // an unfinished or failed table pass: the host looks at its flags first
+    const unsigned n_hz = *n_hz_ptr;
+    if (*s.err || *end_group >= n_groups || n_hz > hz_cap) {
+        if (threadIdx.x == 0) *out = res;
+        return;
+    }
+    const bool staged_hz = n_hz <= kReplayHazards;
+    if (staged_hz) {
+#pragma unroll 4
+        for (u32 i = threadIdx.x; i < n_hz; i += kReplayBlock) near_hz[i] = hz[i];
+        __syncthreads();
+    }
+    auto add_piece = [&](const u64* src, u64 t, u64 n) {
+        if (n == 0) return;
+        if (res.n_pieces == piece_cap) {
+            res.full = 1;
+            return;
+        }
+        if (threadIdx.x == 0) pieces[res.n_pieces] = OrbitPiece{src, t, n};
+        ++res.n_pieces;
+    };
+    long long d = 0;
+    u64 cur_f = 0, cur_t = 0, n_starts = 0;
+    bool ended = false;
+    while (!ended && !res.full && !res.retry) {
+        // the next hazard on the orbit at this shift
+        if (threadIdx.x == 0) best = 0xFFFFFFFFu;
+        __syncthreads();
+        unsigned mine = 0xFFFFFFFFu;
+        for (u32 i = threadIdx.x; i < n_hz; i += kReplayBlock) {
+            const Hazard h = staged_hz ? near_hz[i] : hz[i];
+            if (h.d == d && h.r >= cur_f) mine = min(mine, h.r);
+        }
+        if (mine != 0xFFFFFFFFu) atomicMin(&best, mine);
+        __syncthreads();
+        const unsigned at = best;
+        if (at == 0xFFFFFFFFu || static_cast<long long>(at) + d >= static_cast<long long>(n_pres)) break;
+        add_piece(orbit + cur_f, cur_t, at - cur_f);
+        u64 c = orbit[at], r = static_cast<u64>(static_cast<long long>(at) + d);
+        const u64 t_autapse = r, first_start = n_starts;
+        u64 from = at;
+        bool on_orbit_start = true;  // batch 0's first pre is the hazard itself, on the table orbit
+        bool rejoined = false;
+        u32 batch_max = 4;
+        while (!rejoined && !ended) {
+            const u64 i0 = c - sec_start;  // the window: lengths and words from c on
+            const u32 window = batch_max == 4 ? 4 * kMaxPre : kReplayWindow;
+#pragma unroll 8
+            for (u32 i = threadIdx.x; i < window; i += kReplayBlock) len[i] = i0 + i < n_lens ? lens[i0 + i] : u16(0);
+#pragma unroll 8
+            for (u32 i = threadIdx.x; i < window + kWordsAhead; i += kReplayBlock) words[i] = peek(s, c + i);
+            if (threadIdx.x < kReplayOrbit)
+                near_orbit[threadIdx.x] = from + threadIdx.x < n_orbit ? orbit[from + threadIdx.x] : ~u64(0);
+            if (threadIdx.x == 0) {
+                merge_at = auto_at = 0xFFFFFFFFu;
+                past_lens = 0;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                u32 x = 0, n = 0;
+                while (n < batch_max && r + n < n_pres && x + kMaxPre <= window) {
+                    const u32 l = len[x];
+                    if (l == 0 || l == kLongPre) {
+                        if (i0 + x >= n_lens) past_lens = 1;
+                        else atomicOr(s.err, l ? kErrDelta : kErrCache);
+                        break;
+                    }
+                    batch[n++] = c + x;
+                    x += l;
+                }
+                batch[n] = c + x;
+                n_batch = n;
+            }
+            __syncthreads();
+            const u32 n = n_batch;
+            if (n == 0) {  // the walk left the lengths, or (flagged) the cache, or met a pre that is too long
+                res.retry = past_lens;
+                if (threadIdx.x == 0) *out = res;
+                return;
+            }
+            if (threadIdx.x < n) {
+                const u32 q = threadIdx.x;
+                const u64 start = batch[q];
+                // an autapse: the walk lands on its true index (src/astrosim_fused.cu:696)
+                const unsigned lanes = n == 32 ? 0xFFFFFFFFu : (1u << n) - 1u;
+                const u32 self = static_cast<u32>(r + q) - s.post_off;
+                u32 x = static_cast<u32>(start - c), left = s.post_count;
+                bool hit_self = false;
+                u32 skip = words[x++];
+                for (;;) {
+                    const u32 g = skip & kSkipMax;
+                    if (g >= left) break;
+                    if (x + 3 > window + kWordsAhead) {
+                        atomicOr(s.err, kErrDelta);
+                        break;
+                    }
+                    const bool own = s.post_count - left + g == self;
+                    hit_self = hit_self || own;
+                    left -= g + 1;
+                    if (s.third && !own) x += (words[x] & kHitBit) ? 2 : 1;
+                    if (left == 0) break;
+                    skip = words[x++];
+                }
+                long long k = -1;
+                if (q || !on_orbit_start) {
+                    if (start <= near_orbit[kReplayOrbit - 1]) {
+                        const u32 at_near = lower_bound_near(near_orbit, start);
+                        if (near_orbit[at_near] == start) k = static_cast<long long>(from + at_near);
+                    } else {
+                        k = find_in_orbit(orbit, n_orbit, start, from + kReplayOrbit - 1);
+                    }
+                }
+                if (k >= 0) atomicMin(&merge_at, q);
+                if (hit_self) atomicMin(&auto_at, q);
+                __syncwarp(lanes);
+                if (k >= 0 && merge_at == q) merge_k = static_cast<u64>(k);
+                if (hit_self && auto_at == q) auto_end = c + x;
+            }
+            __syncthreads();
+            const u32 m = merge_at, a = auto_at;
+            const u32 taken = m <= a && m != 0xFFFFFFFFu ? m : (a != 0xFFFFFFFFu ? a + 1 : n);
+            if (threadIdx.x < taken) starts[n_starts + threadIdx.x] = batch[threadIdx.x];
+            n_starts += taken;
+            r += taken;
+            if (m <= a && m != 0xFFFFFFFFu) {
+                cur_f = merge_k;
+                cur_t = r;
+                d = static_cast<long long>(r) - static_cast<long long>(cur_f);
+                rejoined = true;
+            } else {
+                c = a != 0xFFFFFFFFu ? auto_end : batch[n];
+                if (r >= n_pres) {
+                    ended = true;
+                    res.end = c;
+                    cur_t = r;
+                }
+            }
+            on_orbit_start = false;
+            batch_max = kReplayBatch;
+            // the table starts from the walk's place on; one that outran them catches up by a search
+            if (c <= near_orbit[kReplayOrbit - 1]) {
+                from += lower_bound_near(near_orbit, c);
+            } else {
+                u64 lo = from + kReplayOrbit - 1, hi = n_orbit;
+                while (lo < hi) {
+                    const u64 mid = (lo + hi) >> 1;
+                    if (orbit[mid] < c) lo = mid + 1; else hi = mid;
+                }
+                from = lo;
+            }
+            __syncthreads();  // the batch and the window are read before the next ones are written
+        }
+        add_piece(starts + first_start, t_autapse, n_starts - first_start);
+        if (rejoined && (d < -K || d > K)) res.retry = 1;
+    }
+    if (!ended && !res.full && !res.retry) {
+        const u64 n = n_pres - cur_t;
+        if (cur_f + n > n_orbit) {
+            res.retry = 1;  // the table orbit ends before the section does
+        } else {
+            add_piece(orbit + cur_f, cur_t, n);
+            // the last pre is no autapse (it would have been a hazard), so its length holds
+            if (n) res.end = orbit[cur_f + n - 1] + lens[orbit[cur_f + n - 1] - sec_start];
+        }
+    }
+    if (threadIdx.x == 0) *out = res;
+}
+
+__global__ void splice_orbit_kernel(const OrbitPiece* pieces, const Replay* replay, u64 n, u64* dst) {
     const u64 i = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const u32 n_pieces = replay->n_pieces;
+    if (i >= n || n_pieces == 0) return;
     u32 lo = 0, hi = n_pieces;  // the last piece with t_start <= i
     while (hi - lo > 1) {
         const u32 mid = (lo + hi) >> 1;
         if (pieces[mid].t_start <= i) lo = mid; else hi = mid;
     }
     const OrbitPiece p = pieces[lo];
-    dst[i] = p.src[i - p.t_start];
+    if (i - p.t_start < p.len) dst[i] = p.src[i - p.t_start];
 }
 
 // ---------------------------------------------------------------- count and emit
@@ -755,11 +701,6 @@ __global__ void fill_rows_kernel(const u64* o, u64 n, u64 base, u64 total, u32* 
     for (u64 i = b + (threadIdx.x & 31u); i < e; i += 32) out[i] = static_cast<u32>(r);
 }
 
-__global__ void section_end_kernel(Sec s, const u64* orbit, u64 last, int self_mode, u32 self_off, u64* end) {
-    NoVisit nv;
-    *end = walk_pre(s, orbit[last], self_post_of(self_mode, static_cast<u32>(last), self_off), nv);
-}
-
 // Excitatory edge layout, source-major: pre r's E-block edges (exc targets) then its
 // I-block edges (inh targets) at fwd_rs[r] = oe_e[r] + oe_i[r] (the two blocks'
 // exclusive scans over the same pres); o_e / o_i (the scans, in place) become each
@@ -852,68 +793,43 @@ Status guess_pool_prefix(u64 seed, u32 nN, u32 nA, u32 take, u64 c0, u64* prefix
     return Status::Ok();
 }
 
-// Resident 128-thread blocks of swarm_kernel per SM, read once.
-u32 swarm_blocks_per_sm() {
-    static std::atomic<int> cached{0};
-    int v = cached.load();
-    if (v > 0) return static_cast<u32>(v);
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, swarm_kernel, 128, 0) != cudaSuccess || nb <= 0) {
-        cudaGetLastError();
-        nb = 8;
-    }
-    cached.store(nb);
-    return static_cast<u32>(nb);
-}
-
-// The (exit, pres) table of every chunk candidate: t_exit/t_cnt[chunk * delta + d]
-// for the walk from tape position sec_start + chunk * chunk_len + d.
-// A section's chunks of swarm_min_chunk positions and more go to the warp swarms;
-// shorter ones (the shortened chunks of small networks) to one CTA per chunk, which
-// walks all candidates at once and measured faster there (N = 2e3-3e4: 0.3 vs 1.3
-// ms per section; N = 1e7: 268 ms vs 33 ms for the E block the other way round).
-Status chunk_tables(Sec s, u64 sec_start, u32 chunk_len, u32 delta, u32 n_chunks, u32 swarm_min_chunk, u32 handoff,
-                    u64* t_exit, u32* t_cnt, cudaStream_t st) {
-    // ASTROSIM_CHUNK_TABLES=cta|swarm forces one of the two (exact, equivalent) table
-    // algorithms; the tests build the same networks both ways.
-    bool cta = chunk_len < swarm_min_chunk;
-    if (const char* env = std::getenv("ASTROSIM_CHUNK_TABLES")) {
-        if (std::strcmp(env, "cta") == 0) cta = true;
-        else if (std::strcmp(env, "swarm") == 0) cta = false;
-    }
-    if (cta) {
-        table_kernel<<<n_chunks, delta, 0, st>>>(s, sec_start, chunk_len, delta, t_exit, t_cnt);
-        AS_CUDA(cudaGetLastError());
-        return Status::Ok();
-    }
-    const u64 n = static_cast<u64>(n_chunks) * delta;
-    const u32 blocks = std::max<u32>(1, std::min<u32>(ceil_div(n_chunks, 4), sm_count() * swarm_blocks_per_sm()));
-    const unsigned cont_cap = n_chunks * handoff;
-    DevBuf<unsigned long long> tables;
-    DevBuf<int> par;
-    DevBuf<u32> mycnt, pcnt;
-    DevBuf<u64> ex;
-    DevBuf<SwarmCont> cont;
-    DevBuf<unsigned> counters;  // next chunk, handed-off walks
-    AS_TRY(tables.alloc(static_cast<u64>(blocks) * 4 * kSwarmSlots));
-    AS_TRY(par.alloc(n));
-    AS_TRY(mycnt.alloc(n));
-    AS_TRY(pcnt.alloc(n));
-    AS_TRY(ex.alloc(n));
-    AS_TRY(cont.alloc(cont_cap));
-    AS_TRY(counters.alloc_zero(2, st));
-    const SwarmRec rec{par.get(), mycnt.get(), pcnt.get(), ex.get()};
-    swarm_kernel<<<blocks, 128, 0, st>>>(s, sec_start, chunk_len, delta, n_chunks, handoff, counters.get(),
-                                         tables.get(), rec, cont.get(), counters.get() + 1, cont_cap);
-    AS_CUDA(cudaGetLastError());
-    const u32 lanes = walking_lanes(cont_cap, sm_count() * 4);
-    swarm_continue_kernel<<<walk_blocks(cont_cap, lanes), kWalkBlock, ring_bytes(lanes), st>>>(
-        s, sec_start, chunk_len, delta, cont.get(), counters.get() + 1, cont_cap, rec, lanes);
-    AS_CUDA(cudaGetLastError());
-    swarm_resolve_kernel<<<ceil_div(n, 256), 256, 0, st>>>(delta, n, rec, s.err, t_exit, t_cnt);
-    AS_CUDA(cudaGetLastError());
+// Lets the kernels below use more than 48 KB of shared memory, once per device.
+Status allow_large_shared() {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    AS_CUDA(cudaGetDevice(&dev));
+    if (dev < 64 && done[dev].load()) return Status::Ok();
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    AS_CUDA(cudaFuncSetAttribute(pre_length_kernel, attr, static_cast<int>(kLenShared)));
+    AS_CUDA(cudaFuncSetAttribute(replay_kernel, attr, static_cast<int>(kReplayShared)));
+    if (dev < 64) done[dev].store(true);
     return Status::Ok();
 }
+
+// Several arrays in one allocation: a build makes hundreds of small ones otherwise, and
+// concurrent builds queue for the allocator.
+class Arena {
+public:
+    template <typename T>
+    void want(T** p, u64 n) {
+        slots_.push_back(Slot{reinterpret_cast<void**>(p), bytes_});
+        bytes_ += (n * sizeof(T) + 255) / 256 * 256;
+    }
+    Status alloc() {
+        AS_TRY(buf_.alloc(bytes_));
+        for (const Slot& s : slots_) *s.p = buf_.get() + s.at;
+        return Status::Ok();
+    }
+
+private:
+    struct Slot {
+        void** p;
+        size_t at;
+    };
+    std::vector<Slot> slots_;
+    size_t bytes_ = 0;
+    DevBuf<unsigned char> buf_;
+};
 
 struct SectionPlan {
     const char* name;
@@ -921,240 +837,126 @@ struct SectionPlan {
     int third;
     u64 n_pres;
     double draws_per_pre;
-    u32 chunk_len, delta;
+    u32 delta;
     int self_mode;  // 0: no autapse possible; 1: autapse at post == r + self_off
     u32 self_off;
     bool autapse_shifts_stream;
-    // Chunk tables by warp swarms from this chunk length up, handing off at most
-    // `handoff` walks per chunk.  The continuation and orbit walks are one serial
-    // walk per chunk, so their time follows the chunk length; the swarms' follows
-    // the number of chunks.  Measured per section (N = 3e6, ncu): shortening the I
-    // block's chunks (about 40 draws per pre) from 16384 to 4096 positions took its
-    // tables and orbit from 10.8 to 3.8 ms, and the inhibitory section's (about 80
-    // draws per pre, no third-factor draws) from 16384 to 8192 with hand-off at 6
-    // from 17.5 to 9.6 ms; the E block (about 150 draws per pre) keeps 32768 and 4
-    // (hand-off at 3: 16.9 instead of 14.4 ms).
-    u32 swarm_min_chunk, handoff;
+};
+
+// What the host reads back after a section's passes.
+struct SectionResult {
+    int err;
+    u32 end_group;
+    u64 end;
+    unsigned n_hazards;
+    u32 pad_;
+    Replay replay;
 };
 
 // Finds the start of every pre of one section (steps 3 and 4 of the file comment).
 // On success `orbit` holds n_pres starts and *end the tape position after the section.
-Status section_orbit(const SectionPlan& P, Sec s, u64 start, DevBuf<int>& err, DevBuf<u64>& orbit, u64* end,
-                     cudaStream_t st) {
-    u32 chunk_len = P.chunk_len, delta = P.delta;
+// All passes are enqueued before the one read-back.
+Status section_orbit(const SectionPlan& P, Sec s, u64 start, DevBuf<u64>& orbit, u64* end, cudaStream_t st) {
+    u32 chunk_len = kChunkLen, delta = P.delta;
     {
         const double draws = static_cast<double>(P.n_pres) * P.draws_per_pre;
         while (chunk_len > kMinChunkLen && draws / chunk_len < target_chunks()) chunk_len /= 2;
     }
     double slack = 1.04;
     int K = 32;
-    // Explicit pre starts kept per speculative re-merge walk.  Walks rejoin after a
-    // median of 2 pres (at most about 900 in every network measured, N = 2e3-1e6),
-    // and the replay uses only the 50-90 on its chain of about 5,200; so every walk
-    // stops at 64 starts and the replay continues, one at a time, the capped walks it
-    // reaches.  The kernel then waits for 64 pres instead of the longest walk.
-    const u32 max_explicit = 64;
+    constexpr u32 kPieces = 65536;
+    AS_TRY(allow_large_shared());
     PhaseClock pc(st);
     for (int attempt = 0; attempt < 8; ++attempt) {
-        AS_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
         const u64 margin = P.autapse_shifts_stream ? static_cast<u64>(K) + 16 : 0;
         const u64 target = P.n_pres + margin;
         const double est = static_cast<double>(target) * P.draws_per_pre * slack + 8.0 * chunk_len;
         const u32 n_chunks = std::max<u32>(1, static_cast<u32>(est / chunk_len) + 1);
-        const u32 n_groups = ceil_div(n_chunks, kGroup);
-        DevBuf<u64> t_exit, g_exit, g_cnt, g_entry, g_g0, c_entry, c_g0;
-        DevBuf<u32> t_cnt, endg;
-        AS_TRY(t_exit.alloc(static_cast<u64>(n_chunks) * delta));
-        AS_TRY(t_cnt.alloc(static_cast<u64>(n_chunks) * delta));
-        AS_TRY(g_exit.alloc(static_cast<u64>(n_groups) * delta));
-        AS_TRY(g_cnt.alloc(static_cast<u64>(n_groups) * delta));
-        AS_TRY(g_entry.alloc(n_groups));
-        AS_TRY(g_g0.alloc(n_groups));
-        AS_TRY(c_entry.alloc(n_chunks));
-        AS_TRY(c_g0.alloc(n_chunks));
-        AS_TRY(endg.alloc(1));
-        AS_TRY(chunk_tables(s, start, chunk_len, delta, n_chunks, P.swarm_min_chunk, P.handoff, t_exit.get(),
-                            t_cnt.get(), st));
-        group_compose_kernel<<<n_groups, delta, 0, st>>>(s, start, chunk_len, delta, n_chunks, t_exit.get(),
-                                                         t_cnt.get(), g_exit.get(), g_cnt.get());
-        AS_CUDA(cudaGetLastError());
-        top_compose_kernel<<<1, 1, 0, st>>>(s, start, chunk_len, delta, n_groups, g_exit.get(), g_cnt.get(), target,
-                                            g_entry.get(), g_g0.get(), endg.get());
-        AS_CUDA(cudaGetLastError());
-        int herr = 0;
-        u32 hend = 0;
-        AS_TRY(read_err(err, &herr, st));
-        AS_TRY(to_host(&hend, endg.get(), 1, st));
-        pc.mark("  chunk tables + composition");
-        if (herr & kErrHash) { chunk_len /= 2; continue; }
-        if (herr & kErrDelta) {
-            if (delta >= kMaxDelta) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: a pre longer than %u draws", P.name, kMaxDelta);
-            delta = std::min<u32>(kMaxDelta, delta * 2);
-            continue;
+        // groups of about the square root: the compositions follow a group's chunks, then the groups
+        u32 group = 8;
+        while (group < 64 && group * group < n_chunks) group *= 2;
+        const u32 n_groups = ceil_div(n_chunks, group);
+        const u64 n_lens = static_cast<u64>(n_chunks) * chunk_len;
+        const unsigned hz_cap =
+            P.autapse_shifts_stream ? static_cast<unsigned>(std::min<double>(4e6, 200.0 * (2 * K + 1) + 4096)) : 0;
+        Arena mem;
+        u16* lens = nullptr;
+        u64 *t_exit = nullptr, *g_exit = nullptr, *g_cnt = nullptr, *g_entry = nullptr, *g_g0 = nullptr,
+            *c_entry = nullptr, *c_g0 = nullptr, *forbit = nullptr, *starts = nullptr;
+        u32* t_cnt = nullptr;
+        Hazard* hz = nullptr;
+        OrbitPiece* pieces = nullptr;
+        SectionResult* res = nullptr;
+        mem.want(&lens, n_lens);
+        mem.want(&t_exit, static_cast<u64>(n_chunks) * delta);
+        mem.want(&t_cnt, static_cast<u64>(n_chunks) * delta);
+        mem.want(&g_exit, static_cast<u64>(n_groups) * delta);
+        mem.want(&g_cnt, static_cast<u64>(n_groups) * delta);
+        mem.want(&g_entry, n_groups);
+        mem.want(&g_g0, n_groups);
+        mem.want(&c_entry, n_chunks);
+        mem.want(&c_g0, n_chunks);
+        mem.want(&res, 1);
+        if (P.autapse_shifts_stream) {
+            mem.want(&forbit, target);
+            mem.want(&hz, hz_cap);
+            mem.want(&starts, P.n_pres + kReplayBatch);
+            mem.want(&pieces, kPieces);
         }
-        if (herr & kErrCache) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s walk left the skip cache", P.name);
-        if (hend >= n_groups) { slack *= 1.25; continue; }
-        const u32 used_groups = hend + 1;
-        const u32 used_chunks = std::min<u32>(n_chunks, used_groups * kGroup);
-        // sentinel entries: a chunk left unset would start past every chunk end and write nothing
-        AS_CUDA(cudaMemsetAsync(c_entry.get(), 0xFF, c_entry.bytes(), st));
-        AS_CUDA(cudaMemsetAsync(c_g0.get(), 0xFF, c_g0.bytes(), st));
-        chunk_entry_kernel<<<ceil_div(used_groups, 128), 128, 0, st>>>(s, start, chunk_len, delta, n_chunks,
-                                                                       used_groups, t_exit.get(), t_cnt.get(),
-                                                                       g_entry.get(), g_g0.get(), c_entry.get(),
-                                                                       c_g0.get());
+        AS_TRY(mem.alloc());
+        AS_TRY(orbit.alloc(P.n_pres));
+        AS_CUDA(cudaMemsetAsync(res, 0, sizeof(SectionResult), st));
+        s.err = &res->err;
+        u64* const table_orbit = P.autapse_shifts_stream ? forbit : orbit.get();
+        pre_length_kernel<<<ceil_div(n_lens, kLenTile), kLenBlock, kLenShared, st>>>(s, start, n_lens, lens);
         AS_CUDA(cudaGetLastError());
-        AS_TRY(read_err(err, &herr, st));
-        if (herr & kErrDelta) {
-            if (delta >= kMaxDelta) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: a pre longer than %u draws", P.name, kMaxDelta);
-            delta = std::min<u32>(kMaxDelta, delta * 2);
-            continue;
-        }
-        DevBuf<u64> forbit;
-        AS_TRY(forbit.alloc(target));
-        const u32 lanes = walking_lanes(used_chunks, sm_count() * 4);
-        materialize_kernel<<<walk_blocks(used_chunks, lanes), kWalkBlock, ring_bytes(lanes), st>>>(
-            s, start, chunk_len, used_chunks, c_entry.get(), c_g0.get(), target, forbit.get(), lanes);
+        table_kernel<<<n_chunks, delta, chunk_len * sizeof(u16), st>>>(s, lens, start, chunk_len, delta, t_exit, t_cnt);
         AS_CUDA(cudaGetLastError());
-        AS_TRY(read_err(err, &herr, st));
-        if (herr & kErrDelta) {
-            if (delta >= kMaxDelta) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: a pre longer than %u draws", P.name, kMaxDelta);
-            delta = std::min<u32>(kMaxDelta, delta * 2);
-            continue;
-        }
-        if (herr) return make_error(ASTROSIM_ERR_CUDA, "%s orbit materialisation failed (flags %d)", P.name, herr);
-        pc.mark("  chunk entries + orbit");
-
-        if (!P.autapse_shifts_stream) {
-            orbit = std::move(forbit);
-            DevBuf<u64> e;
-            AS_TRY(e.alloc(1));
-            section_end_kernel<<<1, 1, 0, st>>>(s, orbit.get(), P.n_pres - 1, P.self_mode, P.self_off, e.get());
+        group_compose_kernel<<<n_groups, delta, 0, st>>>(s, start, chunk_len, delta, n_chunks, group, t_exit, t_cnt,
+                                                         g_exit, g_cnt);
+        AS_CUDA(cudaGetLastError());
+        top_compose_kernel<<<1, 1, 0, st>>>(s, start, chunk_len, delta, n_groups, group, g_exit, g_cnt, target, g_entry,
+                                            g_g0, &res->end_group);
+        AS_CUDA(cudaGetLastError());
+        chunk_entry_kernel<<<ceil_div(n_groups, 32), 32, 0, st>>>(s, start, chunk_len, delta, n_chunks, n_groups, group,
+                                                                  t_exit, t_cnt, g_entry, g_g0, &res->end_group,
+                                                                  c_entry, c_g0);
+        AS_CUDA(cudaGetLastError());
+        materialize_kernel<<<n_chunks, 128, chunk_len * sizeof(u16), st>>>(s, lens, start, chunk_len, n_chunks, c_entry,
+                                                                           c_g0, target, P.n_pres - 1, table_orbit,
+                                                                           &res->end);
+        AS_CUDA(cudaGetLastError());
+        if (P.autapse_shifts_stream) {
+            hazard_kernel<<<ceil_div(target, 128), 128, 0, st>>>(s, table_orbit, target, K, hz, &res->n_hazards, hz_cap,
+                                                                 &res->end_group, n_groups);
             AS_CUDA(cudaGetLastError());
-            AS_TRY(to_host(end, e.get(), 1, st));
+            replay_kernel<<<1, kReplayBlock, kReplayShared, st>>>(s, lens, start, n_lens, hz, &res->n_hazards, hz_cap,
+                                                                  table_orbit, target, P.n_pres, K, &res->end_group,
+                                                                  n_groups, starts, pieces, kPieces, &res->replay);
+            AS_CUDA(cudaGetLastError());
+            splice_orbit_kernel<<<ceil_div(P.n_pres, 256), 256, 0, st>>>(pieces, &res->replay, P.n_pres, orbit.get());
+            AS_CUDA(cudaGetLastError());
+        }
+        SectionResult h{};
+        AS_TRY(to_host(&h, res, 1, st));
+        pc.mark("  lengths, tables, orbit");
+        if (h.err & kErrDelta) {
+            if (delta >= kMaxDelta) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: a pre longer than %u draws", P.name, kMaxDelta);
+            delta = std::min<u32>(kMaxDelta, delta * 2);
+            continue;
+        }
+        if (h.err & kErrCache) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s walk left the draw cache", P.name);
+        if (h.end_group >= n_groups) { slack *= 1.25; continue; }
+        if (h.err) return make_error(ASTROSIM_ERR_CUDA, "%s orbit materialisation failed (flags %d)", P.name, h.err);
+        if (!P.autapse_shifts_stream) {
+            *end = h.end;
             return Status::Ok();
         }
-
-        // ---- autapses of the E block (step 4)
-        const unsigned hz_cap = static_cast<unsigned>(std::min<double>(4e6, 200.0 * (2 * K + 1) + 4096));
-        DevBuf<Hazard> hz;
-        DevBuf<unsigned> hz_n;
-        AS_TRY(hz.alloc(hz_cap));
-        AS_TRY(hz_n.alloc_zero(1, st));
-        hazard_kernel<<<ceil_div(target, 128), 128, 0, st>>>(s, forbit.get(), target, K, hz.get(), hz_n.get(),
-                                                             hz_cap);
-        AS_CUDA(cudaGetLastError());
-        unsigned n_hz = 0;
-        AS_TRY(to_host(&n_hz, hz_n.get(), 1, st));
-        if (n_hz > hz_cap)
-            return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: %u autapse hazards exceed the buffer", P.name, n_hz);
-        std::vector<Hazard> hh(n_hz);
-        if (n_hz) AS_TRY(to_host(hh.data(), hz.get(), n_hz, st));
-        std::sort(hh.begin(), hh.end(), [](const Hazard& a, const Hazard& b) {
-            return a.r != b.r ? a.r < b.r : a.d < b.d;
-        });
-        pc.mark("  autapse hazards");
-        // speculative exact walks from every hazard
-        DevBuf<Hazard> hz_sorted;
-        DevBuf<Remerge> rm;
-        DevBuf<u64> expl;
-        AS_TRY(hz_sorted.alloc(std::max<unsigned>(1, n_hz)));
-        AS_TRY(rm.alloc(std::max<unsigned>(1, n_hz)));
-        AS_TRY(expl.alloc(static_cast<u64>(std::max<unsigned>(1, n_hz)) * max_explicit));
-        std::vector<Remerge> rr(n_hz);
-        if (n_hz) {
-            AS_CUDA(cudaMemcpyAsync(hz_sorted.get(), hh.data(), n_hz * sizeof(Hazard), cudaMemcpyHostToDevice, st));
-            const u32 walk_lanes = walking_lanes(n_hz, sm_count() * 4);
-            remerge_kernel<<<walk_blocks(n_hz, walk_lanes), kWalkBlock, ring_bytes(walk_lanes), st>>>(
-                s, hz_sorted.get(), n_hz, forbit.get(), target, P.n_pres, max_explicit, expl.get(), rm.get(),
-                walk_lanes);
-            AS_CUDA(cudaGetLastError());
-            AS_TRY(to_host(rr.data(), rm.get(), n_hz, st));
-            AS_TRY(read_err(err, &herr, st));
-            if (herr) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: re-merge walks failed (flags %d)", P.name, herr);
-        }
-        pc.mark("  re-merge walks");
-        // replay the hazards in order with the running shift (true index - table index)
-        struct Piece { const u64* src; u64 t_start, len; };
-        std::vector<Piece> pieces;
-        std::vector<DevBuf<u64>> cont_starts;  // starts of the capped walks the replay continued
-        DevBuf<Remerge> cont_res;
-        AS_TRY(cont_res.alloc(1));
-        long long d = 0;
-        u64 cur_f = 0, cur_t = 0;
-        bool ended = false;
-        u64 end_pos = 0;
-        bool shift_overflow = false;
-        for (unsigned i = 0; i < n_hz && !ended; ++i) {
-            const Hazard& h = hh[i];
-            if (h.r < cur_f || h.d != d) continue;
-            if (static_cast<long long>(h.r) + d >= static_cast<long long>(P.n_pres)) break;  // past the section
-            Remerge m = rr[i];
-            if (h.r > cur_f) pieces.push_back(Piece{forbit.get() + cur_f, cur_t, h.r - cur_f});
-            const u64 t_autapse = static_cast<u64>(static_cast<long long>(h.r) + d);
-            pieces.push_back(Piece{expl.get() + static_cast<u64>(i) * max_explicit, t_autapse, m.m});
-            u64 walked = m.m;
-            // This walk is on the chain: continue it from where it stopped (its tape
-            // position and true index are all the state it has), in pieces of growing
-            // size, until it rejoins the table orbit or the section ends.
-            for (u32 cap = 4096; m.capped; cap = std::min<u32>(cap * 8, 1u << 24)) {
-                DevBuf<u64> buf;
-                AS_TRY(buf.alloc(cap));
-                remerge_continue_kernel<<<1, 32, 0, st>>>(s, m.c_next, m.r_next, forbit.get(), target, P.n_pres, cap,
-                                                         buf.get(), cont_res.get());
-                AS_CUDA(cudaGetLastError());
-                Remerge m2{};
-                AS_TRY(to_host(&m2, cont_res.get(), 1, st));
-                pieces.push_back(Piece{buf.get(), t_autapse + walked, m2.m});
-                walked += m2.m;
-                cont_starts.push_back(std::move(buf));
-                m = m2;
-            }
-            if (!m.ok) return make_error(ASTROSIM_ERR_CUDA, "%s: re-merge walk incomplete", P.name);
-            if (m.k < 0) {
-                ended = true;
-                end_pos = m.end;
-                cur_t = t_autapse + walked;
-                break;
-            }
-            cur_t = t_autapse + walked;
-            cur_f = static_cast<u64>(m.k);
-            d = m.shift;
-            if (d < -K || d > K) { shift_overflow = true; break; }
-        }
-        if (shift_overflow) { K *= 4; continue; }
-        if (!ended) {
-            const u64 len = P.n_pres - cur_t;
-            if (cur_f + len > target) { K *= 4; continue; }  // needed table orbit beyond the margin
-            if (len) pieces.push_back(Piece{forbit.get() + cur_f, cur_t, len});
-            cur_t += len;
-        }
-        if (cur_t != P.n_pres) return make_error(ASTROSIM_ERR_CUDA, "%s: spliced orbit has %llu of %llu pres", P.name,
-                                                 static_cast<unsigned long long>(cur_t),
-                                                 static_cast<unsigned long long>(P.n_pres));
-        AS_TRY(orbit.alloc(P.n_pres));
-        std::vector<OrbitPiece> table;
-        for (const Piece& pc : pieces)
-            if (pc.len) table.push_back(OrbitPiece{pc.src, pc.t_start, pc.len});
-        if (!table.empty()) {
-            DevBuf<OrbitPiece> dtab;
-            AS_TRY(dtab.alloc(table.size()));
-            AS_CUDA(cudaMemcpyAsync(dtab.get(), table.data(), table.size() * sizeof(OrbitPiece),
-                                    cudaMemcpyHostToDevice, st));
-            splice_orbit_kernel<<<ceil_div(P.n_pres, 256), 256, 0, st>>>(dtab.get(), static_cast<u32>(table.size()),
-                                                                         P.n_pres, orbit.get());
-            AS_CUDA(cudaGetLastError());
-            AS_CUDA(cudaStreamSynchronize(st));  // the host table
-        }
-        if (ended) {
-            *end = end_pos;
-        } else {
-            DevBuf<u64> e;
-            AS_TRY(e.alloc(1));
-            section_end_kernel<<<1, 1, 0, st>>>(s, orbit.get(), P.n_pres - 1, P.self_mode, P.self_off, e.get());
-            AS_CUDA(cudaGetLastError());
-            AS_TRY(to_host(end, e.get(), 1, st));
-        }
+        if (h.n_hazards > hz_cap)
+            return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: %u autapse hazards exceed the buffer", P.name, h.n_hazards);
+        if (h.replay.full) return make_error(ASTROSIM_ERR_UNSUPPORTED, "%s: more than %u orbit pieces", P.name, kPieces);
+        if (h.replay.retry) { K *= 4; slack *= 1.05; continue; }
+        *end = h.replay.end;
         return Status::Ok();
     }
     return make_error(ASTROSIM_ERR_CUDA, "%s: chunked walk did not settle", P.name);
@@ -1211,15 +1013,15 @@ Status build_parallel(const Sizes& sz, u64 seed, u64 c0, Network& net, cudaStrea
     if (nN >= kSkipMax) return make_error(ASTROSIM_ERR_OUT_OF_MEMORY, "%u neurons need a draw cache of over 100 GB", nN);
     const double ne = sz.n_exc, ni = sz.n_inh, nn = nN, p = sz.p;
     SectionPlan plans[3] = {
-        {"E block", sz.n_exc, 0, 1, sz.n_exc, 1.0 + p * ne * (2.0 + kPThird), 32768, 384, 1, 0, true, 16384, 4},
-        {"I block", sz.n_inh, sz.n_exc, 1, sz.n_exc, 1.0 + p * ni * (2.0 + kPThird), 4096, 192, 0, 0, false, 4096, 4},
-        {"inhibitory", nN, 0, 0, sz.n_inh, 1.0 + p * nn, 8192, 192, 1, sz.n_exc, false, 8192, 6},
+        {"E block", sz.n_exc, 0, 1, sz.n_exc, 1.0 + p * ne * (2.0 + kPThird), 384, 1, 0, true},
+        {"I block", sz.n_inh, sz.n_exc, 1, sz.n_exc, 1.0 + p * ni * (2.0 + kPThird), 192, 0, 0, false},
+        {"inhibitory", nN, 0, 0, sz.n_inh, 1.0 + p * nn, 192, 1, sz.n_exc, false},
     };
     double est_total = 0.0;
     for (const auto& P : plans) est_total += static_cast<double>(P.n_pres) * P.draws_per_pre;
     const u64 cache_len = static_cast<u64>(est_total * 1.12) + 64ull * 65536 + 1000000;
     DevBuf<u32> cache;
-    AS_TRY(cache.alloc(cache_words(cache_len)));
+    AS_TRY(cache.alloc(cache_len));
     const double L = std::log1p(-p);  // host value, as the reference computes it (src/astrosim_fused.cu:622)
     {
         DevBuf<u64> amb_pos;
@@ -1261,7 +1063,7 @@ Status build_parallel(const Sizes& sz, u64 seed, u64 c0, Network& net, cudaStrea
         s.post_off = plans[k].post_off;
         s.third = plans[k].third;
         u64 end = 0;
-        AS_TRY(section_orbit(plans[k], s, start, err, orbits[k], &end, st));
+        AS_TRY(section_orbit(plans[k], s, start, orbits[k], &end, st));
         start = end;
         pc.mark(plans[k].name);
     }

@@ -34,7 +34,7 @@ double now_s() {
 u64 Server::estimate_bytes(const astrosim_config& cfg) {
     // Resident: target and source-keyed CSRs (~8 B per synapse, 116 synapses per
     // neuron), state and window buffers (~300 B per neuron); while building, edge
-    // lists, the skip cache and sort buffers roughly double that.  Measured at
+    // lists, the draw cache and sort buffers roughly double that.  Measured at
     // N = 1e7 the resident total is about 15 GB.
     const double n = cfg.n_total;
     return static_cast<u64>(n * 3200.0) + (64ull << 20);

@@ -5,7 +5,9 @@
 // give, whether it passes the third-factor test and which pool entry it would pick.  The
 // cache holds all three in one word per position, so a walk is a chain of cached words
 // and needs no hashing: a landing costs one load latency instead of a load after a dependent
-// hash (one thread walking one pre after the other: 260 ns per landing with hashes).
+// hash.  And because where a pre that starts at a position ends is then a function of that
+// position alone (but for its autapse), the lengths of the pres at all positions are
+// computed in parallel, and walking pre after pre is one table read per pre.
 //
 // Device code, also compiled on the host by CPU tests (tests/walk_equivalence.cpp,
 // tests/walk_words.cpp) that supply __ldg and atomicOr.
@@ -18,8 +20,7 @@ namespace astrosim {
 constexpr u32 kNoSelf = 0xFFFFFFFFu;  // no autapse rule for this walk
 
 enum ErrBits : int {
-    kErrCache = 1,     // a walk left the skip cache
-    kErrHash = 2,      // claim table full
+    kErrCache = 1,     // a walk left the draw cache
     kErrDelta = 4,     // an entry fell outside the candidate window
     kErrOrbit = 8      // materialised chunk did not meet its successor (internal)
 };
@@ -130,143 +131,65 @@ __device__ __forceinline__ u64 walk_pre_end(const Sec& s, u64 c, u32 self_post) 
     return walk_pre(s, c, self_post, nv);
 }
 
-// A stretch of consecutive pres as a machine that makes one landing per step, pre ends
-// included: the lanes of a warp then stay together whatever their pres' lengths.  It holds
-// the words around its place, so that a step is a short chain of selections; the words
-// that it may need next are read behind it.  `at` is the cache index after the current
-// skip's, less `origin`.  It draws exactly what walk_pre draws, pre after pre.
-struct Stretch {
-    u64 origin;
-    u32 at, rem;           // rem: posts left in the current pre's block
-    u32 skip, test, a1, a2, a3;  // the words at - 1, at, at + 1, at + 2, at + 3
-    // From tape position c, with cache index `first` of its segment as the origin.
-    __device__ __forceinline__ Stretch(const Sec& s, u64 c, u64 first)
-        : origin(first), at(static_cast<u32>(c - s.cache_base - first) + 1), rem(s.post_count), skip(0), test(0), a1(0),
-          a2(0), a3(0) {}
-    template <class Word>
-    __device__ __forceinline__ void begin(Word word) {
-        skip = word(at - 1);
-        test = word(at);
-        a1 = word(at + 1);
-        a2 = word(at + 2);
-        a3 = word(at + 3);
-    }
-    // When a pre has just ended: the next one's start (its skip is already taken).
-    __device__ __forceinline__ u64 start(const Sec& s) const { return s.cache_base + origin + at - 1; }
-    // Past the cache: the current skip (a walk that goes on), or a draw before start().
-    __device__ __forceinline__ bool out(const Sec& s) const { return origin + at > s.cache_len; }
-    __device__ __forceinline__ bool overran(const Sec& s) const { return origin + at - 1 > s.cache_len; }
-    // `self_post`: the current pre's autapse.  Returns true when the pre ended.
-    template <class Word>
-    __device__ __forceinline__ bool step(const Sec& s, u32 self_post, Word word) {
-        const u32 g = skip & kSkipMax, n = s.post_count;
-        const bool past = g >= rem;
-        const bool self = s.post_off + (n - rem) + g == self_post;
-        const bool tested = s.third && !past && !self;
-        const bool hit = tested && (test & kHitBit);
-        const u32 left = rem - g - 1;
-        const bool ended = past || left == 0;
-        rem = ended ? n : left;
-        at += hit ? 3u : (tested ? 2u : 1u);
-        skip = hit ? a2 : (tested ? a1 : test);
-        test = hit ? a3 : (tested ? a2 : a1);
-        a1 = word(at + 1);
-        a2 = word(at + 2);
-        a3 = word(at + 3);
-        return ended;
-    }
-};
+// ------------------------------------------------------------------ pre lengths
+// How many draws a pre takes that starts at a tape position, for every position.  A walk
+// of a pre moves on by landings, and where a landing at a position leads does not depend
+// on how the walk got there; so the landings are first joined into jumps of 4 and of 16
+// (their posts passed and draws taken added up), and a pre is then a few jumps that stay
+// inside its block and the last landings one by one: about 8 steps instead of 68.
+constexpr u32 kMaxPre = 512;         // the longest pre, in draws (E block: 178 on average)
+constexpr u32 kLongPre = 0xFFFF;     // a longer one
+constexpr u32 kJumpFull = (1u << 26) - 1;  // posts of a jump that passes more than fit
 
-#ifdef __CUDACC__
-// The tape ahead of a warp's stretches: a ring of four segments of 32 words per walking
-// lane in shared memory, filled by asynchronous copies.  One thread walks one stretch of
-// the tape after another; reading the cache directly, some lane of the warp crossed into
-// a new 32-byte sector at every landing and the warp waited for it: 650 ns per landing
-// from DRAM (N = 3e5), 230 ns from L2 (N = 1e3).  Every kRefill landings all lanes top
-// up together (the copies of a warp are counted together, so a lane that waited for its
-// own would wait for the others' newest) and copies have two more refills to arrive.
-// The cache is padded past its end to whole segments (cache_words).
-constexpr u32 kSegment = 32, kRingSegments = 4, kRefill = 8;
-constexpr u32 kRingWords = kRingSegments * kSegment + 4;  // an odd number of 16-byte units: lanes spread over the banks
-static_assert(3 * kRefill + 4 <= kSegment, "a refill of one segment keeps up with the walk");
-inline __host__ __device__ u64 cache_words(u64 len) { return (len / kSegment + 2 * kRingSegments) * kSegment; }
-
-struct TapeRing {
-    u32* ring;   // this lane's kRingWords
-    u64 first;   // the segment that the stretch starts in
-    u32 filled;  // segments from `first` on that are in the ring or on their way
-    __device__ __forceinline__ void fetch(const Sec& s) {
-        const u64 g = first + filled;
-        const u32 slot = filled++ & (kRingSegments - 1);
-        if (g >= cache_words(s.cache_len) / kSegment) return;  // a walk that left the cache
-        const u32* from = s.cache + g * kSegment;
-        const u32 to = static_cast<u32>(__cvta_generic_to_shared(ring + slot * kSegment));
-#pragma unroll
-        for (u32 k = 0; k < kSegment / 4; ++k)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * k), "l"(from + 4 * k) : "memory");
+// posts << 6 | draws
+__host__ __device__ __forceinline__ u32 landing_jump(const Sec& s, u32 skip_word, u32 test_word) {
+    const u32 g = skip_word & kSkipMax;
+    const u32 posts = g >= kJumpFull ? kJumpFull : g + 1;
+    return posts << 6 | (s.third ? ((test_word & kHitBit) ? 3u : 2u) : 1u);
+}
+__host__ __device__ __forceinline__ u32 join_jumps(u32 a, u32 b) {
+    const u32 posts = (a >> 6) + (b >> 6);
+    return (posts < kJumpFull ? posts : kJumpFull) << 6 | ((a & 63u) + (b & 63u));
+}
+// Four landings from index i of `words`.
+__host__ __device__ __forceinline__ u32 jump4(const Sec& s, const u32* words, u32 i) {
+    u32 j = 0;
+    for (int k = 0; k < 4; ++k) j = join_jumps(j, landing_jump(s, words[i + (j & 63u)], words[i + (j & 63u) + 1]));
+    return j;
+}
+// Sixteen, from the jumps of four.
+__host__ __device__ __forceinline__ u32 jump16(const u32* jumps4, u32 i) {
+    u32 j = 0;
+    for (int k = 0; k < 4; ++k) j = join_jumps(j, jumps4[i + (j & 63u)]);
+    return j;
+}
+// The draws of the pre that starts at index i (kLongPre: more than kMaxPre).
+__host__ __device__ __forceinline__ u32 pre_length(const Sec& s, const u32* words, const u32* jumps4,
+                                                   const u32* jumps16, u32 i) {
+    u32 at = i, left = s.post_count;
+    for (u32 j = jumps16[at]; (j >> 6) < left && (j >> 6) != kJumpFull; j = jumps16[at]) {
+        left -= j >> 6;
+        at += j & 63u;
+        if (at - i > kMaxPre) return kLongPre;
     }
-    __device__ __forceinline__ TapeRing(const Sec& s, u32* shared, bool live, u64 c)
-        : ring(shared), first((c - s.cache_base) / kSegment), filled(0) {
-        if (live)
-            for (u32 k = 0; k < kRingSegments; ++k) fetch(s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    for (u32 j = jumps4[at]; (j >> 6) < left && (j >> 6) != kJumpFull; j = jumps4[at]) {
+        left -= j >> 6;
+        at += j & 63u;
+        if (at - i > kMaxPre) return kLongPre;
     }
-    // Every lane of the warp, every kRefill landings.
-    __device__ __forceinline__ void refill(const Sec& s, bool live, u32 at) {
-        if (live && filled < (at - 1) / kSegment + kRingSegments) fetch(s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
-    }
-    __device__ __forceinline__ u32 word(u32 i) const { return ring[i & (kRingSegments * kSegment - 1)]; }
-};
-
-// The lane's stretch from tape position c (when live), on its ring in `shared`: on_pre(start)
-// is called at every pre end with the next pre's start and says whether to go on; self()
-// names the current pre's autapse.  Every lane of the warp takes part.
-template <class OnPre, class Self>
-__device__ __forceinline__ void walk_stretch(const Sec& s, u64 c, bool live, u32* shared, OnPre on_pre, Self self) {
-    live = live && s.post_count != 0;
-    if (live && c - s.cache_base >= s.cache_len) {
-        atomicOr(s.err, kErrCache);
-        live = false;
-    }
-    if (!live) c = s.cache_base;
-    TapeRing ring(s, shared, live, c);
-    Stretch w(s, c, ring.first * kSegment);
-    auto word = [&](u32 i) { return ring.word(i); };
-    if (live) w.begin(word);
-    while (__any_sync(0xffffffffu, live)) {
-        if (live) {
-#pragma unroll
-            for (u32 k = 0; k < kRefill; ++k) {
-                if (w.step(s, self(), word)) {
-                    if (w.overran(s)) {
-                        atomicOr(s.err, kErrCache);
-                        live = false;
-                    } else {
-                        live = on_pre(w.start(s));
-                    }
-                    if (!live) break;
-                }
-            }
-            if (live && w.out(s)) {
-                atomicOr(s.err, kErrCache);
-                live = false;
-            }
+    while (at - i <= kMaxPre) {
+        const u32 g = words[at] & kSkipMax;
+        if (g >= left) {  // the skip reaches the end of the block
+            ++at;
+            break;
         }
-        __syncwarp();
-        ring.refill(s, live, w.at);
+        left -= g + 1;
+        at += landing_jump(s, words[at], words[at + 1]) & 63u;
+        if (left == 0) break;
     }
+    return at - i > kMaxPre ? kLongPre : at - i;
 }
-
-// Walks per warp for `walks` stretches: all 32 lanes when there are warps enough for every
-// scheduler, fewer otherwise, because a warp waits whenever one of its lanes ends a pre.
-inline u32 walking_lanes(u64 walks, u32 schedulers) {
-    u32 lanes = 32;
-    while (lanes > 1 && walks * 2 / lanes <= 2ull * schedulers) lanes /= 2;
-    return lanes;
-}
-#endif
+// Words that pre_length may read past index i, and those its jumps start at.
+constexpr u32 kWordsAhead = kMaxPre + 64, kJumpsAhead = kMaxPre + 48;
 
 }  // namespace astrosim

@@ -13,6 +13,7 @@ def test_cached_walk_makes_the_streams_draws(tmp_path):
                     os.path.join(HERE, "walk_words.cpp")], check=True)
     r = subprocess.run([str(exe), "500"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
-    m = re.search(r"walks (\d+) mismatches (\d+) cache_overruns (\d+) hits (\d+)", r.stdout)
+    m = re.search(r"walks (\d+) mismatches (\d+) cache_overruns (\d+) hits (\d+) lengths (\d+) long (\d+)", r.stdout)
     assert m and int(m.group(1)) == 20000 and int(m.group(2)) == 0
     assert int(m.group(3)) > 0 and int(m.group(4)) > 0
+    assert int(m.group(5)) > 100000 and int(m.group(6)) > 0

@@ -3,7 +3,9 @@
 // positions, walk_pre on the cached words visits the posts, third-factor results and
 // pool picks, and ends at the position, of a walk that makes every draw from the counter
 // stream itself in the reference's order (src/astrosim_fused.cu:617-624, 688-723).
+// The pre lengths joined from jumps are those of the same walk, at every position.
 // Test infrastructure.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -54,7 +56,7 @@ static u64 plain_walk(const Sec& s, double L, u64 c, u32 self, std::vector<Visit
 int main(int argc, char** argv) {
     const int trials = argc > 1 ? std::atoi(argv[1]) : 500;
     std::mt19937_64 rng(11);
-    long walks = 0, bad = 0, overruns = 0, hits = 0;
+    long walks = 0, bad = 0, overruns = 0, hits = 0, lengths = 0, longs = 0;
     for (int trial = 0; trial < trials; ++trial) {
         const u64 len = 500 + rng() % 6000;
         const double p = trial % 5 == 0 ? 1e-9 : 0.01 + static_cast<double>(rng() % 1000) / 1000.0 * 0.8;
@@ -63,7 +65,7 @@ int main(int argc, char** argv) {
         s.seed = rng();
         s.cache_base = rng() % 100000;
         s.cache_len = len;
-        s.post_count = static_cast<u32>(rng() % 400);
+        s.post_count = static_cast<u32>(rng() % (trial % 3 ? 400 : 1500));
         s.post_off = static_cast<u32>(rng() % 5000);
         s.third = static_cast<int>(rng() % 4 != 0);
         s.take = 1 + static_cast<u32>(rng() % 5);
@@ -75,6 +77,21 @@ int main(int argc, char** argv) {
         }
         s.cache = cache.data();
         s.pool = pool.data();
+        // the lengths of the pres at every position against the plain walk's
+        std::vector<u32> words(len + kWordsAhead + 64, 0xFFFFFFFFu), jumps4(len + kJumpsAhead + 48), jumps16(len + kJumpsAhead);
+        std::copy(cache.begin(), cache.end(), words.begin());
+        for (u64 i = 0; i < len + kJumpsAhead + 36; ++i) jumps4[i] = jump4(s, words.data(), static_cast<u32>(i));
+        for (u64 i = 0; i < len + kJumpsAhead; ++i) jumps16[i] = jump16(jumps4.data(), static_cast<u32>(i));
+        for (u64 i = 0; s.post_count && i < len; i += 1 + rng() % 7) {
+            std::vector<Visit> none;
+            const u64 draws = plain_walk(s, L, s.cache_base + i, kNoSelf, none) - s.cache_base - i;
+            if (i + draws > len) continue;  // past the cache, where the lengths are not used
+            ++lengths;
+            if (pre_length(s, words.data(), jumps4.data(), jumps16.data(), static_cast<u32>(i)) !=
+                (draws > kMaxPre ? kLongPre : draws))
+                ++bad;
+            longs += draws > kMaxPre;
+        }
         for (int w = 0; w < 40; ++w) {
             const u64 c0 = s.cache_base + rng() % len;
             const u32 self = rng() % 2 ? kNoSelf : s.post_off + static_cast<u32>(rng() % (s.post_count + 1));
@@ -93,6 +110,7 @@ int main(int argc, char** argv) {
             }
         }
     }
-    std::printf("walks %ld mismatches %ld cache_overruns %ld hits %ld\n", walks, bad, overruns, hits);
+    std::printf("walks %ld mismatches %ld cache_overruns %ld hits %ld lengths %ld long %ld\n", walks, bad, overruns, hits,
+                lengths, longs);
     return bad != 0;
 }
