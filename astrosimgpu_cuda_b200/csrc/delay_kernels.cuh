@@ -1,0 +1,271 @@
+// delay_kernels.cuh -- stepping with delays that the windowed engine does not take
+// (unequal ones, one step, or more than 16 steps).
+//
+// A cell's step reads only spikes and SIC factors that are at least min(d) steps old, so
+// one launch advances every cell by a window of up to min(d) steps (at most 16) without
+// any cell waiting for another; the state stays in registers.  A launch per step took
+// 20.5 us a step at N = 20011 (FP64), most of it in the rows' walk by one thread per
+// cell; windows of six steps take FIGURE.
+//
+// A window's spikes are one word per neuron (bit s: a spike at its step s), kept for
+// as many windows as the longest delay reaches back, so one load of a source tells its
+// spikes at all delayed steps of the window, and one bit per neuron (any spike in the
+// window) spares most of those loads.  The values that spikes carry and the SIC
+// factors are in rings by step; the words say which entries mean something.
+#pragma once
+
+#include "window_kernels.cuh"
+
+namespace astrosim {
+
+// Where the delayed steps of a window lie, for one delay d = q W + shift: step s of window
+// k sees step s - shift of window k - q, or for s < shift step s - shift + W of window
+// k - q - 1.
+struct Delayed {
+    u32 row, row_before;  // their rows in the rings of words
+    u32 shift;
+    u32 slot;             // ring slot that step 0 of the window sees
+};
+
+// One launch: steps [s_begin, s_end) of the window that starts at step `start`.
+struct DelayWindow {
+    i64 start, mark;  // mark: the step at which the pre-run ends
+    int W, s_begin, s_end;
+    u32 row, row_next;     // the window's and the next one's rows of words
+    u32 slot, slots;       // step 0's ring slot, slots of the ring
+    Delayed e, i, a2n;
+};
+
+// Shared memory of a warp: per step and lane three sums (excitatory or IP3, inhibitory,
+// SIC), and before them, in the same place, its background draws.
+template <typename R>
+__host__ __device__ __forceinline__ u32 delay_warp_bytes(int W) {
+    const u32 sums = 32 * 3 * static_cast<u32>(W) * static_cast<u32>(sizeof(R));
+    const u32 draws = 32 * (static_cast<u32>(W) * static_cast<u32>(sizeof(u32)) + count_bytes(1));
+    return sums > draws ? sums : draws;
+}
+template <typename R>
+inline size_t delay_shared_bytes(int W, int block) {
+    return static_cast<size_t>(block / 32) * delay_warp_bytes<R>(W);
+}
+
+__device__ __forceinline__ u32 delayed_steps(const u32* __restrict__ words, u64 n, const Delayed& d, int W, u32 src) {
+    u32 m = words[d.row * n + src] << d.shift;
+    if (d.shift) m |= words[d.row_before * n + src] >> (W - static_cast<int>(d.shift));
+    return m;
+}
+__device__ __forceinline__ u32 delayed_slot(const DelayWindow& w, const Delayed& d, int s) {
+    const u32 slot = d.slot + static_cast<u32>(s);
+    return slot >= w.slots ? slot - w.slots : slot;
+}
+
+// Sums, for every step in `steps`, the delayed spike values of lane i's CSR row in row
+// order, for the warp's 32 consecutive rows (those from `end_row` on are empty; every lane
+// calls).  Skipped terms are +0.0 in the reference's dense ring, so the sums are
+// bit-identical.  The rows lie one behind the other, so the warp reads their entries as
+// one coalesced run, kGatherRun of them in flight per lane since latency bounds the walk;
+// the values of the few that spiked go to their rows' lanes one by one, in order.
+constexpr int kGatherRun = 8;
+template <typename R>
+__device__ __forceinline__ void gather_spikes(const DelayWindow& w, const Delayed& d, const StepPtrs<R>& p, u64 n_src, u64 words,
+                                              const u32* __restrict__ rs, const u32* __restrict__ src, u32 row,
+                                              u32 end_row, u32 steps, R* sums) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31;
+    for (int s = w.s_begin; s < w.s_end; ++s) sums[32 * s + lane] = static_cast<R>(0.0);
+    const u32 *bits = p.spk_bits + d.row * words, *bits_before = p.spk_bits + d.row_before * words;
+    const u32 lo = rs[min(row, end_row)];
+    const u32 end = __shfl_sync(kAll, rs[min(row + 1, end_row)], 31);
+    for (u64 k0 = __shfl_sync(kAll, lo, 0); k0 < end; k0 += 32 * kGatherRun) {
+        u32 id[kGatherRun], hit[kGatherRun];
+#pragma unroll
+        for (int i = 0; i < kGatherRun; ++i) {
+            const u64 k = k0 + 32 * i + lane;
+            id[i] = k < end ? src[k] : ~0u;
+        }
+        u32 any = 0;
+#pragma unroll
+        for (int i = 0; i < kGatherRun; ++i) {
+            hit[i] = 0;
+            if (id[i] != ~0u) {
+                hit[i] = bits[id[i] >> 5];
+                if (d.shift) hit[i] |= bits_before[id[i] >> 5];
+                hit[i] &= 1u << (id[i] & 31);
+            }
+            any |= hit[i];
+        }
+        if (!__any_sync(kAll, any != 0)) continue;
+#pragma unroll
+        for (int i = 0; i < kGatherRun; ++i)
+            if (hit[i]) hit[i] = delayed_steps(p.spk_word, n_src, d, w.W, id[i]) & steps;
+#pragma unroll
+        for (int i = 0; i < kGatherRun; ++i) {
+            auto value = [&](u32 m, u32 source) {  // of the first step in m
+                return p.val[delayed_slot(w, d, __ffs(static_cast<int>(m)) - 1) * n_src + source];
+            };
+            const R v = hit[i] ? value(hit[i], id[i]) : static_cast<R>(0.0);
+            for (unsigned left = __ballot_sync(kAll, hit[i] != 0); left; left &= left - 1) {
+                const int from = __ffs(static_cast<int>(left)) - 1;
+                const R first = __shfl_sync(kAll, v, from);
+                u32 m = __shfl_sync(kAll, hit[i], from);
+                const u32 source = __shfl_sync(kAll, id[i], from);
+                // the entry's row: the last one that starts at it or before
+                const unsigned owner = __popc(__ballot_sync(kAll, lo <= k0 + 32 * i + from)) - 1;
+                if (lane != owner) continue;
+                sums[32 * (__ffs(static_cast<int>(m)) - 1) + lane] += first;
+                while (m &= m - 1) sums[32 * (__ffs(static_cast<int>(m)) - 1) + lane] += value(m, source);
+            }
+        }
+    }
+}
+
+// Sums the delayed SIC factors of neuron j's a2n row for the steps in `steps`, in row
+// order (a factor of 0 adds nothing and is not read).  A thread walks its own row, four
+// steps and four entries at a time, so that sixteen loads are in flight where every
+// astrocyte is active; one value after the other took FIGURE.
+template <typename R>
+__device__ __forceinline__ void gather_sic(const DelayWindow& w, const StepPtrs<R>& p, u64 n_astro, u32 j, u32 steps,
+                                           R* sums) {
+    constexpr int kSteps = 4;
+    const unsigned lane = threadIdx.x & 31;
+    const u32 k0 = p.sic_rs[j], k1 = p.sic_rs[j + 1];
+    u32 any = 0;
+#pragma unroll 8
+    for (u32 k = k0; k < k1; ++k) any |= delayed_steps(p.act_word, n_astro, w.a2n, w.W, p.sic_src[k]);
+    steps &= any;
+    for (int s0 = w.s_begin; s0 < w.s_end; s0 += kSteps) {
+        const u32 now = (steps >> s0) & ((1u << kSteps) - 1u);
+        R sum[kSteps] = {};
+        if (now)
+#pragma unroll 4
+            for (u32 k = k0; k < k1; ++k) {
+                const u32 a = p.sic_src[k];
+                const u32 m = (delayed_steps(p.act_word, n_astro, w.a2n, w.W, a) >> s0) & now;
+                const R* factors = p.sic_ring + static_cast<u64>(a) * w.slots;
+#pragma unroll
+                for (int i = 0; i < kSteps; ++i)
+                    if ((m >> i) & 1u) sum[i] += factors[delayed_slot(w, w.a2n, s0 + i)];
+            }
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i)
+            if (s0 + i < w.s_end) sums[32 * (s0 + i) + lane] = sum[i];
+    }
+}
+
+// One astrocyte through the launch's steps (src/astrosim_fused.cu:374-427); called by whole warps.
+template <typename R>
+__device__ __forceinline__ void astro_delay_window(const RunConsts& rc, const NetScalars& ns, const StepPtrs<R>& p,
+                                                   const DelayWindow& w, u32 a, u32 end, u32 steps, R* sums) {
+    const unsigned lane = threadIdx.x & 31;
+    // the e2a delay is d_e (src/astrosim_fused.cu:384)
+    gather_spikes<R>(w, w.e, p, ns.n_neurons, ns.words, p.e2a_rs, p.e2a_src, a, end, steps, sums);
+    __syncwarp();
+    if (a >= end) return;
+    AstroRegs<R> s = load_astro<R>(p.Ca[a], p.IP3[a], p.h[a], p.Ca_tot[a], p.IP3_0[a], p.tau_IP3[a], p.delta_IP3[a]);
+    const unsigned char ever_in = p.ever_active[a];
+    unsigned char ever = ever_in;
+    u64 pbase = step_base(ns.seed, kAstroPoissonKey, w.start + w.s_begin, a);
+    u64 nbase = step_base(ns.seed, kAstroNoiseKey, w.start + w.s_begin, a);
+    i64 rphase = p.ca_rec ? (w.start + w.s_begin + 1) % p.rec_every : 1;
+    u32 active = 0;
+    R factor = static_cast<R>(0.0);
+    for (int st = w.s_begin; st < w.s_end; ++st) {
+        const i64 t = w.start + st;
+        factor = astro_advance_step<R>(rc, ns, s, sums[32 * st + lane], a, t, pbase, nbase);
+        pbase += kStepAdvance;
+        nbase += kStepAdvance;
+        if (p.ca_rec) {
+            record_ca<R>(p, a, t, rphase == 0, s.Ca);
+            if (++rphase == p.rec_every) rphase = 0;
+        }
+        if (factor > static_cast<R>(0.0)) ever = 1;
+        if (t == w.mark) ever = 0;
+        if (factor != static_cast<R>(0.0)) {
+            const u32 slot = w.slot + static_cast<u32>(st);
+            p.sic_ring[static_cast<u64>(a) * w.slots + (slot >= w.slots ? slot - w.slots : slot)] = factor;
+            active |= 1u << st;
+        }
+    }
+    p.Ca[a] = s.Ca;
+    p.IP3[a] = s.IP3;
+    p.h[a] = s.h;
+    if (ever != ever_in) p.ever_active[a] = ever;
+    p.sic_last[a] = factor;
+    u32* word = p.act_word + static_cast<u64>(w.row) * ns.n_astro + a;
+    *word = w.s_begin == 0 ? active : (*word | active);
+}
+
+// One neuron through the launch's steps (src/astrosim_fused.cu:433-587); called by whole warps.
+template <typename R, bool EXC>
+__device__ __forceinline__ void neuron_delay_window(const RunConsts& rc, const NetScalars& ns, const NeuronK& pk,
+                                                    const StepPtrs<R>& p, const DelayWindow& w, u32 j, u32 end,
+                                                    u32 steps, R* sums) {
+    const unsigned lane = threadIdx.x & 31;
+    const u64 nN = ns.n_neurons;
+    R *ex = sums, *in = sums + 32 * w.W, *sic = in + 32 * w.W;
+    const double lambda = EXC ? ns.lambda_exc : ns.lambda_inh;
+    const u64 lim53 = EXC ? ns.lim53_exc : ns.lim53_inh;
+    u64 counts;
+    poisson_window<1>(ns.seed, w.start, w.W, j, false, lambda, lim53, reinterpret_cast<u32*>(sums), lane, 32, &counts);
+    counts >>= 4 * w.s_begin;  // four bits per step, this step's lowest
+    __syncwarp();
+    gather_spikes<R>(w, w.e, p, nN, ns.words, p.exc_rs, p.exc_src, j, end, steps, ex);
+    // inh sources are local inhibitory indices that index the ring by global id (458-463)
+    gather_spikes<R>(w, w.i, p, nN, ns.words, p.inh_rs, p.inh_src, j, end, steps, in);
+    __syncwarp();
+    if (j >= end) return;
+    WindowSchedule sched = window_schedule(rc, w.start, w.s_begin, w.s_end);
+    gather_sic<R>(w, p, ns.n_astro, j, sched.refresh, sic);
+    NeuronCore<R> n(p, j);
+    R I_sic = p.I_sic[j];
+    const double nstd = EXC ? rc.noise_exc : rc.noise_inh;
+    const bool has_noise = nstd > 0.0 && rc.independent_noise;
+    R noise = static_cast<R>(0.0);
+    if (has_noise) noise = static_cast<R>(neuron_noise<R>(ns, nstd, sched.noise_idx, j));
+    const R w_a2n = as_r<R>(ns.w_a2n, ns.f_w_a2n), neg_w_i = as_r<R>(-rc.w_i, rc.f_neg_w_i);
+    u32 spikes = 0;
+    for (int st = w.s_begin; st < w.s_end; ++st) {
+        int events = static_cast<int>(static_cast<u32>(counts) & kExactCount);
+        counts >>= 4;
+        if (events == static_cast<int>(kExactCount))
+            events = poisson_exact(step_base(ns.seed, kNeuronPoissonKey, w.start + st, j), lambda,
+                                   EXC ? ns.limit_exc : ns.limit_inh, lim53);
+        if ((sched.refresh >> st) & 1u) I_sic = w_a2n * sic[32 * st + lane];
+        if (has_noise && ((sched.noise >> st) & 1u))
+            noise = static_cast<R>(neuron_noise<R>(ns, nstd, ++sched.noise_idx, j));
+        n.external(pk, has_noise ? I_sic + noise : I_sic);
+        if (!n.step(rc, pk, exc_input_of<R>(rc, EXC, ex[32 * st + lane], events), neg_w_i * in[32 * st + lane])) continue;
+        const i64 t = w.start + st;
+        const u32 slot = w.slot + static_cast<u32>(st);
+        p.val[static_cast<u64>(slot >= w.slots ? slot - w.slots : slot) * nN + j] =
+            stp_on_spike<R>(rc, p.stp_x[j], p.stp_u[j], p.stp_t[j], t);
+        atomicAdd(&p.counts[t], 1u);
+        if (t < p.raster_steps) atomicOr(&p.raster[static_cast<u64>(t) * ns.words + (j >> 5)], 1u << (j & 31));
+        spikes |= 1u << st;
+    }
+    n.store(p, j);
+    p.I_sic[j] = I_sic;
+    p.refr[j] = n.refr();
+    u32* word = p.spk_word + static_cast<u64>(w.row) * nN + j;
+    *word = w.s_begin == 0 ? spikes : (*word | spikes);
+    if (spikes) atomicOr(&p.spk_bits[static_cast<u64>(w.row) * ns.words + (j >> 5)], 1u << (j & 31));
+}
+
+template <typename R>
+__global__ void __launch_bounds__(sizeof(R) == 4 ? 1024 : 736) delay_kernel(RunConsts rc, StepPtrs<R> p, DelayWindow w, CellTiles tiles) {
+    extern __shared__ __align__(16) unsigned char shared[];
+    const NetScalars ns = net_scalars(rc);
+    const Tile tile = tile_of(tiles, blockIdx.x);
+    const u32 cell = tile.base + threadIdx.x, end = tile.end;
+    R* sums = reinterpret_cast<R*>(shared + (threadIdx.x >> 5) * delay_warp_bytes<R>(w.W));
+    if (w.s_begin == 0) {  // the next window's bits start clear; no one reads or sets them yet
+        const u64 i = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
+        if (i < ns.words) p.spk_bits[static_cast<u64>(w.row_next) * ns.words + i] = 0;
+    }
+    const u32 steps = (1u << w.s_end) - (1u << w.s_begin);
+    if (tile.kind == kAstroCells) astro_delay_window<R>(rc, ns, p, w, cell, end, steps, sums);
+    else if (tile.kind == kExcCells) neuron_delay_window<R, true>(rc, ns, rc.pe, p, w, cell, end, steps, sums);
+    else neuron_delay_window<R, false>(rc, ns, rc.pi, p, w, cell, end, steps, sums);
+}
+
+}  // namespace astrosim

@@ -55,22 +55,22 @@ __device__ __forceinline__ u64 pack_counts(const u32* words) {
     return static_cast<u64>(half[1]) << 32 | half[0];
 }
 
-// Draws the counts of cells j and (when have1) j + blockDim.x over the window of W steps
-// that starts at step win_start, into counts[cell].
+// Draws the counts of cells j and (when have1) j + threads over the window of W steps that
+// starts at step win_start, into counts[0] and counts[threads].  `shared`: poisson_bytes
+// for `threads` threads, of which the caller is number `thread`.
 template <int CELLS>
 __device__ __forceinline__ void poisson_window(u64 seed, i64 win_start, int W, u32 j, bool have1, double lambda,
-                                               u64 lim53, u32* shared, u64* counts) {
-    const u32 threads = blockDim.x;
+                                               u64 lim53, u32* shared, u32 thread, u32 threads, u64* counts) {
     const u32 gap = have1 ? threads : 0;
     if (!(lambda > 0.0) || !(lambda <= kPoissonWindowLambda)) {
         const u64 all = lambda > 0.0 ? ~u64(0) : u64(0);
-        counts[j] = all;
-        if (have1) counts[j + gap] = all;
+        counts[0] = all;
+        if (have1) counts[gap] = all;
         return;
     }
-    u32* const list = shared + threadIdx.x;
+    u32* const list = shared + thread;
     u8* const bytes = reinterpret_cast<u8*>(shared + static_cast<u32>(W) * CELLS * threads) +
-                      threadIdx.x * count_bytes(CELLS);
+                      thread * count_bytes(CELLS);
     u32* const words = reinterpret_cast<u32*>(bytes);
 #pragma unroll
     for (int i = 0; i < CELLS * kRowSteps / 4; ++i) words[i] = 0;
@@ -123,8 +123,8 @@ __device__ __forceinline__ void poisson_window(u64 seed, i64 win_start, int W, u
         }
     }
     for (; undecided; undecided &= undecided - 1) bytes[__ffs(undecided) - 1] = static_cast<u8>(kExactCount);
-    counts[j] = pack_counts(words);
-    if (CELLS == 2 && have1) counts[j + gap] = pack_counts(words + kRowSteps / 4);
+    counts[0] = pack_counts(words);
+    if (CELLS == 2 && have1) counts[gap] = pack_counts(words + kRowSteps / 4);
 }
 
 // The steps of a window's counts that are left to the exact draw.

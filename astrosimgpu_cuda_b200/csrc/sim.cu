@@ -10,8 +10,8 @@
 #include <vector>
 
 #include "biology.cuh"
+#include "delay_kernels.cuh"
 #include "sim.cuh"
-#include "step_kernels.cuh"
 #include "window.cuh"
 #include "builder_internal.cuh"
 #include "reduce.cuh"
@@ -19,38 +19,6 @@
 namespace astrosim {
 
 namespace {
-
-
-// One launch = one time step for every cell: the first `astro_blocks` blocks update
-// astrocytes, the rest update neurons.  The two populations of one step read only
-// rings written at least one step earlier (every delay is >= 1 step), so they may
-// run concurrently; this replaces the reference's two launches per step
-// (src/astrosim_fused.cu:1054-1064).
-template <typename R>
-__global__ void fused_step_kernel(RunConsts rc, StepPtrs<R> p, i64 step, u32 astro_blocks,
-                                                         int sic_refresh, u64 noise_idx) {
-    const NetScalars ns = net_scalars(rc);
-    if (blockIdx.x < astro_blocks) {
-        const u32 a = blockIdx.x * blockDim.x + threadIdx.x;
-        if (a < rc.n_astro) astro_cell_step<R>(rc, ns, p, a, step);
-        return;
-    }
-    const u32 j = (blockIdx.x - astro_blocks) * blockDim.x + threadIdx.x;
-    R out = static_cast<R>(0.0);
-    bool spiked = false;
-    if (j < rc.n_neurons) spiked = neuron_cell_step<R>(rc, ns, p, j, step, sic_refresh != 0, noise_idx, out);
-    // pack this warp's 32 spike bits into one word of the ring (warps cover aligned 32-neuron groups)
-    const unsigned ballot = __ballot_sync(0xffffffffu, spiked);
-    const int S = rc.slots;
-    const u64 slot = static_cast<u64>(step % S);
-    if ((threadIdx.x & 31) == 0 && j < rc.n_neurons) {
-        const u32 word = j >> 5;
-        p.bits[slot * rc.words + word] = ballot;
-        if (ballot) atomicAdd(&p.counts[step], static_cast<u32>(__popc(ballot)));
-        if (step < p.raster_steps) p.raster[static_cast<u64>(step) * rc.words + word] = ballot;
-    }
-    if (spiked) p.val[slot * rc.n_neurons + j] = out;
-}
 
 // exp(-lambda) of the Poisson drives and the constant synaptic decays are evaluated
 // on the device, where the reference evaluates them (src/astrosim_fused.cu:167, 515-516).
@@ -188,7 +156,7 @@ Status Simulation::create(const astrosim_config& cfg, const char* biology_json, 
     rc.d_e = delay_to_steps(bio_.d_e, cfg.dt);
     rc.d_i = delay_to_steps(bio_.d_i, cfg.dt);
     rc.d_a2n = delay_to_steps(bio_.d_a2n, cfg.dt);
-    rc.slots = std::max({rc.d_e, rc.d_i, rc.d_a2n}) + 1;
+    rc.slots = std::max({rc.d_e, rc.d_i, rc.d_a2n}) + 1;  // grown by delay_setup
     rc.steps_per_noise = std::max(1, static_cast<int>(std::llround(bio_.noise_dt / cfg.dt)));
     rc.sic_interval = bio_.sic_interval;
     rc.w_e = bio_.w_e;
@@ -262,10 +230,8 @@ Status Simulation::create(const astrosim_config& cfg, const char* biology_json, 
                 rc.n_neurons < (1u << 27) &&  // spike-list entries pack the neuron id in 27 bits
                 !(stepper && std::strcmp(stepper, "plain") == 0);
     if (!windowed_) {
-        net_.drop_forward();  // the per-step path reads only the target CSRs
-        AS_TRY(st_.spike_bits.alloc_zero(static_cast<u64>(rc.slots) * rc.words, stream_));
-        AS_TRY(st_.spike_val_raw.alloc_zero(static_cast<u64>(rc.slots) * nN * rbytes, stream_));
-        AS_TRY(st_.sic_ring_raw.alloc_zero(static_cast<u64>(rc.slots) * nA * rbytes, stream_));
+        net_.drop_forward();  // the delay windows read only the target CSRs
+        AS_TRY(delay_setup());
     } else {
         win_ = new WindowState();
         PhaseClock pc(stream_);
@@ -311,25 +277,68 @@ Status Simulation::launch_steps(i64 first, i64 count) {
         const i64 mark = pre_steps_ == 0 ? 0 : pre_steps_ - 1;
         return window_launch(rc_, st_, net_, fp32_, *win_, cfg_.raster_steps, mark, first, count, stream_, cfg_.block);
     }
-    const u32 astro_blocks = ceil_div(rc_.n_astro, block_);
-    const u32 neuron_blocks = ceil_div(rc_.n_neurons, block_);
-    for (i64 s = first; s < first + count; ++s) {
-        // per-step scalars of the reference loop (src/astrosim_fused.cu:1043-1046)
-        const u64 noise_idx = static_cast<u64>(s / rc_.steps_per_noise);
-        const bool refresh = (s - rc_.d_a2n >= 0) && ((s - rc_.d_a2n) % rc_.sic_interval == 0);
-        if (fp32_) {
-            auto p = make_ptrs<float>(st_, net_, rc_, cfg_.raster_steps);
-            fused_step_kernel<float><<<astro_blocks + neuron_blocks, block_, 0, stream_>>>(
-                rc_, p, s, astro_blocks, refresh ? 1 : 0, noise_idx);
-        } else {
-            auto p = make_ptrs<double>(st_, net_, rc_, cfg_.raster_steps);
-            fused_step_kernel<double><<<astro_blocks + neuron_blocks, block_, 0, stream_>>>(
-                rc_, p, s, astro_blocks, refresh ? 1 : 0, noise_idx);
-        }
+    return delay_launch(first, count);
+}
+
+// Windows of as many steps as the shortest delay allows (at most kMaxWindow, or fewer
+// where a large block's sums would not fit in shared memory).
+Status Simulation::delay_setup() {
+    RunConsts& rc = rc_;
+    constexpr size_t kPlainShared = 48 << 10, kMostShared = 200 << 10;
+    const auto bytes = [&](int W) {
+        return fp32_ ? delay_shared_bytes<float>(W, block_) : delay_shared_bytes<double>(W, block_);
+    };
+    const int longest = std::max({rc.d_e, rc.d_i, rc.d_a2n});
+    int W = std::min({rc.d_e, rc.d_i, rc.d_a2n, kMaxWindow});
+    while (W > 1 && bytes(W) > kMostShared) --W;
+    if (bytes(W) > kPlainShared) {
+        const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if (fp32_) AS_CUDA(cudaFuncSetAttribute(delay_kernel<float>, attr, static_cast<int>(kMostShared)));
+        else AS_CUDA(cudaFuncSetAttribute(delay_kernel<double>, attr, static_cast<int>(kMostShared)));
+    }
+    delay_W_ = W;
+    delay_windows_ = longest / W + 3;  // as far back as a delay reaches, this window and the next
+    rc.slots = longest + W;  // a window's own steps and those its first step may still read
+    const u64 nN = rc.n_neurons, nA = rc.n_astro, real = fp32_ ? sizeof(float) : sizeof(double);
+    AS_TRY(st_.spike_word.alloc_zero(delay_windows_ * nN, stream_));
+    AS_TRY(st_.spike_bits.alloc_zero(static_cast<u64>(delay_windows_) * rc.words, stream_));
+    AS_TRY(st_.active_word.alloc_zero(delay_windows_ * nA, stream_));
+    AS_TRY(st_.spike_val_raw.alloc_zero(static_cast<u64>(rc.slots) * nN * real, stream_));
+    AS_TRY(st_.sic_ring_raw.alloc_zero(static_cast<u64>(rc.slots) * nA * real, stream_));
+    return Status::Ok();
+}
+
+Status Simulation::delay_launch(i64 first, i64 count) {
+    const int W = delay_W_;
+    const CellTiles tiles = cell_tiles(rc_.n_exc, 0, rc_.n_neurons, 0, rc_.n_astro, static_cast<u32>(block_));
+    const auto wrap = [](i64 x, i64 n) { return static_cast<u32>((x % n + n) % n); };
+    for (i64 t = first; t < first + count;) {
+        const i64 k = t / W;
+        DelayWindow w{};
+        w.start = k * W;
+        w.mark = pre_steps_ == 0 ? 0 : pre_steps_ - 1;  // forget the transient's crossings (src/astrosim_fused.cu:1066-1076)
+        w.W = W;
+        w.s_begin = static_cast<int>(t - w.start);
+        w.s_end = static_cast<int>(std::min<i64>(W, first + count - w.start));
+        w.row = wrap(k, delay_windows_);
+        w.row_next = wrap(k + 1, delay_windows_);
+        w.slot = wrap(w.start, rc_.slots);
+        w.slots = static_cast<u32>(rc_.slots);
+        const auto delayed = [&](int d) {
+            return Delayed{wrap(k - d / W, delay_windows_), wrap(k - d / W - 1, delay_windows_),
+                           static_cast<u32>(d % W), wrap(w.start - d, rc_.slots)};
+        };
+        w.e = delayed(rc_.d_e);
+        w.i = delayed(rc_.d_i);
+        w.a2n = delayed(rc_.d_a2n);
+        if (fp32_)
+            delay_kernel<float><<<total_tiles(tiles), block_, delay_shared_bytes<float>(W, block_), stream_>>>(
+                rc_, make_ptrs<float>(st_, net_, rc_, cfg_.raster_steps), w, tiles);
+        else
+            delay_kernel<double><<<total_tiles(tiles), block_, delay_shared_bytes<double>(W, block_), stream_>>>(
+                rc_, make_ptrs<double>(st_, net_, rc_, cfg_.raster_steps), w, tiles);
         AS_CUDA(cudaGetLastError());
-        // end of the pre-run: forget threshold crossings of the transient (src/astrosim_fused.cu:1066-1076)
-        if (s == pre_steps_ - 1 || (pre_steps_ == 0 && s == 0))
-            AS_CUDA(cudaMemsetAsync(st_.ever_active.get(), 0, rc_.n_astro, stream_));
+        t = w.start + w.s_end;
     }
     return Status::Ok();
 }

@@ -96,9 +96,13 @@ struct StateBuffers {
     DevBuf<double> stp_t;
     DevBuf<int> refr;
     DevBuf<unsigned char> ever_active;
-    DevBuf<u32> spike_bits;        // [slots][words]
+    // The delay windows' rings: a word per cell and window (bit s: a spike, or a SIC factor
+    // other than 0, at its step s), a bit per neuron and window (any spike), and by step what
+    // those entries carry.
+    DevBuf<u32> spike_word, active_word;  // [windows][n_neurons], [windows][n_astro]
+    DevBuf<u32> spike_bits;               // [windows][words]
     DevBuf<unsigned char> spike_val_raw;  // [slots][n_neurons] real, written only by spiking neurons
-    DevBuf<unsigned char> sic_ring_raw;   // [slots][n_astro] real
+    DevBuf<unsigned char> sic_ring_raw;   // [n_astro][slots] real, written only where it is not 0
     DevBuf<unsigned char> sic_last_raw;   // [n_astro] real
     DevBuf<u32> counts;            // spikes per step
     DevBuf<u32> raster;            // [raster_steps][words]
@@ -165,6 +169,8 @@ public:
 private:
     Status launch_steps(i64 first, i64 count);
     Status ensure_counts(i64 steps);
+    Status delay_setup();
+    Status delay_launch(i64 first, i64 count);
 
     astrosim_config cfg_{};
     Biology bio_;
@@ -182,6 +188,7 @@ private:
     i64 counts_cap_ = 0;
     double run_seconds_ = 0.0;
     bool windowed_ = false;
+    int delay_W_ = 0, delay_windows_ = 0;  // steps of a delay window, windows in the rings of words
     WindowState* win_ = nullptr;  // owned; set when the windowed engine runs this network
 };
 

@@ -18,9 +18,8 @@ struct StepPtrs {
     double* stp_t;
     int* refr;
     unsigned char* ever_active;
-    u32* bits;     // [slots][words] spike bits
-    R* val;        // [slots][n_neurons] STP multiplier of each spike
-    R* sic_ring;   // [slots][n_astro]
+    u32 *spk_word, *spk_bits, *act_word;  // rings of the delay windows (delay_kernels.cuh); see StateBuffers
+    R *val, *sic_ring;
     R* sic_last;   // [n_astro]
     u32* counts;   // spikes per step
     u32* raster;   // [raster_steps][words]
@@ -40,21 +39,6 @@ __device__ __forceinline__ void record_ca(const StepPtrs<R>& p, u32 a, i64 t, bo
     if (!due || i >= p.rec_n) return;
     const i64 k = (t + 1) / p.rec_every - p.rec_k0;
     if (k >= 0 && k < p.rec_cap) p.ca_rec[static_cast<u64>(k) * p.rec_n + i] = ca;
-}
-
-// Sum of the delayed spike values of one CSR row, in row order, reading the packed
-// bit ring first and the value ring only for sources that spiked.  Skipped terms are
-// +0.0 in the reference's dense ring, so the sum is bit-identical.
-template <typename R>
-__device__ __forceinline__ R gather_spikes(const u32* __restrict__ rs, const u32* __restrict__ src, u32 row,
-                                           const u32* __restrict__ bits_slot, const R* __restrict__ val_slot) {
-    R sum = static_cast<R>(0.0);
-    const u32 k1 = rs[row + 1];
-    for (u32 k = rs[row]; k < k1; ++k) {
-        const u32 s = src[k];
-        if ((bits_slot[s >> 5] >> (s & 31)) & 1u) sum += val_slot[s];
-    }
-    return sum;
 }
 
 // Li-Rinzel RK4 with clamps (src/astrosim_fused.cu:255-278); noise held over the stages.
@@ -220,26 +204,6 @@ __device__ __forceinline__ R astro_advance_step(const RunConsts& rc, const NetSc
 constexpr u64 kStepAdvance = kCellStride * kStreamMul;
 __device__ __forceinline__ u64 step_base(u64 seed, u64 key, i64 step, u32 cell) {
     return rng_base(seed ^ key, static_cast<u64>(step) * kCellStride + cell);
-}
-
-// One astrocyte for step `step` on the per-step rings (src/astrosim_fused.cu:374-427).
-template <typename R>
-__device__ __forceinline__ void astro_cell_step(const RunConsts& rc, const NetScalars& ns, const StepPtrs<R>& p, u32 a,
-                                                i64 step) {
-    const int S = rc.slots;
-    const int read_slot = static_cast<int>((step + S - rc.d_e) % S);  // the e2a delay is d_e (384)
-    const R gathered = gather_spikes<R>(p.e2a_rs, p.e2a_src, a, p.bits + static_cast<u64>(read_slot) * ns.words,
-                                        p.val + static_cast<u64>(read_slot) * ns.n_neurons);
-    AstroRegs<R> s = load_astro<R>(p.Ca[a], p.IP3[a], p.h[a], p.Ca_tot[a], p.IP3_0[a], p.tau_IP3[a], p.delta_IP3[a]);
-    const R factor = astro_advance_step<R>(rc, ns, s, gathered, a, step, step_base(ns.seed, kAstroPoissonKey, step, a),
-                                           step_base(ns.seed, kAstroNoiseKey, step, a));
-    p.Ca[a] = s.Ca;
-    p.IP3[a] = s.IP3;
-    p.h[a] = s.h;
-    if (p.ca_rec) record_ca<R>(p, a, step, (step + 1) % p.rec_every == 0, s.Ca);
-    if (factor > static_cast<R>(0.0)) p.ever_active[a] = 1;
-    p.sic_ring[static_cast<u64>(step % S) * ns.n_astro + a] = factor;
-    p.sic_last[a] = factor;
 }
 
 // The AdEx right-hand side at one set of conductances (each RK4 step uses three:
@@ -452,58 +416,6 @@ __device__ __forceinline__ double neuron_noise(const NetScalars& ns, double nstd
     }
 }
 
-// One neuron for step `step` on the per-step rings (src/astrosim_fused.cu:433-587).
-// Returns whether it spiked and the value its ring entry carries.
-template <typename R>
-__device__ __forceinline__ bool neuron_cell_step(const RunConsts& rc, const NetScalars& ns, const StepPtrs<R>& p, u32 j,
-                                                 i64 step,
-                                                 bool sic_refresh, u64 noise_idx, R& out_value) {
-    const int S = rc.slots;
-    const bool excitatory = j < ns.n_exc;
-    const NeuronK& pk = excitatory ? rc.pe : rc.pi;
-    const int slot_ex = static_cast<int>((step + S - rc.d_e) % S);
-    const int slot_in = static_cast<int>((step + S - rc.d_i) % S);
-    const R exc_sum = gather_spikes<R>(p.exc_rs, p.exc_src, j, p.bits + static_cast<u64>(slot_ex) * ns.words,
-                                       p.val + static_cast<u64>(slot_ex) * ns.n_neurons);
-    // inh sources are local inhibitory indices that index the ring by global id (458-463)
-    const R inh_sum = gather_spikes<R>(p.inh_rs, p.inh_src, j, p.bits + static_cast<u64>(slot_in) * ns.words,
-                                       p.val + static_cast<u64>(slot_in) * ns.n_neurons);
-    R sic_sum = static_cast<R>(0.0);
-    if (sic_refresh) {
-        const int slot_sic = static_cast<int>((step + S - rc.d_a2n) % S);
-        const R* row = p.sic_ring + static_cast<u64>(slot_sic) * ns.n_astro;
-        const u32 k1 = p.sic_rs[j + 1];
-        for (u32 k = p.sic_rs[j]; k < k1; ++k) sic_sum += row[p.sic_src[k]];
-    }
-    const double nstd = excitatory ? rc.noise_exc : rc.noise_inh;
-    const bool has_noise = nstd > 0.0 && rc.independent_noise;
-    const double noise = has_noise ? neuron_noise<R>(ns, nstd, noise_idx, j) : 0.0;
-    NeuronRegs<R> n{p.V[j],     p.w[j],     p.V_reset + j, p.b + j, p.g_ex[j],
-                    p.dg_ex[j], p.g_in[j], p.dg_in[j],    p.I_sic[j], p.refr[j]};
-    const R ex_decay = as_r<R>(pk.ex_decay, pk.f_ex_decay), in_decay = as_r<R>(pk.in_decay, pk.f_in_decay);
-    const double lambda = excitatory ? ns.lambda_exc : ns.lambda_inh;
-    int events = 0;
-    if (lambda > 0.0)
-        events = rng_poisson_at(step_base(ns.seed, kNeuronPoissonKey, step, j), lambda,
-                                excitatory ? ns.limit_exc : ns.limit_inh, excitatory ? ns.lim53_exc : ns.lim53_inh);
-    if (sic_refresh) n.I_sic = as_r<R>(ns.w_a2n, ns.f_w_a2n) * sic_sum;
-    R I_ext = n.I_sic;
-    if (has_noise) I_ext += static_cast<R>(noise);
-    const bool spiked = neuron_ode_step<R>(rc, pk, n, exc_input_of<R>(rc, excitatory, exc_sum, events),
-                                           as_r<R>(-rc.w_i, rc.f_neg_w_i) * inh_sum, I_ext, ex_decay, in_decay);
-    p.V[j] = n.V;
-    p.w[j] = n.w;
-    p.g_ex[j] = n.g_ex;
-    p.dg_ex[j] = n.dg_ex;
-    p.g_in[j] = n.g_in;
-    p.dg_in[j] = n.dg_in;
-    p.refr[j] = n.refr;
-    if (sic_refresh) p.I_sic[j] = n.I_sic;
-    out_value = static_cast<R>(0.0);
-    if (spiked) out_value = stp_on_spike<R>(rc, p.stp_x[j], p.stp_u[j], p.stp_t[j], step);
-    return spiked;
-}
-
 // Device pointers of a simulation's state and network (host side).
 template <typename R>
 inline StepPtrs<R> make_ptrs(StateBuffers& s, Network& n, const RunConsts& rc, i64 raster_steps) {
@@ -525,7 +437,9 @@ inline StepPtrs<R> make_ptrs(StateBuffers& s, Network& n, const RunConsts& rc, i
     p.stp_t = s.stp_t.get();
     p.refr = s.refr.get();
     p.ever_active = s.ever_active.get();
-    p.bits = s.spike_bits.get();
+    p.spk_word = s.spike_word.get();
+    p.spk_bits = s.spike_bits.get();
+    p.act_word = s.active_word.get();
     p.val = reinterpret_cast<R*>(s.spike_val_raw.get());
     p.sic_ring = reinterpret_cast<R*>(s.sic_ring_raw.get());
     p.sic_last = reinterpret_cast<R*>(s.sic_last_raw.get());

@@ -759,8 +759,9 @@ __device__ __forceinline__ void draw_events(const NetScalars& ns, u64* events, i
     const u32 j = tile.base + threadIdx.x;
     if (j >= tile.end) return;
     const bool exc = tile.kind == kExcCells;
-    poisson_window<CELLS>(ns.seed, win_start, W, j, CELLS == 2 && tile.end - j > blockDim.x, exc ? ns.lambda_exc : ns.lambda_inh,
-                   exc ? ns.lim53_exc : ns.lim53_inh, shared, events);
+    poisson_window<CELLS>(ns.seed, win_start, W, j, CELLS == 2 && tile.end - j > blockDim.x,
+                          exc ? ns.lambda_exc : ns.lambda_inh,
+                          exc ? ns.lim53_exc : ns.lim53_inh, shared, threadIdx.x, blockDim.x, events + j);
 }
 // The tiles of the neurons [n_lo, n_hi) for it.
 inline CellTiles event_tiles(u32 n_exc, u32 n_lo, u32 n_hi, int block, int cells) {
