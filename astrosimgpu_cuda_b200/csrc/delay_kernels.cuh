@@ -2,15 +2,17 @@
 // (unequal ones, one step, or more than 16 steps).
 //
 // A cell's step reads only spikes and SIC factors that are at least min(d) steps old, so
-// one launch advances every cell by a window of up to min(d) steps (at most 16) without
-// any cell waiting for another; the state stays in registers.  A launch per step took
-// 20.5 us a step at N = 20011 (FP64), most of it in the rows' walk by one thread per
-// cell; windows of six steps take FIGURE.
+// one launch advances every cell by a window of up to min(d) steps (at most 16) without any
+// cell waiting for another; the state stays in registers.  What bounds it is latency: the
+// chain of a cell's steps (about 3 us each in FP64), and before it the walk of its rows.  A
+// launch per step, with a thread walking each row, took 20.5 us a step at N = 20011 and 92
+// at N = 2e5 (FP64); a launch per step with rows walked by warps 14.4 and 65; windows of six
+// steps take 5.3 and 23 (6.8 at N = 20011 with every astrocyte active).
 //
 // A window's spikes are one word per neuron (bit s: a spike at its step s), kept for
 // as many windows as the longest delay reaches back, so one load of a source tells its
 // spikes at all delayed steps of the window, and one bit per neuron (any spike in the
-// window) spares most of those loads.  The values that spikes carry and the SIC
+// window) spares most of those loads (N = 2e5: 41 us a step without it).  The values that spikes carry and the SIC
 // factors are in rings by step; the words say which entries mean something.
 #pragma once
 
@@ -122,7 +124,8 @@ __device__ __forceinline__ void gather_spikes(const DelayWindow& w, const Delaye
 // Sums the delayed SIC factors of neuron j's a2n row for the steps in `steps`, in row
 // order (a factor of 0 adds nothing and is not read).  A thread walks its own row, four
 // steps and four entries at a time, so that sixteen loads are in flight where every
-// astrocyte is active; one value after the other took FIGURE.
+// astrocyte is active (one value after the other: 10 us more per window at N = 20011).  A
+// first walk, over the words alone, is all there is while none is.
 template <typename R>
 __device__ __forceinline__ void gather_sic(const DelayWindow& w, const StepPtrs<R>& p, u64 n_astro, u32 j, u32 steps,
                                            R* sums) {
@@ -252,7 +255,8 @@ __device__ __forceinline__ void neuron_delay_window(const RunConsts& rc, const N
 }
 
 template <typename R>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 1024 : 736) delay_kernel(RunConsts rc, StepPtrs<R> p, DelayWindow w, CellTiles tiles) {
+__global__ void __launch_bounds__(sizeof(R) == 4 ? 1024 : 736)
+    delay_kernel(RunConsts rc, StepPtrs<R> p, DelayWindow w, CellTiles tiles) {
     extern __shared__ __align__(16) unsigned char shared[];
     const NetScalars ns = net_scalars(rc);
     const Tile tile = tile_of(tiles, blockIdx.x);
