@@ -224,7 +224,7 @@ Status Simulation::create(const astrosim_config& cfg, const char* biology_json, 
     AS_TRY(st_.ever_active.alloc(nA));
     // The windowed engine runs whenever every delay is the same D in [2, 16] steps,
     // which holds for the model's 1 ms delays at every dt from 0.0625 to 0.5 ms;
-    // ASTROSIM_STEPPER=plain keeps the per-step path (used to cross-check the two).
+    // ASTROSIM_STEPPER=plain runs the delay windows instead (used to cross-check the two).
     const char* stepper = std::getenv("ASTROSIM_STEPPER");
     windowed_ = rc.d_e == rc.d_i && rc.d_i == rc.d_a2n && rc.d_e >= 2 && rc.d_e <= kMaxWindow &&
                 rc.n_neurons < (1u << 27) &&  // spike-list entries pack the neuron id in 27 bits

@@ -383,7 +383,7 @@ __device__ __forceinline__ bool neuron_ode_step2(const RunConsts& rc, const Neur
 // written out, because the compiler's choice of which multiply-adds to fuse here
 // varied between launch-bounds instantiations of the window kernel (one fused
 // step * dt - t_last; measured on every spike of a run with facilitation): these are
-// the roundings the per-step kernel computes, so every engine and variant gives
+// the roundings one launch per step computed, so every engine and variant gives
 // the same bits.  x = 1 + (x - x u - 1) x_decay with x - x u and the last
 // multiply-add fused; u = U + (u (1 - U)) u_decay with the last one fused.
 template <typename R>

@@ -128,8 +128,8 @@ int astrosim_create(const astrosim_config* cfg, astrosim_handle** out);
  * NULL or "" keeps every default.  Unknown or repeated names, malformed text and
  * values the model cannot run with (a non-positive time constant, capacitance or
  * delay, sic_interval < 1, ...) return ASTROSIM_ERR_INVALID_ARG with the name in
- * astrosim_last_error().  Delays that are not all equal, or not 2-16 steps, run on
- * the per-step engine instead of the windowed one.
+ * astrosim_last_error().  Delays that are not all equal, or not 2-16 steps, run in
+ * windows of the shortest one instead of on the windowed engine.
  */
 int astrosim_create_with_biology(const astrosim_config* cfg, const char* biology_json, astrosim_handle** out);
 
