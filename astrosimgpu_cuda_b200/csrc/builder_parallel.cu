@@ -356,7 +356,8 @@ __device__ __forceinline__ u32 lower_bound_near(const u64* entries, u64 c) {
 // it.  (Walks rejoin after a median of 2 pres, some after hundreds.)  What bounds it is
 // latency: the load of the window and a lane's walk of about a hundred words.  512 threads
 // load, look through the hazards in shared memory and through the table starts around the
-// walk: 1.5 ms at N = 1e3, 3.0 ms at N = 3e5; 128 threads that read hazards and table
+// walk, and a landing waits once for its two words: 1.3 ms at N = 1e3, 2.6 ms at N = 3e5 (1.5
+// and 3.0 with a wait for each); 128 threads that read hazards and table
 // starts from global memory took 2.8 and 6.3 ms.
 constexpr u32 kReplayBlock = 512, kReplayBatch = 32, kReplayWindow = 8192;
 constexpr u32 kReplayWords = kReplayWindow + kWordsAhead;
@@ -467,20 +468,21 @@ __global__ void __launch_bounds__(kReplayBlock) replay_kernel(Sec s, const u16* 
                 const u32 self = static_cast<u32>(r + q) - s.post_off;
                 u32 x = static_cast<u32>(start - c), left = s.post_count;
                 bool hit_self = false;
-                u32 skip = words[x++];
+                u32 skip = words[x++], test = words[x];  // the test's word with the skip's: one wait per landing
                 for (;;) {
                     const u32 g = skip & kSkipMax;
                     if (g >= left) break;
-                    if (x + 3 > window + kWordsAhead) {
+                    if (x + 4 > window + kWordsAhead) {
                         atomicOr(s.err, kErrDelta);
                         break;
                     }
                     const bool own = s.post_count - left + g == self;
                     hit_self = hit_self || own;
                     left -= g + 1;
-                    if (s.third && !own) x += (words[x] & kHitBit) ? 2 : 1;
+                    if (s.third && !own) x += (test & kHitBit) ? 2 : 1;
                     if (left == 0) break;
                     skip = words[x++];
+                    test = words[x];
                 }
                 long long k = -1;
                 if (q || !on_orbit_start) {
