@@ -46,6 +46,15 @@ __host__ __device__ __forceinline__ u32 rng_mix_hi(u64 z) {
     return hi ^ (hi >> 31);
 }
 
+// A first Poisson draw whose upper 32 bits are below these gives no event (lim53: see
+// rng_poisson_at).  Where e^-lambda rounds to 1 (a rate below 1.2e-16 events per step),
+// lim53 is 2^53, whose upper part does not fit: there the largest draws alone are looked at
+// in full.
+__host__ __device__ __forceinline__ u32 poisson_limit_hi(u64 lim53) {
+    const u64 hi = lim53 >> 21;
+    return hi < 0xFFFFFFFFu ? static_cast<u32>(hi) : 0xFFFFFFFFu;
+}
+
 __host__ __device__ __forceinline__ u64 rng_bits(u64 seed, u64 stream, u64 counter) {
     u64 z = seed;
     z += stream * kStreamMul;

@@ -76,7 +76,7 @@ __device__ __forceinline__ void poisson_window(u64 seed, i64 win_start, int W, u
     for (int i = 0; i < CELLS * kRowSteps / 4; ++i) words[i] = 0;
     // u0 > limit exactly when its 53 bits exceed lim53; an equal upper part is listed and
     // then falls within the slack
-    const u32 lim_hi = static_cast<u32>(lim53 >> 21);
+    const u32 lim_hi = poisson_limit_hi(lim53);
     const u32 sure_more = lim_hi < 0xFFFFFFFFu - kPoissonSlack ? lim_hi + kPoissonSlack : 0xFFFFFFFFu;
     const u32 sure_done = lim_hi > kPoissonSlack ? lim_hi - kPoissonSlack : 0;
     const u64 base = rng_base(seed ^ kNeuronPoissonKey, static_cast<u64>(win_start) * kCellStride + j);

@@ -153,7 +153,7 @@ template <typename R>
 __device__ __forceinline__ R astro_kick(const RunConsts& rc, const NetScalars& ns, R gathered, u64 poisson_base) {
     R ip3_input = as_r<R>(rc.w_n2a, rc.f_w_n2a) * gathered;
     // an event needs a first draw whose upper part reaches the limit's (see rng_poisson_at)
-    if (ns.lambda_astro > 0.0 && rng_mix_hi(poisson_base) >= static_cast<u32>(ns.lim53_astro >> 21)) {
+    if (ns.lambda_astro > 0.0 && rng_mix_hi(poisson_base) >= poisson_limit_hi(ns.lim53_astro)) {
         const int ev = poisson_exact(poisson_base, ns.lambda_astro, ns.limit_astro, ns.lim53_astro);
         if (ev > 0) ip3_input += as_r<R>(rc.weight_astro, rc.f_weight_astro) * static_cast<R>(ev);
     }
