@@ -63,6 +63,14 @@ __global__ void init_state_kernel(StepPtrs<R> p, RunConsts rc, double V_e, doubl
     }
 }
 
+template <typename R>
+void launch_delay_window(const RunConsts& rc, const StepPtrs<R>& p, const DelayWindow& w, const CellTiles& tiles,
+                         int block, cudaStream_t st) {
+    const size_t smem = delay_shared_bytes<R>(shared_steps(w), block);
+    if (one_step(w)) delay_kernel<R, true><<<total_tiles(tiles), block, smem, st>>>(rc, p, w, tiles);
+    else delay_kernel<R, false><<<total_tiles(tiles), block, smem, st>>>(rc, p, w, tiles);
+}
+
 Biology biology_for(const astrosim_config& cfg, Biology b) {
     if (b.noise_dt <= 0.0) b.noise_dt = 10.0 * cfg.dt;  // src/astrosim_fused.cu:848
     if (!std::isnan(cfg.w_n2a)) b.w_n2a = cfg.w_n2a;
@@ -293,8 +301,8 @@ Status Simulation::delay_setup() {
     while (W > 1 && bytes(W) > kMostShared) --W;
     if (bytes(W) > kPlainShared) {
         const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        if (fp32_) AS_CUDA(cudaFuncSetAttribute(delay_kernel<float>, attr, static_cast<int>(kMostShared)));
-        else AS_CUDA(cudaFuncSetAttribute(delay_kernel<double>, attr, static_cast<int>(kMostShared)));
+        if (fp32_) AS_CUDA(cudaFuncSetAttribute(delay_kernel<float, false>, attr, static_cast<int>(kMostShared)));
+        else AS_CUDA(cudaFuncSetAttribute(delay_kernel<double, false>, attr, static_cast<int>(kMostShared)));
     }
     delay_W_ = W;
     delay_windows_ = longest / W + 3;  // as far back as a delay reaches, this window and the next
@@ -302,6 +310,9 @@ Status Simulation::delay_setup() {
     const u64 nN = rc.n_neurons, nA = rc.n_astro, real = fp32_ ? sizeof(float) : sizeof(double);
     AS_TRY(st_.spike_word.alloc_zero(delay_windows_ * nN, stream_));
     AS_TRY(st_.spike_bits.alloc_zero(static_cast<u64>(delay_windows_) * rc.words, stream_));
+    // a window clears the next one's rows of bits by step, which none of its own steps reads
+    delay_bit_slots_ = longest + 2 * W;
+    if (W > 1) AS_TRY(st_.step_bits.alloc_zero(static_cast<u64>(delay_bit_slots_) * rc.words, stream_));
     AS_TRY(st_.active_word.alloc_zero(delay_windows_ * nA, stream_));
     AS_TRY(st_.spike_val_raw.alloc_zero(static_cast<u64>(rc.slots) * nN * real, stream_));
     AS_TRY(st_.sic_ring_raw.alloc_zero(static_cast<u64>(rc.slots) * nA * real, stream_));
@@ -324,19 +335,17 @@ Status Simulation::delay_launch(i64 first, i64 count) {
         w.row_next = wrap(k + 1, delay_windows_);
         w.slot = wrap(w.start, rc_.slots);
         w.slots = static_cast<u32>(rc_.slots);
+        w.bit_slot = wrap(w.start, delay_bit_slots_);
+        w.bit_slots = static_cast<u32>(delay_bit_slots_);
         const auto delayed = [&](int d) {
             return Delayed{wrap(k - d / W, delay_windows_), wrap(k - d / W - 1, delay_windows_),
-                           static_cast<u32>(d % W), wrap(w.start - d, rc_.slots)};
+                           static_cast<u32>(d % W), wrap(w.start - d, rc_.slots), wrap(w.start - d, delay_bit_slots_)};
         };
         w.e = delayed(rc_.d_e);
         w.i = delayed(rc_.d_i);
         w.a2n = delayed(rc_.d_a2n);
-        if (fp32_)
-            delay_kernel<float><<<total_tiles(tiles), block_, delay_shared_bytes<float>(W, block_), stream_>>>(
-                rc_, make_ptrs<float>(st_, net_, rc_, cfg_.raster_steps), w, tiles);
-        else
-            delay_kernel<double><<<total_tiles(tiles), block_, delay_shared_bytes<double>(W, block_), stream_>>>(
-                rc_, make_ptrs<double>(st_, net_, rc_, cfg_.raster_steps), w, tiles);
+        if (fp32_) launch_delay_window<float>(rc_, make_ptrs<float>(st_, net_, rc_, cfg_.raster_steps), w, tiles, block_, stream_);
+        else launch_delay_window<double>(rc_, make_ptrs<double>(st_, net_, rc_, cfg_.raster_steps), w, tiles, block_, stream_);
         AS_CUDA(cudaGetLastError());
         t = w.start + w.s_end;
     }

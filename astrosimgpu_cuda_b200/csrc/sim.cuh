@@ -97,10 +97,10 @@ struct StateBuffers {
     DevBuf<int> refr;
     DevBuf<unsigned char> ever_active;
     // The delay windows' rings: a word per cell and window (bit s: a spike, or a SIC factor
-    // other than 0, at its step s), a bit per neuron and window (any spike), and by step what
-    // those entries carry.
+    // other than 0, at its step s), a bit per neuron and window (any spike), and by step a
+    // bit per neuron and what those entries carry.
     DevBuf<u32> spike_word, active_word;  // [windows][n_neurons], [windows][n_astro]
-    DevBuf<u32> spike_bits;               // [windows][words]
+    DevBuf<u32> spike_bits, step_bits;    // [windows][words], [bit slots][words]
     DevBuf<unsigned char> spike_val_raw;  // [slots][n_neurons] real, written only by spiking neurons
     DevBuf<unsigned char> sic_ring_raw;   // [n_astro][slots] real, written only where it is not 0
     DevBuf<unsigned char> sic_last_raw;   // [n_astro] real
@@ -189,6 +189,7 @@ private:
     double run_seconds_ = 0.0;
     bool windowed_ = false;
     int delay_W_ = 0, delay_windows_ = 0;  // steps of a delay window, windows in the rings of words
+    int delay_bit_slots_ = 0;              // steps in the ring of bits by step
     WindowState* win_ = nullptr;  // owned; set when the windowed engine runs this network
 };
 

@@ -18,7 +18,7 @@ struct StepPtrs {
     double* stp_t;
     int* refr;
     unsigned char* ever_active;
-    u32 *spk_word, *spk_bits, *act_word;  // rings of the delay windows (delay_kernels.cuh); see StateBuffers
+    u32 *spk_word, *spk_bits, *step_bits, *act_word;  // rings of the delay windows (delay_kernels.cuh); see StateBuffers
     R *val, *sic_ring;
     R* sic_last;   // [n_astro]
     u32* counts;   // spikes per step
@@ -439,6 +439,7 @@ inline StepPtrs<R> make_ptrs(StateBuffers& s, Network& n, const RunConsts& rc, i
     p.ever_active = s.ever_active.get();
     p.spk_word = s.spike_word.get();
     p.spk_bits = s.spike_bits.get();
+    p.step_bits = s.step_bits.get();
     p.act_word = s.active_word.get();
     p.val = reinterpret_cast<R*>(s.spike_val_raw.get());
     p.sic_ring = reinterpret_cast<R*>(s.sic_ring_raw.get());
