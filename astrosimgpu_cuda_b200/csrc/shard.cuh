@@ -89,7 +89,7 @@ public:
     Status run_window(i64 k);
     Status pack(i64 k);  // export lists and counts; counts reach host_counts() after a stream sync
     Status import(i64 k, const u32* counts_all, u64 stride_spk, u64 stride_ast);  // counts_all: 2 per rank
-    Status push(i64 k);
+    Status push(i64 k, bool more);  // more: window k + 1 follows in this call
     void note_window(double seconds);
 
     const u32* host_counts() const { return h_cnt_; }

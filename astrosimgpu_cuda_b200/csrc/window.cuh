@@ -61,7 +61,7 @@ struct WindowState {
     DevBuf<u32> sic_pos;                      // [2][n_neurons]: positions of active astrocytes in the a2n row
     DevBuf<int> mode;                         // [2]: 0 push, 1 pull
     DevBuf<u64> events;                       // background event counts of one window (poisson_window.cuh)
-    i64 events_window = -1;                   // the window whose counts `events` holds (single-network engine)
+    i64 events_window = -1;                   // the window whose counts `events` holds (not kept by a batch)
     // autotuner: (block size, launch bounds) variant of window_kernel, an index into
     // its table; -1 while timing the candidates, -2 for the generic kernel (a block
     // size outside the table, nothing to tune)
