@@ -41,7 +41,17 @@ constexpr int kTileSizes[kNumTileSizes] = {64, 128, 256};
 int tile_index(int tile) { return tile == 64 ? 0 : (tile == 256 ? 2 : 1); }
 constexpr int kEnsTuneRounds = 2;
 constexpr int kGraphWindows = 10;
-constexpr u32 kPushBlocksPerNet = 4;
+// Blocks that deliver a network's window: one per 256 astrocytes, so that each warp has one
+// word of 32 active ones to mark, and one per 256 neurons up to four (a few spikes' targets).
+// Four for every network whatever its size let 32 warps mark all of a large one's: with every
+// astrocyte active, us per step, one network of 1e6 cells FP32 456, 41 so; FP64 838, 63; 64
+// networks of 500 to 50000 cells FP32 50, 32.
+constexpr u32 kPushCells = 256;
+inline u32 push_blocks_of(u32 n_neurons, u32 n_astro) {
+    return std::min(std::max(ceil_div(n_astro, kPushCells), std::min(4u, ceil_div(n_neurons, kPushCells))),
+                    sm_count() * 8);
+}
+
 // A tile table entry: the population in the upper bits, the tile's index within it below.
 constexpr u32 kTileKindShift = 30;
 constexpr u32 kTileIndexMask = (1u << kTileKindShift) - 1;
@@ -95,24 +105,25 @@ __global__ void __launch_bounds__(TILE, MB) ens_window_kernel(RunConsts common, 
 constexpr int kEnsPushBlock = 256;
 constexpr int kEnsDrawCells = 2;
 
-// After every network's window: the first kPushBlocksPerNet * n_nets blocks deliver its
-// spikes, the others draw the background events of the window that follows (one tile of
-// the draw table each).  `ahead`: 1 after a window, 0 to draw for the current window
-// (no delivery).
+// After every network's window: the first `push_blocks` blocks deliver its spikes (the push
+// table names each one's network, its number within it and how many that network has), the
+// others draw the background events of the window that follows (one tile of the draw table
+// each).  `ahead`: 1 after a window, 0 to draw for the current window (no delivery).
 template <typename R>
 __global__ void __launch_bounds__(kEnsPushBlock) ens_push_kernel(const NetDesc<R>* __restrict__ descs,
                                                                  const i64* __restrict__ win,
                                                                  const i64* __restrict__ stop, int W, u32 push_blocks,
+                                                                 const EnsPushBlock* __restrict__ push,
                                                                  const u32* __restrict__ draw_net,
                                                                  const u32* __restrict__ draw_blk, int ahead) {
     extern __shared__ u32 rows[];
     if (blockIdx.x < push_blocks) {
-        const u32 net = blockIdx.x / kPushBlocksPerNet;
-        const i64 k = win[net];
-        if (k * W + W > stop[net]) return;  // the window did not complete: no window follows it
-        const NetDesc<R>& d = descs[net];
+        const EnsPushBlock b = push[blockIdx.x];
+        const i64 k = win[b.net];
+        if (k * W + W > stop[b.net]) return;  // the window did not complete: no window follows it
+        const NetDesc<R>& d = descs[b.net];
         push_cells<R>(d.w, d.ns.n_exc, d.ns.n_neurons - d.ns.n_exc, d.ns.n_neurons, d.ns.n_astro,
-                      static_cast<int>(k & 1), blockIdx.x % kPushBlocksPerNet, kPushBlocksPerNet);
+                      static_cast<int>(k & 1), b.block, b.blocks);
         return;
     }
     const u32 net = draw_net[blockIdx.x - push_blocks];
@@ -152,17 +163,17 @@ int variant_tile(bool fp32, int v) { return fp32 ? kEnsVariantsF32[v].tile : kEn
 
 // One window and its push for every network.
 template <typename R>
-void launch_ens_window(int v, bool uniform, u32 grid, u32 n, cudaStream_t st, const RunConsts& common,
+void launch_ens_window(int v, bool uniform, u32 grid, cudaStream_t st, const RunConsts& common,
                        const void* rcs, const void* descs, const u32* tn, const u32* tb, const i64* win,
-                       const i64* stop, int W, u32 draws, const u32* draw_net, const u32* draw_blk) {
+                       const i64* stop, int W, u32 push_blocks, const EnsPushBlock* push, u32 draws,
+                       const u32* draw_net, const u32* draw_blk) {
     const RunConsts* r = static_cast<const RunConsts*>(rcs);
     const NetDesc<R>* d = static_cast<const NetDesc<R>*>(descs);
     constexpr auto seq = std::make_integer_sequence<int, kEnsNumVariants>();
     static constexpr auto shared_table = ens_launches<R, true>(seq), own_table = ens_launches<R, false>(seq);
     (uniform ? shared_table : own_table)[v](grid, st, common, r, d, tn, tb, win, stop, W);
-    const u32 push_blocks = kPushBlocksPerNet * n;
     ens_push_kernel<R><<<push_blocks + draws, kEnsPushBlock, poisson_bytes(kEnsDrawCells, W, kEnsPushBlock), st>>>(
-        d, win, stop, W, push_blocks, draw_net, draw_blk, 1);
+        d, win, stop, W, push_blocks, push, draw_net, draw_blk, 1);
 }
 
 // `rc` with the NetScalars fields cleared.  RunConsts has no implicit padding, so
@@ -238,6 +249,7 @@ Ensemble::~Ensemble() {
         tile_net_[ti].release();
         tile_blk_[ti].release();
     }
+    push_.release();
     draw_net_.release();
     draw_blk_.release();
     win_.release();
@@ -369,9 +381,12 @@ Status Ensemble::rebuild() {
     }
     {
         std::vector<u32> dn, db;
+        std::vector<EnsPushBlock> push;
         for (u32 i = 0; i < nets_.size(); ++i) {
             if (!nets_[i]) continue;
             const RunConsts& rc = nets_[i]->consts();
+            const u32 blocks = push_blocks_of(rc.n_neurons, rc.n_astro);
+            for (u32 b = 0; b < blocks; ++b) push.push_back(EnsPushBlock{i, b, blocks, 0});
             const CellTiles t = event_tiles(rc.n_exc, 0, rc.n_neurons, kEnsPushBlock, kEnsDrawCells);
             for (const u32 kind : {u32(kExcCells), u32(kInhCells)})
                 for (u32 b = 0; b < t.tiles[kind]; ++b) {
@@ -379,6 +394,11 @@ Status Ensemble::rebuild() {
                     db.push_back(b | kind << kTileKindShift);
                 }
         }
+        n_push_ = static_cast<u32>(push.size());
+        AS_TRY(push_.alloc(std::max<size_t>(1, push.size())));
+        if (!push.empty())
+            AS_CUDA(cudaMemcpyAsync(push_.get(), push.data(), push.size() * sizeof(EnsPushBlock),
+                                    cudaMemcpyHostToDevice, stream_));
         n_draws_ = static_cast<u32>(dn.size());
         AS_TRY(draw_net_.alloc(std::max<size_t>(1, dn.size())));
         AS_TRY(draw_blk_.alloc(std::max<size_t>(1, db.size())));
@@ -400,16 +420,15 @@ Status Ensemble::rebuild() {
 }
 
 void Ensemble::launch_window(int v) {
-    const u32 n = static_cast<u32>(nets_.size());
     const int ti = tile_index(variant_tile(fp32_, v));
     if (fp32_)
-        launch_ens_window<float>(v, uniform_, n_tiles_[ti], n, stream_, common_, rcs_.get(), descs_.get(),
-                                 tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_, n_draws_,
-                                 draw_net_.get(), draw_blk_.get());
+        launch_ens_window<float>(v, uniform_, n_tiles_[ti], stream_, common_, rcs_.get(), descs_.get(),
+                                 tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_, n_push_,
+                                 push_.get(), n_draws_, draw_net_.get(), draw_blk_.get());
     else
-        launch_ens_window<double>(v, uniform_, n_tiles_[ti], n, stream_, common_, rcs_.get(), descs_.get(),
-                                  tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_, n_draws_,
-                                  draw_net_.get(), draw_blk_.get());
+        launch_ens_window<double>(v, uniform_, n_tiles_[ti], stream_, common_, rcs_.get(), descs_.get(),
+                                  tile_net_[ti].get(), tile_blk_[ti].get(), win_.get(), stop_.get(), W_, n_push_,
+                                  push_.get(), n_draws_, draw_net_.get(), draw_blk_.get());
 }
 
 // The background events of every network's current window: after a change of membership,
@@ -419,12 +438,12 @@ Status Ensemble::draw_current() {
     const size_t smem = poisson_bytes(kEnsDrawCells, W_, kEnsPushBlock);
     if (fp32_)
         ens_push_kernel<float><<<n_draws_, kEnsPushBlock, smem, stream_>>>(
-            reinterpret_cast<const NetDesc<float>*>(descs_.get()), win_.get(), stop_.get(), W_, 0, draw_net_.get(),
-            draw_blk_.get(), 0);
+            reinterpret_cast<const NetDesc<float>*>(descs_.get()), win_.get(), stop_.get(), W_, 0, nullptr,
+            draw_net_.get(), draw_blk_.get(), 0);
     else
         ens_push_kernel<double><<<n_draws_, kEnsPushBlock, smem, stream_>>>(
-            reinterpret_cast<const NetDesc<double>*>(descs_.get()), win_.get(), stop_.get(), W_, 0, draw_net_.get(),
-            draw_blk_.get(), 0);
+            reinterpret_cast<const NetDesc<double>*>(descs_.get()), win_.get(), stop_.get(), W_, 0, nullptr,
+            draw_net_.get(), draw_blk_.get(), 0);
     AS_CUDA(cudaGetLastError());
     return Status::Ok();
 }

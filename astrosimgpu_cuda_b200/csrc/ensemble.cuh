@@ -22,6 +22,11 @@ namespace astrosim {
 
 constexpr int kNumTileSizes = 3;  // tiles of 64, 128 or 256 cells, chosen by the autotuner
 
+// One block of the push: block `block` of the `blocks` that deliver network `net`.
+struct alignas(16) EnsPushBlock {
+    u32 net, block, blocks, pad_;
+};
+
 class Ensemble {
 public:
     ~Ensemble();
@@ -69,8 +74,9 @@ private:
     bool uniform_ = true;
     // tile tables by tile size
     DevBuf<u32> tile_net_[kNumTileSizes], tile_blk_[kNumTileSizes];
+    DevBuf<EnsPushBlock> push_;        // blocks of the push
     DevBuf<u32> draw_net_, draw_blk_;  // tiles of the background draws
-    u32 n_draws_ = 0;
+    u32 n_push_ = 0, n_draws_ = 0;
     DevBuf<i64> win_, stop_;
     u32 n_tiles_[kNumTileSizes] = {};
     bool dirty_ = true;
