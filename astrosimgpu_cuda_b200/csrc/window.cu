@@ -277,13 +277,8 @@ template <typename R, int B, int M>
 cudaError_t launch_one(cudaStream_t st, const RunConsts& rc, const StepPtrs<R>& p, const WinPtrs<R>& w, i64 start,
                        int s0, int s1, int buf, i64 mark, int block) {
     const CellTiles tiles = cell_tiles(rc.n_exc, 0, rc.n_neurons, 0, rc.n_astro, static_cast<u32>(block));
-    const size_t smem = sic_bytes<R>(w.W, block);
-    if (smem > 48 * 1024) {  // large blocks of the generic instantiation
-        const cudaError_t e = cudaFuncSetAttribute(window_kernel<R, B, M>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
-    window_kernel<R, B, M><<<total_tiles(tiles), block, smem, st>>>(rc, p, w, start, s0, s1, buf, mark, tiles);
+    window_kernel<R, B, M><<<total_tiles(tiles), block, sic_bytes<R>(w.W, block), st>>>(rc, p, w, start, s0, s1, buf,
+                                                                                       mark, tiles);
     return cudaGetLastError();
 }
 
@@ -298,6 +293,17 @@ constexpr LaunchFn<R> variant_launch() {
 template <typename R, int... V>
 constexpr std::array<LaunchFn<R>, sizeof...(V)> variant_launches(std::integer_sequence<int, V...>) {
     return {variant_launch<R, V>()...};
+}
+
+// Blocks of the table stay within the 48 KB of shared memory that every kernel may use.  The
+// generic kernel's limit is set to its largest block's longest window, the same for every
+// network, so that networks stepped by different threads don't lower each other's; and when
+// a network first steps, not at each launch (48 networks built by 12 threads with such a call
+// at each launch: 200 ms instead of 130).
+template <typename R>
+cudaError_t allow_generic_blocks() {
+    return cudaFuncSetAttribute(window_kernel<R, 1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(sic_bytes<R>(kMaxWindow, 1024)));
 }
 
 // Launches variant `variant` (an index into the table; -1 = the generic kernel at
@@ -321,7 +327,10 @@ Status launch_impl(const RunConsts& rc, StateBuffers& sb, Network& net, WindowSt
     const u32 push_warps = std::max<u32>(8, std::min<u32>(sm_count() * 64, ws.push_limit));
     int v_first = 0, v_count = 0;
     variant_range(block, &v_first, &v_count);
-    if (v_first < 0) ws.variant = -2;  // a block size outside the table: the generic kernel, nothing to tune
+    if (v_first < 0 && ws.variant != -2) {  // a block size outside the table: the generic kernel, nothing to tune
+        AS_CUDA(allow_generic_blocks<R>());
+        ws.variant = -2;
+    }
     int bucket = 0;
     while ((1ull << bucket) < rc.n_neurons) ++bucket;
     const std::tuple<int, int, int> key{f32 ? 1 : 0, bucket, block};
