@@ -311,8 +311,13 @@ __device__ __forceinline__ void neuron_delay_window(const RunConsts& rc, const N
     if (spikes) atomicOr(&p.spk_bits[static_cast<u64>(w.row) * ns.words + (j >> 5)], 1u << (j & 31));
 }
 
+// Threads of a block: FP64 needs more registers than 1024 threads leave it (88 with 736).  A
+// larger block size of the configuration runs as blocks of this one, to the same results.
+template <typename R>
+constexpr int kDelayThreads = sizeof(R) == 4 ? 1024 : 736;
+
 template <typename R, bool Short>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? 1024 : 736)
+__global__ void __launch_bounds__(kDelayThreads<R>)
     delay_kernel(RunConsts rc, StepPtrs<R> p, DelayWindow w, CellTiles tiles) {
     extern __shared__ __align__(16) unsigned char shared[];
     const NetScalars ns = net_scalars(rc);

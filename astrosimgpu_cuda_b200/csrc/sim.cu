@@ -127,7 +127,6 @@ Status Simulation::create(const astrosim_config& cfg, const char* biology_json, 
     if (cfg.raster_steps < 0) return make_error(ASTROSIM_ERR_INVALID_ARG, "raster_steps must be >= 0");
     cfg_ = cfg;
     fp32_ = cfg.precision == ASTROSIM_PRECISION_FP32;
-    block_ = cfg.block == 0 ? 128 : cfg.block;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         cudaGetLastError();
@@ -293,8 +292,9 @@ Status Simulation::launch_steps(i64 first, i64 count) {
 Status Simulation::delay_setup() {
     RunConsts& rc = rc_;
     constexpr size_t kPlainShared = 48 << 10, kMostShared = 200 << 10;
+    delay_block_ = std::min(cfg_.block == 0 ? 128 : cfg_.block, fp32_ ? kDelayThreads<float> : kDelayThreads<double>);
     const auto bytes = [&](int W) {
-        return fp32_ ? delay_shared_bytes<float>(W, block_) : delay_shared_bytes<double>(W, block_);
+        return fp32_ ? delay_shared_bytes<float>(W, delay_block_) : delay_shared_bytes<double>(W, delay_block_);
     };
     const int longest = std::max({rc.d_e, rc.d_i, rc.d_a2n});
     int W = std::min({rc.d_e, rc.d_i, rc.d_a2n, kMaxWindow});
@@ -321,7 +321,7 @@ Status Simulation::delay_setup() {
 
 Status Simulation::delay_launch(i64 first, i64 count) {
     const int W = delay_W_;
-    const CellTiles tiles = cell_tiles(rc_.n_exc, 0, rc_.n_neurons, 0, rc_.n_astro, static_cast<u32>(block_));
+    const CellTiles tiles = cell_tiles(rc_.n_exc, 0, rc_.n_neurons, 0, rc_.n_astro, static_cast<u32>(delay_block_));
     const auto wrap = [](i64 x, i64 n) { return static_cast<u32>((x % n + n) % n); };
     for (i64 t = first; t < first + count;) {
         const i64 k = t / W;
@@ -344,8 +344,8 @@ Status Simulation::delay_launch(i64 first, i64 count) {
         w.e = delayed(rc_.d_e);
         w.i = delayed(rc_.d_i);
         w.a2n = delayed(rc_.d_a2n);
-        if (fp32_) launch_delay_window<float>(rc_, make_ptrs<float>(st_, net_, rc_, cfg_.raster_steps), w, tiles, block_, stream_);
-        else launch_delay_window<double>(rc_, make_ptrs<double>(st_, net_, rc_, cfg_.raster_steps), w, tiles, block_, stream_);
+        if (fp32_) launch_delay_window<float>(rc_, make_ptrs<float>(st_, net_, rc_, cfg_.raster_steps), w, tiles, delay_block_, stream_);
+        else launch_delay_window<double>(rc_, make_ptrs<double>(st_, net_, rc_, cfg_.raster_steps), w, tiles, delay_block_, stream_);
         AS_CUDA(cudaGetLastError());
         t = w.start + w.s_end;
     }

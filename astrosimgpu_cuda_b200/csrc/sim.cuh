@@ -182,7 +182,7 @@ private:
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     bool have_step_events_ = false;
     int device_ = 0;
-    int block_ = 128;
+    int delay_block_ = 128;
     bool fp32_ = false;
     i64 pre_steps_ = 0, sim_steps_ = 0, total_steps_ = 0, steps_done_ = 0;
     i64 counts_cap_ = 0;

@@ -43,3 +43,14 @@ def test_threads_with_different_windows():
     for run, result in zip(runs, got):
         for a, b in zip(result, want[run["dt"]]):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("block", [736, 768, 1024])
+def test_delay_windows(block, precision):
+    """Delays that the windowed engine does not take: the registers of the FP64 form bound its
+    blocks below the largest that a configuration may ask for."""
+    bio = {"w_e": 25.0, "SIC_th": 0.0715, "d_e": 0.6, "d_i": 1.6, "d_a2n": 1.0}
+    chunks = (3, 47, 50)
+    for a, b in zip(states(chunks, bio, block=block, precision=precision), states(chunks, bio, precision=precision)):
+        np.testing.assert_array_equal(a, b)
