@@ -37,16 +37,18 @@ DT = 0.1
 PRE_MS, SIM_MS = 100.0, 500.0
 
 
-# One steady-state window_kernel launch measured by ncu (profiles/), at
-# N_total = 3e6, where the state streamed per launch is several times the L2:
-# DRAM bytes read + written, warp instructions issued and the fraction of issue
-# slots busy.  Bytes and instructions grow with the cell count, so a launch at N
-# carries about N / 3e6 times these.
+# One steady-state window measured by ncu (profiles/): its window_kernel launch and the
+# push_kernel launch that delivers it and draws the next window's background events, at
+# N_total = 3e6, where the state streamed per launch is several times the L2.  DRAM bytes
+# read + written and warp instructions issued of both, and the fraction of issue slots busy
+# in the window kernel.  Bytes and instructions grow with the cell count, so a window at N
+# takes about N / 3e6 times these.
 PROFILED_WINDOW = {
-    "fp32": {"n": 3_000_000, "dram": 344.72e6, "warp_inst": 239.78e6, "issue_busy": 0.840},
-    "fp64": {"n": 3_000_000, "dram": 472.80e6, "warp_inst": 665.70e6, "issue_busy": 0.707},
+    "fp32": {"n": 3_000_000, "dram": 339.22e6 + 17.96e6, "warp_inst": 240.30e6 + 73.47e6, "issue_busy": 0.851},
+    "fp64": {"n": 3_000_000, "dram": 466.57e6 + 16.91e6, "warp_inst": 665.32e6 + 73.48e6, "issue_busy": 0.710},
 }
-PROFILED_SOURCE = "ncu, one steady-state window_kernel launch at N_total=3e6 (profiles/), scaled to N_total"
+PROFILED_SOURCE = ("ncu, one steady-state window at N_total=3e6 (window_kernel + push_kernel, profiles/), scaled to "
+                   "N_total")
 SCHEDULERS_PER_SM = 4  # warp schedulers per B200 SM: one warp instruction each per cycle at most
 
 
@@ -160,29 +162,29 @@ def gather_step_bytes(s, precision):
 
 
 def window_step_bytes(s, precision, spikes_per_step, window=10):
-    """Algorithmic bytes per time step of the windowed engine (one launch per window).
+    """Algorithmic bytes per time step of the windowed engine (a window launch and a push
+    launch per window).
 
-    Per window each neuron reads V, w, V_reset, b (32 B), five conductance/SIC
-    values, its refractory counter and inbox count (8 B) and its a2n flag bit, and
-    writes V, w, the five values, the counter and its spike word; a neuron whose a2n
-    row holds an active astrocyte also reads the row (8 B of row_start + 4 B per
-    entry; estimated from the active astrocytes at the last step times their a2n
-    fan-out).  Each astrocyte reads Ca, IP3, h, four parameters, its inbox count and
-    flag, and writes Ca, IP3, h, `window` SIC factors, its flag and last factor.
-    Each spike delivers one deposit (key, step, value: 12 B FP32 / 16 B FP64, plus a
-    4 B count update) per outgoing edge.
+    Per window each neuron reads V, w (16 B), five conductance/SIC values, its refractory
+    counter, inbox count and marked a2n positions (12 B) and its background events (8 B),
+    and writes V, w, the four conductances and its spike word; the push wrote its events
+    (8 B).  Each astrocyte reads Ca, IP3, h, four parameters, its inbox count and flag, and
+    writes Ca, IP3, h and its last factor.  An active one (those of the last step stand for
+    the run's) writes `window` SIC factors, which are read once, and each entry of its a2n
+    list is read, marked in its target and read again as the target's row entry (12 B).
+    Each spike reads V_reset and b and delivers one deposit (key, step, value: 12 B FP32 /
+    16 B FP64, plus a 4 B count update) per outgoing edge.
     """
     r = 8 if precision == "fp64" else 4
     nn = s["n_exc"] + s["n_inh"]
     na = s["n_astro"]
-    a2n_fanout = s["n_sic_edges"] / max(1, na)
-    flagged = min(nn, s.get("active_astro", 0) * a2n_fanout)
-    row = s["n_sic_edges"] / max(1, nn)
-    neuron = nn * (32 + 5 * r + 8 + 1 / 8 + 16 + 5 * r + 8) + flagged * (8 + 4 * row)
-    astro = na * (16 + r + 32 + 5 + 16 + r + window * r + 1 + r)
+    active = min(na, s.get("active_astro", 0))
+    neuron = nn * (16 + 5 * r + 12 + 8 + 16 + 4 * r + 4 + 8)
+    astro = na * (16 + r + 32 + 5 + 16 + r + r + 1 / 8)
+    sic = active * (2 * window * r + 12 * s["n_sic_edges"] / max(1, na))
     fanout = (s["n_exc_edges"] + s["n_inh_edges"] + s["n_e2a_edges"]) / max(1, nn)
-    deposits = spikes_per_step * window * fanout * ((16 if r == 8 else 12) + 4)
-    return (neuron + astro + deposits) / window
+    deposits = spikes_per_step * window * (16 + fanout * ((16 if r == 8 else 12) + 4))
+    return (neuron + astro + sic + deposits) / window
 
 
 def sm_count(device):
@@ -194,17 +196,18 @@ def sm_count(device):
 
 
 def roofline(leg, prec, achieved, peak, peak_kind, ms_step, device):
-    """The window kernel's roofline: HBM bytes against the measured copy bandwidth,
-    and, since the kernel is bound by instruction issue, warp instructions issued
-    against one per scheduler per cycle at the SM clock sampled during the run."""
+    """The roofline of a window (its window and push launches): HBM bytes against the
+    measured copy bandwidth, and, since both are bound by instruction issue, warp
+    instructions issued against one per scheduler per cycle at the SM clock sampled
+    during the run."""
     prof = PROFILED_WINDOW[prec]
     scale = N_TOTAL / prof["n"]
     out = {"bound": "issue", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
            "traffic": prof["dram"] * scale if prof["dram"] else None,
            "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum, " + PROFILED_SOURCE,
            "peak_source": peak_kind,
-           "kernel": f"window_kernel<{'float' if prec == 'fp32' else 'double'}> (one launch = one 10-step window, "
-                     f"its push_kernel inside the timed duration)",
+           "kernel": f"window_kernel<{'float' if prec == 'fp32' else 'double'}> (one launch = one 10-step window) "
+                     f"and its push_kernel",
            "algorithmic_bytes_per_step": leg["bytes"],
            "gather_formulation_bytes_per_step": leg["gather_bytes"],
            "gather_formulation_equivalent_gbs": leg["gather_bytes"] / (ms_step * 1e-3) / 1e9}
