@@ -35,14 +35,15 @@ __device__ __forceinline__ WindowSchedule window_schedule(int d_a2n, int sic_int
         fresh = spn - static_cast<int>(t0 % spn);
         if (si > 1) first = (si - static_cast<int>((t0 - d_a2n) % si)) % si;
     }
-    // unsigned: a step and the largest interval add up to less than 2^32
-    const u32 steps = static_cast<u32>(n);
+    // a step past the longest window ends the loops below, which an interval near the
+    // largest int would overflow (added up unsigned: 1 % of the FP64 window at N = 1e6)
+    constexpr int kPast = 16;
     if (si == 1) {
         if (first < n) w.refresh = (1u << n) - (1u << first);
     } else {
-        for (u32 i = static_cast<u32>(first); i < steps; i += static_cast<u32>(si)) w.refresh |= 1u << i;
+        for (int i = first; i < n; i += si < kPast ? si : kPast) w.refresh |= 1u << i;
     }
-    for (u32 i = static_cast<u32>(fresh); i < steps; i += static_cast<u32>(spn)) w.noise |= 1u << i;
+    for (int i = fresh; i < n; i += spn < kPast ? spn : kPast) w.noise |= 1u << i;
     w.refresh <<= s_begin;
     w.noise <<= s_begin;
     return w;
