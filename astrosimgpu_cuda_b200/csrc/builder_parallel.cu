@@ -349,11 +349,12 @@ __device__ __forceinline__ u32 lower_bound_near(const u64* entries, u64 c) {
 // The replay of the E block's autapses in order (one block).  On the table orbit with
 // running shift d (true index - table index) the next autapse is the next hazard that
 // lands d from its table index.  From there the walk leaves the table orbit: its pres are
-// taken in batches of up to 32 (4 in the first, which most walks rejoin in), whose starts
-// follow from the lengths; a lane walks each pre in full for a landing on its true index
-// and looks its start up in the table orbit.  The first of the two ends the batch: an
-// autapse sends the walk on from that pre's exact end, a start on the table orbit ends
-// it.  (Walks rejoin after a median of 2 pres, some after hundreds.)  What bounds it is
+// taken in batches of up to 32, whose starts follow from the lengths; a lane walks each pre
+// in full for a landing on its true index and looks its start up in the table orbit.  The
+// first of the two ends the batch: an autapse sends the walk on from that pre's exact end,
+// a start on the table orbit ends it.  (The first batch, of 4, ends after its first pre,
+// the autapse that the walk starts at; walks rejoin after a median of 2 pres from there,
+// some after hundreds.)  What bounds it is
 // latency: the load of the window and a lane's walk of about a hundred words.  512 threads
 // load, look through the hazards in shared memory and through the table starts around the
 // walk, and a landing waits once for its two words: 1.3 ms at N = 1e3, 2.6 ms at N = 3e5 (1.5

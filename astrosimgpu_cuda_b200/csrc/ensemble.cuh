@@ -3,13 +3,14 @@
 // Each network keeps its own device state exactly as a single Simulation (its own
 // windowed engine buffers).  One window launch covers every cell of every network:
 // a tile table maps each block (a tile of 64, 128 or 256 cells: the autotuner times
-// each size with three occupancy targets) to (network, population, tile), and each block reads its network's descriptor (constants and pointers) into shared memory.
+// each size with three occupancy targets) to (network, population, tile), and each block
+// reads its network's descriptor (constants and pointers) into shared memory.
 // The constants that differ between networks (NetScalars) sit in the descriptor;
 // when every network shares the rest (the same biology, dt and substeps) those come
 // from the kernel parameters, else each block also stages its network's full
 // constants.  Every network has its own window counter and stop step on the device, so the
-// per-window sequence {window, push and next window's draws, advance} is identical for every window and is
-// captured once in a CUDA graph and replayed.
+// per-window sequence {window, push and next window's draws, advance} is identical for
+// every window and is captured once in a CUDA graph and replayed.
 #pragma once
 
 #include <memory>

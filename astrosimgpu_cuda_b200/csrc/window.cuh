@@ -11,8 +11,8 @@
 //     the target sorts its deposits into CSR row order and sums them, which is
 //     bit-identical to the reference's dense gather (its skipped terms are +0.0);
 //   - pull (a busy window, or a target whose slots overflowed): the target walks its
-//     CSR rows against the previous window's per-neuron spike words, exactly like
-//     the per-step gather.
+//     CSR rows against the previous window's per-neuron spike words, in the order in
+//     which the reference's gather sums them.
 // SIC factors are pulled by the neurons whose a2n row holds an astrocyte that was active:
 // the push walks each active astrocyte's forward a2n list and marks its position in each
 // target's row, so that a neuron reads its marked positions only, and a neuron without

@@ -2,7 +2,9 @@
 raster bit that an engine which draws, gathers and rounds every step by itself gave for the
 same runs (golden/window_states.json).  Tile edges and large networks (both forms of the
 background draw), rates on both sides of the window-wide draw's limit, windows of 2 to 16
-steps, busy windows, active astrocytes, facilitation, and calls that split windows."""
+steps, busy windows, active astrocytes, facilitation, and calls that split windows.  The
+digests come from the library of commit 9485e4f with ASTROSIM_STEPPER=plain, the last one
+with such an engine."""
 import hashlib
 import json
 from pathlib import Path
